@@ -43,75 +43,128 @@ __device__ __forceinline__ bool flagged(const uint32_t* status) { return status 
 // ---------------------------------------------------------------------------
 // Count particles per row.  Optionally applies the drift disp += vel * D
 // first (integrator.py:223-225, two roundings as in the reference) and writes
-// the drifted displacement back.  Ranks come from warp-aggregated atomics.
-// With a shift the mesh origin moves (BinShift); particles with valid[i] == 0
-// go to the extra bin after the last row (their records trail the sorted
-// array with kMaskedKey).
-__global__ void bin_count_kernel(const int16_t* __restrict__ pmid, float* __restrict__ disp,
-                                 const float* __restrict__ vel, float drift, int64_t n, Mesh3 m, float cell,
-                                 BinShift sh, const uint8_t* __restrict__ valid, uint32_t* __restrict__ counts,
-                                 uint32_t* __restrict__ row_of, uint32_t* __restrict__ rank_of,
-                                 uint32_t* __restrict__ status) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = i < n;
-  uint32_t row = 0xFFFFFFFFu;
-  if (active) {
-    float d0 = disp[3 * i], d1 = disp[3 * i + 1], d2 = disp[3 * i + 2];
-    if (vel != nullptr) {
-      d0 = __fadd_rn(d0, __fmul_rn(vel[3 * i], drift));
-      d1 = __fadd_rn(d1, __fmul_rn(vel[3 * i + 1], drift));
-      d2 = __fadd_rn(d2, __fmul_rn(vel[3 * i + 2], drift));
-      disp[3 * i] = d0;
-      disp[3 * i + 1] = d1;
-      disp[3 * i + 2] = d2;
-    }
-    if (!(isfinite(d0) && isfinite(d1) && isfinite(d2))) raise_flag(status, kFlagNonFiniteDisp);
-    if (valid != nullptr && !valid[i]) {
-      row = (uint32_t)m.rows();
-    } else {
-      Binned b = bin_particle(pmid, d0, d1, d2, i, m, cell, sh);
-      row = (uint32_t)((int64_t)b.cx * m.ny + b.cy);
-    }
-  }
-  unsigned full = __ballot_sync(0xFFFFFFFFu, active);
-  if (!active) return;
-  unsigned peers = __match_any_sync(full, row);
-  int leader = __ffs(peers) - 1;
-  int lane = threadIdx.x & 31;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(&counts[row], (uint32_t)__popc(peers));
-  base = __shfl_sync(peers, base, leader);
-  row_of[i] = row;
-  rank_of[i] = base + __popc(peers & ((1u << lane) - 1u));
+// the drifted displacement back.  With a shift the mesh origin moves
+// (BinShift); particles with valid[i] == 0 go to the extra bin after the last
+// row (their records trail the sorted array with kMaskedKey).
+//
+// Ranks come from one atomic per run of equal rows in the warp: particles come
+// in lattice order, z fastest, so neighbouring lanes mostly share a row, and a
+// run is found with one shuffle and one ballot.  (Grouping all equal rows of
+// the warp with __match_any_sync saves some atomics but its own issue was the
+// bound: 342 us for 256^3 and 2.71 ms for 512^3 clustered particles, 174 us
+// and 1.26 ms by runs; the bytes take 0.07 and 0.6 ms.)  kSortPer particles a
+// thread, a block apart, so that their loads overlap.
+constexpr int kSortThreads = 256;
+constexpr int kSortPer = 4;
+
+__device__ __forceinline__ uint32_t row_bin(const int16_t* __restrict__ pmid, float d0, float d1, float d2, int64_t i,
+                                            Mesh3 m, float cell, const BinShift& sh,
+                                            const uint8_t* __restrict__ valid) {
+  if (valid != nullptr && !valid[i]) return (uint32_t)m.rows();
+  const Binned b = bin_particle(pmid, d0, d1, d2, i, m, cell, sh);
+  return (uint32_t)b.cx * (uint32_t)m.ny + (uint32_t)b.cy;
 }
 
-__global__ void bin_place_kernel(const int16_t* __restrict__ pmid, const float* __restrict__ disp, int64_t n,
-                                 Mesh3 m, float cell, BinShift sh, const uint32_t* __restrict__ offs,
-                                 const uint32_t* __restrict__ row_of, const uint32_t* __restrict__ rank_of,
-                                 Rec* __restrict__ rec, uint32_t* __restrict__ perm) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const int16_t* __restrict__ pmid,
+                                                                 float* __restrict__ disp,
+                                                                 const float* __restrict__ vel, float drift, int64_t n,
+                                                                 Mesh3 m, float cell, BinShift sh,
+                                                                 const uint8_t* __restrict__ valid,
+                                                                 uint32_t* __restrict__ counts,
+                                                                 uint32_t* __restrict__ row_of,
+                                                                 uint32_t* __restrict__ rank_of,
+                                                                 uint32_t* __restrict__ flag) {
+  const int64_t base = (int64_t)blockIdx.x * (kSortThreads * kSortPer) + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const unsigned upto = 0xFFFFFFFFu >> (31 - lane);  // lanes 0 .. lane
+  float d[kSortPer][3];
+#pragma unroll
+  for (int k = 0; k < kSortPer; ++k) {
+    const int64_t i = base + k * kSortThreads;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) d[k][a] = i < n ? disp[3 * i + a] : 0.f;
+  }
+  if (vel != nullptr) {
+#pragma unroll
+    for (int k = 0; k < kSortPer; ++k) {
+      const int64_t i = base + k * kSortThreads;
+      if (i < n) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          d[k][a] = __fadd_rn(d[k][a], __fmul_rn(vel[3 * i + a], drift));
+          disp[3 * i + a] = d[k][a];
+        }
+      }
+    }
+  }
+  uint32_t head_base[kSortPer];
+  int head[kSortPer];
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < kSortPer; ++k) {
+    const int64_t i = base + k * kSortThreads;
+    bad |= !(isfinite(d[k][0]) && isfinite(d[k][1]) && isfinite(d[k][2]));
+    uint32_t row = 0xFFFFFFFFu;
+    if (i < n) row_of[i] = row = row_bin(pmid, d[k][0], d[k][1], d[k][2], i, m, cell, sh, valid);
+    const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, row, 1);
+    const unsigned heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || row != prev);
+    head[k] = 31 - __clz(heads & upto);
+    head_base[k] = 0;
+    if (head[k] == lane && i < n) {
+      const unsigned after = heads & ~upto;
+      const int len = (after ? __ffs(after) - 1 : 32) - lane;
+      head_base[k] = atomicAdd(&counts[row], (uint32_t)len);
+    }
+  }
+  if (bad) raise_flag(flag, kFlagNonFiniteDisp);
+#pragma unroll
+  for (int k = 0; k < kSortPer; ++k) {
+    const int64_t i = base + k * kSortThreads;
+    const uint32_t b = __shfl_sync(0xFFFFFFFFu, head_base[k], head[k]);
+    if (i < n) rank_of[i] = b + (uint32_t)(lane - head[k]);
+  }
+}
+
+// Records to their places: bound by the scattered stores (about one 128-byte
+// line per run of equal rows for the record and one for the index; 0.29 ms for
+// 256^3 clustered particles against 0.11 ms for the bytes).  Two or four
+// particles a thread, streaming loads and forming the row again instead of
+// reading row_of all measured slower (0.31 - 0.33 ms).
+__global__ void __launch_bounds__(kSortThreads) bin_place_kernel(const int16_t* __restrict__ pmid,
+                                                                 const float* __restrict__ disp, int64_t n, Mesh3 m,
+                                                                 float cell, BinShift sh,
+                                                                 const uint32_t* __restrict__ offs,
+                                                                 const uint32_t* __restrict__ row_of,
+                                                                 const uint32_t* __restrict__ rank_of,
+                                                                 Rec* __restrict__ rec, uint32_t* __restrict__ perm) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t row = row_of[i];
-  uint32_t dst = offs[row] + rank_of[i];
+  const uint32_t dst = offs[row] + rank_of[i];
   Rec r;
   if (row == (uint32_t)m.rows()) {
     r.fx = r.fy = r.fz = 0.f;
     r.key = kMaskedKey;
   } else {
-    Binned b = bin_particle(pmid, disp[3 * i], disp[3 * i + 1], disp[3 * i + 2], i, m, cell, sh);
+    const Binned b = bin_particle(pmid, disp[3 * i], disp[3 * i + 1], disp[3 * i + 2], i, m, cell, sh);
     r.fx = b.fx;
     r.fy = b.fy;
     r.fz = b.fz;
-    r.key = (uint32_t)(((int64_t)b.cx * m.ny + b.cy) * m.nz + b.cz);
+    r.key = row * (uint32_t)m.nz + (uint32_t)b.cz;
   }
   rec[dst] = r;
   perm[dst] = (uint32_t)i;
 }
 
-// Exclusive scan of row counts, three phases over tiles of 4096 entries.
+// Exclusive scan of row counts: one block up to kScanOne entries (the row
+// counts of a 128^3 mesh; 7 us, as the three launches it replaces, with two
+// launches saved on the host), else two launches over tiles of 4096 entries,
+// the second adding the sum of the tiles before its own.
 constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 4;
 constexpr int kScanTile = kScanThreads * kScanPer;
+constexpr int kScanOneTiles = 4;
+constexpr int64_t kScanOne = kScanOneTiles * kScanTile + 1;
 
 __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* sh, uint32_t* total) {
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -138,9 +191,73 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* sh, uint32_t* tot
   return r;
 }
 
-__global__ void scan_tiles_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int64_t n,
-                                  uint32_t* __restrict__ tile_sums) {
+// A flag word raised by the counting pass, handed on to the sorted buffer's
+// status word by the scan (both may be null).
+__device__ __forceinline__ void hand_on_flag(const uint32_t* flag, uint32_t* status) {
+  if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = flag != nullptr ? *flag : 0u;
+}
+
+// All entries in one block: kScanOneTiles coalesced groups of four entries a
+// thread, scanned side by side.  The last entry (n - 1) is only written: no
+// exclusive sum contains its count.
+__global__ void __launch_bounds__(kScanThreads) scan_one_kernel(const uint32_t* in, uint32_t* out, int64_t n,
+                                                                const uint32_t* flag, uint32_t* status) {
+  __shared__ uint32_t sh[kScanOneTiles][33];
+  hand_on_flag(flag, status);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t last = n - 1;
+  uint32_t v[kScanOneTiles][kScanPer], x[kScanOneTiles], own[kScanOneTiles];
+#pragma unroll
+  for (int c = 0; c < kScanOneTiles; ++c) {
+    const int64_t base = (int64_t)c * kScanTile + (int64_t)threadIdx.x * kScanPer;
+    uint32_t s = 0;
+#pragma unroll
+    for (int j = 0; j < kScanPer; ++j) {
+      v[c][j] = base + j < last ? in[base + j] : 0u;
+      s += v[c][j];
+    }
+    own[c] = x[c] = s;
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+    for (int c = 0; c < kScanOneTiles; ++c) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x[c], o);
+      if (lane >= o) x[c] += y;
+    }
+  if (lane == 31)
+#pragma unroll
+    for (int c = 0; c < kScanOneTiles; ++c) sh[c][warp] = x[c];
+  __syncthreads();
+  if (warp < kScanOneTiles) {
+    uint32_t w = sh[warp][lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+      if (lane >= o) w += y;
+    }
+    sh[warp][lane] = w;
+  }
+  __syncthreads();
+  uint32_t carry = 0;
+#pragma unroll
+  for (int c = 0; c < kScanOneTiles; ++c) {
+    const int64_t base = (int64_t)c * kScanTile + (int64_t)threadIdx.x * kScanPer;
+    uint32_t off = carry + (warp ? sh[c][warp - 1] : 0u) + x[c] - own[c];
+#pragma unroll
+    for (int j = 0; j < kScanPer; ++j) {
+      if (base + j < last) out[base + j] = off;
+      off += v[c][j];
+    }
+    carry += sh[c][31];
+  }
+  if (threadIdx.x == 0) out[last] = carry;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const uint32_t* in, uint32_t* out, int64_t n,
+                                                                  uint32_t* __restrict__ tile_sums,
+                                                                  const uint32_t* flag, uint32_t* status) {
   __shared__ uint32_t sh[32];
+  hand_on_flag(flag, status);
   int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanPer;
   uint32_t v[kScanPer];
   uint32_t s = 0;
@@ -157,37 +274,42 @@ __global__ void scan_tiles_kernel(const uint32_t* __restrict__ in, uint32_t* __r
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-__global__ void scan_sums_kernel(uint32_t* __restrict__ sums, int64_t ntiles, uint32_t* __restrict__ grand) {
+// Adds the sum of the tiles before this block's own (block 0 has none).
+__global__ void __launch_bounds__(kScanThreads) scan_add_kernel(uint32_t* __restrict__ out, int64_t n,
+                                                                const uint32_t* __restrict__ tile_sums) {
   __shared__ uint32_t sh[32];
-  uint32_t carry = 0;
-  for (int64_t b = 0; b < ntiles; b += blockDim.x) {
-    int64_t i = b + threadIdx.x;
-    uint32_t v = i < ntiles ? sums[i] : 0u;
-    uint32_t total;
-    uint32_t off = block_exclusive_scan(v, sh, &total);
-    if (i < ntiles) sums[i] = carry + off;
-    carry += total;
+  const int64_t tile = (int64_t)blockIdx.x + 1;
+  uint32_t s = 0;
+  for (int64_t t = threadIdx.x; t < tile; t += kScanThreads) s += tile_sums[t];
+  uint32_t before;
+  block_exclusive_scan(s, sh, &before);
+#pragma unroll
+  for (int j = 0; j < kScanPer; ++j) {
+    const int64_t i = tile * kScanTile + j * kScanThreads + threadIdx.x;
+    if (i < n) out[i] += before;
   }
-  if (threadIdx.x == 0) *grand = carry;
-}
-
-__global__ void scan_add_kernel(uint32_t* __restrict__ out, int64_t n, const uint32_t* __restrict__ sums) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += sums[i / kScanTile];
 }
 
 int64_t scan_tmp_elems(int64_t len) { return (len + kScanTile - 1) / kScanTile + 1; }
 
 // Exclusive scan of len uint32 values (in == out allowed); tile_sums needs
-// scan_tmp_elems(len) entries.
-int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t len, uint32_t* tile_sums, cudaStream_t s) {
+// scan_tmp_elems(len) entries.  flag / status: hand_on_flag.
+static int exclusive_scan(const uint32_t* in, uint32_t* out, int64_t len, uint32_t* tile_sums, const uint32_t* flag,
+                          uint32_t* status, cudaStream_t s) {
   if (len <= 0) return kOk;
-  const int64_t ntiles = (len + kScanTile - 1) / kScanTile;
-  scan_tiles_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, out, len, tile_sums);
-  scan_sums_kernel<<<1, 1024, 0, s>>>(tile_sums, ntiles, tile_sums + ntiles);
-  scan_add_kernel<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(out, len, tile_sums);
+  if (len <= kScanOne) {
+    scan_one_kernel<<<1, kScanThreads, 0, s>>>(in, out, len, flag, status);
+  } else {
+    const int64_t ntiles = (len + kScanTile - 1) / kScanTile;
+    scan_tiles_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, out, len, tile_sums, flag, status);
+    scan_add_kernel<<<(unsigned)(ntiles - 1), kScanThreads, 0, s>>>(out, len, tile_sums);
+  }
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
+}
+
+int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t len, uint32_t* tile_sums, cudaStream_t s) {
+  return exclusive_scan(in, out, len, tile_sums, nullptr, nullptr, s);
 }
 
 int64_t bin_scratch_bytes(int64_t n, Mesh3 m) {
@@ -205,30 +327,27 @@ int bin_particles(const int16_t* pmid, float* disp, const float* vel, float drif
   if (shift != nullptr) sh = *shift;
   int64_t rows = m.rows();
   char* p = (char*)scratch;
+  const int64_t len = rows + 1;
   uint32_t* counts = (uint32_t*)p;
-  p += align_up(4 * (rows + 1), 256);
+  p += align_up(4 * len, 256);
+  // the counting pass raises its flag in the word after the counts, cleared
+  // together with them (a separate launch costs 2 us)
+  uint32_t* flag = (uint32_t*)p;
+  p += 256;
   uint32_t* row_of = (uint32_t*)p;
   p += align_up(4 * n, 256);
   uint32_t* rank_of = (uint32_t*)p;
   p += align_up(4 * n, 256);
   uint32_t* tile_sums = (uint32_t*)p;
-  int64_t len = rows + 1;
-  int64_t ntiles = (len + kScanTile - 1) / kScanTile;
-  PMB_CUDA_CHECK(cudaMemsetAsync(counts, 0, 4 * len, s));
-  if (status != nullptr) PMB_CUDA_CHECK(cudaMemsetAsync(status, 0, 4, s));
-  if (n > 0) {
-    int th = 256;
-    bin_count_kernel<<<(unsigned)((n + th - 1) / th), th, 0, s>>>(pmid, disp, vel, drift, n, m, cell, sh, valid,
-                                                                    counts, row_of, rank_of, status);
-  }
-  (void)ntiles;
-  int st = exclusive_scan_u32(counts, offs, len, tile_sums, s);
+  PMB_CUDA_CHECK(cudaMemsetAsync(counts, 0, align_up(4 * len, 256) + 4, s));
+  const auto grid_of = [n](int per) { return (unsigned)((n + kSortThreads * per - 1) / (kSortThreads * per)); };
+  if (n > 0)
+    bin_count_kernel<<<grid_of(kSortPer), kSortThreads, 0, s>>>(pmid, disp, vel, drift, n, m, cell, sh, valid, counts,
+                                                             row_of, rank_of, flag);
+  int st = exclusive_scan(counts, offs, len, tile_sums, flag, status, s);
   if (st != kOk) return st;
-  if (n > 0) {
-    int th = 256;
-    bin_place_kernel<<<(unsigned)((n + th - 1) / th), th, 0, s>>>(pmid, disp, n, m, cell, sh, offs, row_of,
-                                                                    rank_of, rec, perm);
-  }
+  if (n > 0)
+    bin_place_kernel<<<grid_of(1), kSortThreads, 0, s>>>(pmid, disp, n, m, cell, sh, offs, row_of, rank_of, rec, perm);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }

@@ -29,9 +29,9 @@ __device__ __forceinline__ Binned bin_particle(const int16_t* __restrict__ pmid,
   b.fx = __fsub_rn(q0, l0);
   b.fy = __fsub_rn(q1, l1);
   b.fz = __fsub_rn(q2, l2);
-  b.cx = pmod((int)pmid[3 * i + 0] + (int)l0, m.nx);
-  b.cy = pmod((int)pmid[3 * i + 1] + (int)l1, m.ny);
-  b.cz = pmod((int)pmid[3 * i + 2] + (int)l2, m.nz);
+  b.cx = wrap((int)pmid[3 * i + 0] + (int)l0, m.nx);
+  b.cy = wrap((int)pmid[3 * i + 1] + (int)l1, m.ny);
+  b.cz = wrap((int)pmid[3 * i + 2] + (int)l2, m.nz);
   return b;
 }
 
@@ -55,9 +55,9 @@ __device__ __forceinline__ Binned bin_particle(const int16_t* __restrict__ pmid,
   b.fx = __fsub_rn(q0, l0);
   b.fy = __fsub_rn(q1, l1);
   b.fz = __fsub_rn(q2, l2);
-  b.cx = pmod((int)pmid[3 * i + 0] - sh.qx + (int)l0, m.nx);
-  b.cy = pmod((int)pmid[3 * i + 1] - sh.qy + (int)l1, m.ny);
-  b.cz = pmod((int)pmid[3 * i + 2] - sh.qz + (int)l2, m.nz);
+  b.cx = wrap((int)pmid[3 * i + 0] - sh.qx + (int)l0, m.nx);
+  b.cy = wrap((int)pmid[3 * i + 1] - sh.qy + (int)l1, m.ny);
+  b.cz = wrap((int)pmid[3 * i + 2] - sh.qz + (int)l2, m.nz);
   return b;
 }
 

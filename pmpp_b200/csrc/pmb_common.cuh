@@ -50,6 +50,14 @@ __host__ __device__ inline int pmod(int a, int m) {
   return r < 0 ? r + m : r;
 }
 
+// pmod with a short cut for indices less than one period outside the mesh (a
+// remainder by a variable costs about twenty instructions).
+__device__ __forceinline__ int wrap(int a, int m) {
+  if ((unsigned)a < (unsigned)m) return a;
+  const int b = a < 0 ? a + m : a - m;
+  return (unsigned)b < (unsigned)m ? b : pmod(a, m);
+}
+
 __host__ __device__ inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
 // Particle binning shared by every CIC kernel.  Restates the float32

@@ -163,14 +163,13 @@ int pmb_scatter_rows(const void* sorted, int64_t n, int nx, int ny, int nz, int 
   PMB_REQUIRE(C >= 1 && C <= 4, "pmb_scatter_rows: 1..4 channels supported");
   PMB_REQUIRE(mode == 0 || mode == 1, "pmb_scatter_rows: mode must be 0 or 1");
   SortedView v = sorted_view((void*)sorted, n, m);
-  double* scale = (double*)scratch16;
-  unsigned int* tmp = (unsigned int*)((char*)scratch16 + 8);
+  // a constant value's scale needs no device word
+  double* scale = nullptr;
   if (val != nullptr) {
-    PMB_TRY(compute_scale(val, n * C, n, scale, tmp, S(stream)));
+    scale = (double*)scratch16;
+    PMB_TRY(compute_scale(val, n * C, n, scale, (unsigned int*)((char*)scratch16 + 8), S(stream)));
   } else {
-    float a = fabsf(val_const);
-    PMB_REQUIRE(a < INFINITY, "pmb_scatter_rows: non-finite value");
-    PMB_TRY(set_double(scale, fixed_point_scale(fixed_point_pow2(n), a), S(stream)));
+    PMB_REQUIRE(fabsf(val_const) < INFINITY, "pmb_scatter_rows: non-finite value");
   }
   return scatter_sorted(v.rec, v.perm, v.offs, m, C, val, val_sorted, val_const, scale, mode, src_mul, out,
                         S(stream), n, v.status);

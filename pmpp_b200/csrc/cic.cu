@@ -10,13 +10,16 @@
 //    ((x*My + y)*Mz + z, core/utils.py:292-326) at row granularity;
 //  * the scatter is a pull kernel: one CTA owns an RX x RY block of output
 //    rows, reads the particles of the (RX+1) x (RY+1) source rows that can
-//    reach it, and accumulates in shared memory in 64-bit fixed point.  The
+//    reach it, and accumulates in shared memory in 64-bit fixed point (split
+//    over two 32-bit planes).  The
 //    result is independent of accumulation order (bit-deterministic), every
 //    output cell is written exactly once with coalesced stores, and no
 //    global atomics or mesh zero-fill pass are needed;
 //  * gathers and adjoint position terms walk particles in sorted order so the
 //    eight corner loads of neighbouring threads hit the same cache lines.
 #include <cstdio>
+#include <tuple>
+#include <type_traits>
 
 #include "pmb_cic_device.cuh"
 #include "pmb_common.cuh"
@@ -404,358 +407,188 @@ int compute_scale(const float* val, int64_t count, int64_t n, double* scale_dev,
 // ---------------------------------------------------------------------------
 // Pull scatter
 // ---------------------------------------------------------------------------
-// Epilogue: mode 0 writes the density sum, mode 1 writes the Poisson source
-// (rho - 1) * src_mul (gravity.py:628-630), both in float.
-template <int C>
-__global__ void __launch_bounds__(256) scatter_pull_kernel(const Rec* __restrict__ rec, const uint32_t* __restrict__ perm,
-                                                           const uint32_t* __restrict__ offs, Mesh3 m, int RX, int RY,
-                                                           const float* __restrict__ val, int val_sorted,
-                                                           float val_const, const double* __restrict__ scale_dev,
-                                                           int mode, float src_mul, float* __restrict__ out,
-                                                           uint32_t* __restrict__ status) {
-  extern __shared__ __align__(16) unsigned int acc_smem[];  // ScatterSmem::acc_bytes(RX, RY, C, nz)
-  __shared__ ScatterSmem sm;
-  if (flagged(status)) return;
-  if (!(*scale_dev == *scale_dev)) {  // NaN scale: a non-finite value
-    if (threadIdx.x == 0) raise_flag(status, kFlagNonFiniteValue);
-    return;
-  }
-  const int nby = (m.ny + RY - 1) / RY;
-  const int x0 = (int)(blockIdx.x / nby) * RX;
-  const int y0 = (int)(blockIdx.x % nby) * RY;
-  scatter_tile<C>(rec, perm, offs, m, RX, RY, x0, y0, val, val_sorted, val_const, *scale_dev, mode, src_mul, out,
-                  acc_smem, sm);
-}
-
-// ---------------------------------------------------------------------------
-// Pull scatter with 32-bit planes (meshes with nz % 4 == 0)
-// ---------------------------------------------------------------------------
-// Same exact fixed-point sums as scatter_tile, in 8 bytes per output cell:
-// each contribution q = rint(val * w * scale) (64-bit in scatter_tile) is
-// split as q = h * 2^s + l with h = rint(q / 2^s) and |l| <= 2^(s-1), and h
-// and l are summed by signed 32-bit shared atomics on two planes.  The block
-// picks s from its particle count K (every cell takes at most K
-// contributions, K < 2^L) and the global bound |q| <= 2^E:
-//   s >= E - 21        keeps |q / 2^s| < 2^22, so h and l come from float
-//                      additions of the magic constant 1.5 * 2^23 (exact,
-//                      round-half-even like the 64-bit conversion);
-//   s >= L + E - 31    keeps |sum h| < 2^31;    s <= 32 - L keeps |sum l| < 2^31;
-//   s <= 22            keeps l exact in the same float addition.
-// A block without such an s (tiny particle counts give E up to 52, or a
-// block holding very many particles) adds the 64-bit q with 64-bit atomics
-// on the same 8 bytes.  The recombined sum h * 2^s + l equals the 64-bit sum
-// exactly, so the output is bit-identical to scatter_tile's.
+// One block owns RX x RY output rows and pulls the particles of the
+// (RX + 1) x (RY + 1) source rows that reach them.  Each contribution q =
+// rint(val * w * scale) (64 bits in scatter_tile, pmb_cic_device.cuh) is split
+// as q = h 2^s + l, and h and l are summed by 32-bit shared atomics on two
+// planes (8 bytes per output cell); the recombined sum equals the 64-bit sum
+// exactly, so the output is bit-identical to scatter_tile's and independent of
+// the particle order.
 //
-// Work is handed out in chunks of 32 particles of one source row, so a warp
-// always works on one row and its corner set is a compile-time case (no
-// divergence, no bounds tests per corner).
-constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
-constexpr int kMagicBits = 0x4B400000;
-
-struct SplitAcc {
-  unsigned int* acc;
-  int cells;
-  float y_scale;  // scale * 2^-s
-  float two_s;    // 2^s
-  // q = rint(contrib * scale) as h * 2^s + l: t = y + M rounds y = q / 2^s
-  // to h (the float ulp at M is 1), y - h is exact (Sterbenz), and
-  // fma(y - h, 2^s, M) rounds (y - h) 2^s to l in the same way.
-  __device__ __forceinline__ void add(int a, float contrib) const {
-    const float y = __fmul_rn(contrib, y_scale);
-    const float t = __fadd_rn(y, kMagic);
-    const float r = __fsub_rn(y, __fsub_rn(t, kMagic));
-    const float u = __fmaf_rn(r, two_s, kMagic);
-    atomicAdd(reinterpret_cast<int*>(&acc[a]), __float_as_int(u) - kMagicBits);
-    atomicAdd(reinterpret_cast<int*>(&acc[cells + a]), __float_as_int(t) - kMagicBits);
-  }
+// The kernel is bound by the shared atomics (L1 throughput 92%; the memory it
+// must touch takes a third of its time), after the split was made of few
+// instructions; with one corner set, conversion and address at a time it was
+// bound by instruction issue (800 instructions per particle; now 380): one
+// channel 24.4 -> 8.7 us for 64^3 particles on 128^3 cells, 519 -> 281 us for
+// 256^3 on 512^3, 3065 -> 2190 us for 512^3 on 1024^3; three channels 1312 ->
+// 822 us for 256^3 on 512^3.  The value is scaled by the power of two
+// scale 2^-s 2^-49 first, so that a contribution c counts units of 2^-49 of h
+// (an exact change of exponent); then t = c 2^-100 is a subnormal float whose
+// bit pattern is the integer h (rounded by the multiplication itself, linear
+// up to 2^24), r = c - t 2^100 is its exact remainder, and r 2^(s - 100) is a
+// subnormal whose bits are l.  Two z corners go through each step as one
+// packed operation (f32x2).
+//   unsigned values: h = floor, so 0 <= l <= 2^s and both planes count in
+//     32 unsigned bits: s >= E - 24, s >= L + E - 32, s <= 24, s <= 32 - L;
+//   signed values: |val| goes through with h to nearest and l biased by
+//     2^(s - 1), and the sign is applied to the integers:
+//     s >= E - 24, s >= L + E - 31, 2 <= s <= 23, s <= 32 - L
+// where K < 2^L particles can reach a cell of the block and |q| <= 2^E.  A
+// block without such an s (very small particle counts, or a block holding very
+// many particles), or a scale outside [2^-50, 2^100], adds the 64-bit q with
+// 64-bit atomics on the same 8 bytes.
+//
+// Particles are handed out one a thread over the block's source rows: for one
+// x the rows y0 - 1 .. y0 + RY - 1 are contiguous in the sorted records
+// (pass 0; row ny - 1 before row 0 is pass 1), so every lane is busy whatever
+// the number of particles in a row, and a record's own key says which output
+// rows it reaches.  NZP: the row stride of the accumulator (nz rounded up to
+// one of a few lengths), a constant so that every corner's address is one of
+// two registers plus an immediate.
+struct FastDiv {  // exact n / d for every 32-bit n
+  uint32_t mul;
+  int sh1, sh2;
 };
 
-// Deposit of one particle of source row (SX, SY) relative to the block.
-template <int C, int RX, int RY, int SX, int SY, bool SPLIT>
-__device__ __forceinline__ void deposit_row(const Rec& r, const float* v, int nz, int cz, const SplitAcc& A,
-                                            unsigned long long* acc64, double scale) {
-  const int cz1 = cz + 1 == nz ? 0 : cz + 1;
-  const float wz0 = axis_weight(r.fz, 0), wz1 = axis_weight(r.fz, 1);
-#pragma unroll
-  for (int bx = 0; bx < 2; ++bx) {
-    const int lx = SX + bx;
-    if (lx < 0 || lx >= RX) continue;
-    const float wx = axis_weight(r.fx, bx);
-#pragma unroll
-    for (int by = 0; by < 2; ++by) {
-      const int ly = SY + by;
-      if (ly < 0 || ly >= RY) continue;
-      const float wxy = __fmul_rn(wx, axis_weight(r.fy, by));
-      const float w0 = __fmul_rn(wxy, wz0), w1 = __fmul_rn(wxy, wz1);
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int base = ((lx * RY + ly) * C + c) * nz;
-        const float c0 = __fmul_rn(v[c], w0), c1 = __fmul_rn(v[c], w1);
-        if (SPLIT) {
-          A.add(base + cz, c0);
-          A.add(base + cz1, c1);
-        } else {
-          atomicAdd(&acc64[base + cz], (unsigned long long)__double2ll_rn((double)c0 * scale));
-          atomicAdd(&acc64[base + cz1], (unsigned long long)__double2ll_rn((double)c1 * scale));
-        }
-      }
-    }
-  }
+inline FastDiv fast_div(uint32_t d) {
+  int l = 0;
+  while (l < 32 && (1ull << l) < d) ++l;
+  FastDiv f;
+  f.mul = (uint32_t)((((1ull << l) - d) << 32) / d + 1);
+  f.sh1 = l < 1 ? l : 1;
+  f.sh2 = l > 1 ? l - 1 : 0;
+  return f;
 }
 
-// Dispatch on the source row index k = (SX + 1) * (RY + 1) + (SY + 1).
-template <int C, int RX, int RY, bool SPLIT, int K = 0>
-__device__ __forceinline__ void deposit_k(int k, const Rec& r, const float* v, int nz, int cz, const SplitAcc& A,
-                                          unsigned long long* acc64, double scale) {
-  if constexpr (K < (RX + 1) * (RY + 1)) {
-    if (k == K) {
-      deposit_row<C, RX, RY, K / (RY + 1) - 1, K % (RY + 1) - 1, SPLIT>(r, v, nz, cz, A, acc64, scale);
-      return;
-    }
-    deposit_k<C, RX, RY, SPLIT, K + 1>(k, r, v, nz, cz, A, acc64, scale);
-  }
+__device__ __forceinline__ uint32_t div_by(uint32_t n, FastDiv f) {
+  const uint32_t q = __umulhi(f.mul, n);
+  return (q + ((n - q) >> f.sh1)) >> f.sh2;
 }
 
-// Epilogue of the split scatters: (float)(sum / scale) as scatter_tile
-// computes it, for the block's RX x RY rows of C channels.  With |h|, |l| <
-// 2^22 both convert exactly through the magic constant and one fma forms
-// h 2^s + l with a single rounding; |sum| < 2^53, so this equals the
-// double-precision route (which the other cells take).
-template <int C, int RX, int RY>
-__device__ __forceinline__ void split_epilogue(const unsigned int* acc, int cells, bool split, int s, double scale,
-                                               float two_s, Mesh3 m, int x0, int y0, int mode, float src_mul,
-                                               float* __restrict__ out) {
-  const double inv = 1.0 / scale;
-  const float invf = (float)inv;
-  const bool fconv = split && invf >= 0x1p-126f;
-  const int64_t mcells = m.cells();
-  const int nz = m.nz, nz4 = nz >> 2;
-  const unsigned long long* acc64 = reinterpret_cast<const unsigned long long*>(acc);
-#pragma unroll
-  for (int lx = 0; lx < RX; ++lx) {
-    if (x0 + lx >= m.nx) break;
-#pragma unroll
-    for (int ly = 0; ly < RY; ++ly) {
-      if (y0 + ly >= m.ny) break;
-      const int64_t row_off = ((int64_t)(x0 + lx) * m.ny + (y0 + ly)) * nz;
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int a0 = ((lx * RY + ly) * C + c) * nz;
-        float* o = out + (int64_t)c * mcells + row_off;
-        for (int z4 = threadIdx.x; z4 < nz4; z4 += blockDim.x) {
-          float res[4];
-          if (split) {
-            const int4 lo = *reinterpret_cast<const int4*>(&acc[a0 + 4 * z4]);
-            const int4 hi = *reinterpret_cast<const int4*>(&acc[cells + a0 + 4 * z4]);
-            const int los[4] = {lo.x, lo.y, lo.z, lo.w};
-            const int his[4] = {hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int h = his[q], l = los[q];
-              if (fconv && h > -(1 << 22) && h < (1 << 22) && l > -(1 << 22) && l < (1 << 22)) {
-                const float hf = __fsub_rn(__int_as_float(kMagicBits + h), kMagic);
-                const float lf = __fsub_rn(__int_as_float(kMagicBits + l), kMagic);
-                res[q] = __fmul_rn(__fmaf_rn(hf, two_s, lf), invf);
-              } else {
-                res[q] = (float)((double)((long long)h * (1ll << s) + (long long)l) * inv);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) res[q] = (float)((double)(long long)acc64[a0 + 4 * z4 + q] * inv);
-          }
-          if (mode == 1) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) res[q] = __fmul_rn(__fsub_rn(res[q], 1.0f), src_mul);
-          }
-          *reinterpret_cast<float4*>(o + 4 * z4) = make_float4(res[0], res[1], res[2], res[3]);
-        }
-      }
-    }
-  }
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2_pack(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_bits(F2 x, int& a, int& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul_rz(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
 }
 
-// Split parameters of a block holding ntot particles (contributions per cell
-// at most ntot * dup): the plane shift s and whether the 32-bit planes apply.
-__device__ __forceinline__ void split_shift(uint32_t ntot, int dup, int E, double scale, int& s, bool& split) {
-  const uint64_t kmax = (uint64_t)ntot * (uint64_t)dup;
-  const int L = kmax ? 64 - __clzll((long long)kmax) : 0;  // kmax < 2^L
-  s = E - 21;
-  if (L + E - 31 > s) s = L + E - 31;
-  if (s < 1) s = 1;
-  split = s <= 22 && s <= 32 - L && scale < 0x1p126;
-}
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }  // -126 <= e <= 127
 
-template <int C, int RX, int RY>
-__global__ void __launch_bounds__(256) scatter_split_kernel(const Rec* __restrict__ rec,
-                                                            const uint32_t* __restrict__ perm,
-                                                            const uint32_t* __restrict__ offs, Mesh3 m,
-                                                            const float* __restrict__ val, int val_sorted,
-                                                            float val_const, const double* __restrict__ scale_dev,
-                                                            int E, int dup, int mode, float src_mul,
-                                                            float* __restrict__ out, uint32_t* __restrict__ status) {
-  constexpr int NSRC = (RX + 1) * (RY + 1);
+constexpr int kRowThreads = 256;
+
+template <int C, int RX, int RY, int NZP, bool EXACT, bool SIGNED>
+__global__ void __launch_bounds__(kRowThreads)
+    scatter_rows_kernel(const Rec* __restrict__ rec, const uint32_t* __restrict__ perm,
+                        const uint32_t* __restrict__ offs, Mesh3 m, FastDiv by_nz, FastDiv by_nby,
+                        const float* __restrict__ val, int val_sorted, float val_const,
+                        const double* __restrict__ scale_dev, double scale_const, int E, int dup, int mode,
+                        float src_mul, float* __restrict__ out, uint32_t* __restrict__ status) {
+  constexpr int CH = RX * RY * NZP;   // cells of one channel, row (lx, ly) at (lx * RY + ly) * NZP
+  constexpr int PLANE = C * CH;       // cells per plane
+  constexpr int GROUPS = PLANE / 4;   // groups of four cells per plane
+  constexpr int T = kRowThreads;
+  static_assert(NZP % 4 == 0, "rows of whole groups");
   if (flagged(status)) return;
-  if (!(*scale_dev == *scale_dev)) {  // NaN scale: a non-finite value
+  const double scale = scale_dev != nullptr ? *scale_dev : scale_const;
+  if (!(scale == scale)) {  // NaN scale: a non-finite value
     if (threadIdx.x == 0) raise_flag(status, kFlagNonFiniteValue);
     return;
   }
-  extern __shared__ __align__(16) unsigned int acc[];  // 8 * RX * RY * C * nz bytes
-  __shared__ uint32_t seg_beg[NSRC], seg_cnt[NSRC], item_pre[NSRC + 1];
-  __shared__ uint32_t s_ntot;
-  const int nby = (m.ny + RY - 1) / RY;
-  const int x0 = (int)(blockIdx.x / nby) * RX, y0 = (int)(blockIdx.x % nby) * RY;
-  const int nz = m.nz;
-  const int cells = RX * RY * C * nz;
+  extern __shared__ __align__(16) unsigned int acc[];  // 2 * PLANE
+  // source segments: [pass][k] for source row x0 + k - 1
+  __shared__ uint32_t s_beg[2][RX + 1], s_cnt[2][RX + 1], s_row[2][RX + 1];
+  const int tid = threadIdx.x;
+  const int nz = EXACT ? NZP : m.nz, nz4 = (nz + 3) >> 2;
+  int x0, y0;
+  {
+    const uint32_t bx = div_by(blockIdx.x, by_nby);
+    x0 = (int)bx * RX;
+    y0 = (int)(blockIdx.x - bx * (uint32_t)((m.ny + RY - 1) / RY)) * RY;
+  }
+  const int rxe = RX == 1 ? 1 : min(RX, m.nx - x0), rye = RY == 1 ? 1 : min(RY, m.ny - y0);  // rows in the mesh
+  if (tid < 2 * (RX + 1)) {
+    const int pass = tid > RX, k = tid - pass * (RX + 1);
+    uint32_t b = 0, c = 0, row = 0;
+    if (k - 1 < rxe && (pass == 0 || y0 == 0)) {
+      const int x = k == 0 ? (x0 == 0 ? m.nx - 1 : x0 - 1) : x0 + k - 1;
+      row = (uint32_t)((int64_t)x * m.ny) + (uint32_t)(pass == 0 ? y0 : m.ny);  // the record's ly = its row - this
+      const int64_t lo = pass == 0 ? (int64_t)row - (y0 > 0) : (int64_t)row - 1;
+      const int64_t hi = pass == 0 ? (int64_t)row + rye : (int64_t)row;
+      b = offs[lo];
+      c = offs[hi] - b;
+    }
+    s_beg[pass][k] = b;
+    s_cnt[pass][k] = c;
+    s_row[pass][k] = EXACT ? row * (uint32_t)NZP : row;
+  }
   {
     uint4* a4 = reinterpret_cast<uint4*>(acc);
-    const int n4 = (2 * cells) >> 2;
-    for (int t = threadIdx.x; t < n4; t += blockDim.x) a4[t] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  if (threadIdx.x < 32) {
-    // source segments and their 32-particle work items (warp prefix sums)
-    const int k = threadIdx.x;
-    uint32_t b = 0, c = 0;
-    if (k < NSRC) {
-      const int px = pmod(x0 + k / (RY + 1) - 1, m.nx), py = pmod(y0 + k % (RY + 1) - 1, m.ny);
-      const int64_t row = (int64_t)px * m.ny + py;
-      b = offs[row];
-      c = offs[row + 1] - b;
-    }
-    uint32_t items = (c + 31) >> 5, tot = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, items, o);
-      const uint32_t z = __shfl_up_sync(0xFFFFFFFFu, tot, o);
-      if (k >= o) {
-        items += y;
-        tot += z;
-      }
-    }
-    if (k < NSRC) {
-      seg_beg[k] = b;
-      seg_cnt[k] = c;
-      item_pre[k + 1] = items;
-    }
-    if (k == 0) item_pre[0] = 0;
-    if (k == 31) s_ntot = tot;
+#pragma unroll 4
+    for (int g = tid; g < 2 * GROUPS; g += T)
+      if (EXACT || g % (NZP / 4) < nz4) a4[g] = make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
-  const uint32_t ntot = s_ntot;
-  const uint32_t nitems = item_pre[NSRC];
-  const double scale = *scale_dev;
+  uint32_t kcell = 0;  // particles that may reach one cell: those of two neighbouring source x
+#pragma unroll
+  for (int k = 0; k < RX; ++k) kcell = max(kcell, s_cnt[0][k] + s_cnt[1][k] + s_cnt[0][k + 1] + s_cnt[1][k + 1]);
   int s;
   bool split;
-  split_shift(ntot, dup, E, scale, s, split);
-  SplitAcc A;
-  A.acc = acc;
-  A.cells = cells;
-  A.y_scale = split ? __fmul_rn((float)scale, __int_as_float((127 - s) << 23)) : 0.f;
-  A.two_s = __int_as_float((127 + s) << 23);
-  unsigned long long* acc64 = reinterpret_cast<unsigned long long*>(acc);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const bool zpow2 = (nz & (nz - 1)) == 0;
-  int k = 0;
-  for (uint32_t it = warp; it < nitems; it += nwarps) {
-    while (it >= item_pre[k + 1]) ++k;
-    const uint32_t j = ((it - item_pre[k]) << 5) + lane;
-    if (j < seg_cnt[k]) {
-      const uint32_t i = seg_beg[k] + j;
-      const Rec r = rec[i];
-      const int cz = zpow2 ? (int)(r.key & (uint32_t)(nz - 1)) : (int)(r.key % (uint32_t)nz);
-      float v[C];
-      if (val != nullptr) {
-        const int64_t src = val_sorted ? (int64_t)i : (int64_t)perm[i];
-#pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = val[src * C + c];
-      } else {
-#pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = val_const;
-      }
-      if (split)
-        deposit_k<C, RX, RY, true>(k, r, v, nz, cz, A, acc64, scale);
-      else
-        deposit_k<C, RX, RY, false>(k, r, v, nz, cz, A, acc64, scale);
-    }
+  {
+    const uint64_t kmax = (uint64_t)kcell * (uint64_t)dup;
+    const int L = kmax ? 64 - __clzll((long long)kmax) : 0;  // kmax < 2^L
+    const int lo = max(max(E - 24, L + E - (SIGNED ? 31 : 32)), SIGNED ? 2 : 1);
+    const int hi = min(SIGNED ? 23 : 24, 32 - L);
+    // half of the bits to each plane where that is allowed, so that the sums
+    // of both stay within the epilogue's short conversion
+    s = max(lo, min(hi, (E + 1) / 2));
+    split = lo <= hi && scale >= 0x1p-50 && scale <= 0x1p100;
   }
-  __syncthreads();
-  split_epilogue<C, RX, RY>(acc, cells, split, s, scale, A.two_s, m, x0, y0, mode, src_mul, out);
-}
+  unsigned long long* acc64 = reinterpret_cast<unsigned long long*>(acc);
+  if (!EXACT && !split) {  // the 64-bit sums lie elsewhere in the rows than the planes cleared above
+    for (int g = tid; g < PLANE; g += T) acc64[g] = 0ull;
+    __syncthreads();
+  }
+  const float y_scale = split ? __fmul_rn((float)scale, pow2f(-s - 49)) : 0.f;
+  const F2 to_h = f2_pack(pow2f(-100), pow2f(-100)), back = f2_pack(-pow2f(100), -pow2f(100));
+  const F2 to_l = f2_pack(pow2f(s - 100), pow2f(s - 100));
+  const int bias = SIGNED ? 1 << (s - 1) : 0;
+  const F2 bias2 = f2_pack(__int_as_float(bias), __int_as_float(bias));
+  int* const planes = reinterpret_cast<int*>(acc);
 
-// One output row per block (1 x 1 tile) with the particle visits of its four
-// source rows flattened over the block's threads: consecutive threads take
-// consecutive records whatever their source row, so every lane is busy (the
-// per-row 32-particle chunks of scatter_split_kernel leave the last chunk of
-// each row part-empty).  A particle of source row (x0 - 1 + sx, y0 - 1 + sy)
-// reaches the row through its corner (1 - sx, 1 - sy).  Same split planes
-// and epilogue, so the output is bit-identical.  Used for three channels,
-// where it measured 14-15% faster at 512^3 / 1024^3.
-template <int C>
-__global__ void __launch_bounds__(256) scatter_flat_kernel(const Rec* __restrict__ rec,
-                                                           const uint32_t* __restrict__ perm,
-                                                           const uint32_t* __restrict__ offs, Mesh3 m,
-                                                           const float* __restrict__ val, int val_sorted,
-                                                           float val_const, const double* __restrict__ scale_dev,
-                                                           int E, int dup, int mode, float src_mul,
-                                                           float* __restrict__ out, uint32_t* __restrict__ status) {
-  if (flagged(status)) return;
-  if (!(*scale_dev == *scale_dev)) {  // NaN scale: a non-finite value
-    if (threadIdx.x == 0) raise_flag(status, kFlagNonFiniteValue);
-    return;
-  }
-  extern __shared__ __align__(16) unsigned int acc[];  // 8 * C * nz bytes
-  __shared__ uint32_t s_beg[4], s_pre[5];
-  const int x0 = (int)(blockIdx.x / m.ny), y0 = (int)(blockIdx.x % m.ny);
-  const int nz = m.nz;
-  const int cells = C * nz;
-  {
-    uint4* a4 = reinterpret_cast<uint4*>(acc);
-    const int n4 = (2 * cells) >> 2;
-    for (int t = threadIdx.x; t < n4; t += blockDim.x) a4[t] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  if (threadIdx.x < 32) {
-    const int k = threadIdx.x;
-    uint32_t b = 0, c = 0;
-    if (k < 4) {
-      const int px = pmod(x0 - 1 + (k >> 1), m.nx), py = pmod(y0 - 1 + (k & 1), m.ny);
-      const int64_t row = (int64_t)px * m.ny + py;
-      b = offs[row];
-      c = offs[row + 1] - b;
-    }
-    uint32_t tot = c;
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
-      const uint32_t z = __shfl_up_sync(0xFFFFFFFFu, tot, o);
-      if (k >= o) tot += z;
-    }
-    if (k < 4) {
-      s_beg[k] = b;
-      s_pre[k + 1] = tot;
-    }
-    if (k == 0) s_pre[0] = 0;
-  }
-  __syncthreads();
-  const uint32_t p1 = s_pre[1], p2 = s_pre[2], p3 = s_pre[3], ntot = s_pre[4];
-  // record index = visit index + (segment begin - segment prefix), mod 2^32
-  const uint32_t d0 = s_beg[0], d1 = s_beg[1] - p1, d2 = s_beg[2] - p2, d3 = s_beg[3] - p3;
-  const double scale = *scale_dev;
-  int s;
-  bool split;
-  split_shift(ntot, dup, E, scale, s, split);
-  SplitAcc A;
-  A.acc = acc;
-  A.cells = cells;
-  A.y_scale = split ? __fmul_rn((float)scale, __int_as_float((127 - s) << 23)) : 0.f;
-  A.two_s = __int_as_float((127 + s) << 23);
-  unsigned long long* acc64 = reinterpret_cast<unsigned long long*>(acc);
-  const bool zpow2 = (nz & (nz - 1)) == 0;
-  for (uint32_t vi = threadIdx.x; vi < ntot; vi += blockDim.x) {
-    const int k = (vi >= p1) + (vi >= p2) + (vi >= p3);
-    const uint32_t i = vi + (k == 0 ? d0 : k == 1 ? d1 : k == 2 ? d2 : d3);
-    const Rec r = rec[i];
-    const int cz = zpow2 ? (int)(r.key & (uint32_t)(nz - 1)) : (int)(r.key % (uint32_t)nz);
-    const int cz1 = cz + 1 == nz ? 0 : cz + 1;
+  // One particle: r its record, at its cell in tile row (sx, ly) of channel 0
+  // (RX, RY == 1: of the one row), dz the step to its upper z cell; x0in ..
+  // y1in: the rows that its lower / upper corners along x and y fall into are
+  // this block's.
+  auto visit = [&](const Rec& r, uint32_t i, int at, int dz, int sx, bool low_y, bool x0in, bool x1in, bool y0in,
+                   bool y1in, auto split_tag) {
+    constexpr bool SPLIT = decltype(split_tag)::value;
     float v[C];
+    int sgn[C], nbias[C];
     if (val != nullptr) {
       const int64_t src = val_sorted ? (int64_t)i : (int64_t)perm[i];
 #pragma unroll
@@ -764,33 +597,187 @@ __global__ void __launch_bounds__(256) scatter_flat_kernel(const Rec* __restrict
 #pragma unroll
       for (int c = 0; c < C; ++c) v[c] = val_const;
     }
-    const float wxy = __fmul_rn(axis_weight(r.fx, 1 - (k >> 1)), axis_weight(r.fy, 1 - (k & 1)));
-    const float w0 = __fmul_rn(wxy, axis_weight(r.fz, 0)), w1 = __fmul_rn(wxy, axis_weight(r.fz, 1));
+    if (SPLIT) {
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const float c0 = __fmul_rn(v[c], w0), c1 = __fmul_rn(v[c], w1);
-      if (split) {
-        A.add(c * nz + cz, c0);
-        A.add(c * nz + cz1, c1);
-      } else {
-        atomicAdd(&acc64[c * nz + cz], (unsigned long long)__double2ll_rn((double)c0 * scale));
-        atomicAdd(&acc64[c * nz + cz1], (unsigned long long)__double2ll_rn((double)c1 * scale));
+      for (int c = 0; c < C; ++c) {
+        if (SIGNED) {
+          sgn[c] = v[c] < 0.f ? -1 : 1;
+          nbias[c] = -bias * sgn[c];
+          v[c] = fabsf(v[c]);
+        }
+        v[c] = __fmul_rn(v[c], y_scale);
       }
     }
-  }
+    const float wx0 = axis_weight(r.fx, 0), wx1 = axis_weight(r.fx, 1);
+    const float wy0 = axis_weight(r.fy, 0), wy1 = axis_weight(r.fy, 1);
+    const F2 wz = f2_pack(axis_weight(r.fz, 0), axis_weight(r.fz, 1));
+    // with one output row along an axis a source row reaches it by one corner
+    constexpr int NX = RX == 1 ? 1 : 2, NY = RY == 1 ? 1 : 2;
+    int* const a0 = planes + at;
+    int* const a1 = a0 + dz;
+#pragma unroll
+    for (int bx = 0; bx < NX; ++bx) {
+      const float wx = RX == 1 ? (sx < 0 ? wx1 : wx0) : (bx ? wx1 : wx0);
+#pragma unroll
+      for (int by = 0; by < NY; ++by) {
+        const float wy = RY == 1 ? (low_y ? wy1 : wy0) : (by ? wy1 : wy0);
+        if (!((bx ? x1in : x0in) && (by ? y1in : y0in))) continue;
+        const float wxy = __fmul_rn(wx, wy);
+        const F2 w = f2_mul(f2_pack(wxy, wxy), wz);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const int o = c * CH + (bx * RY + by) * NZP;
+          const F2 q = f2_mul(f2_pack(v[c], v[c]), w);
+          if (SPLIT) {
+            const F2 t = SIGNED ? f2_mul(q, to_h) : f2_mul_rz(q, to_h);
+            const F2 rem = f2_fma(t, back, q);
+            const F2 u = SIGNED ? f2_fma(rem, to_l, bias2) : f2_mul(rem, to_l);
+            int h0, h1, l0, l1;
+            f2_bits(t, h0, h1);
+            f2_bits(u, l0, l1);
+            if (SIGNED) {
+              h0 *= sgn[c];
+              h1 *= sgn[c];
+              l0 = l0 * sgn[c] + nbias[c];
+              l1 = l1 * sgn[c] + nbias[c];
+            }
+            atomicAdd(a0 + o, h0);
+            atomicAdd(a0 + o + PLANE, l0);
+            atomicAdd(a1 + o, h1);
+            atomicAdd(a1 + o + PLANE, l1);
+          } else {
+            int q0, q1;
+            f2_bits(q, q0, q1);
+            atomicAdd(&acc64[at + o], (unsigned long long)__double2ll_rn((double)__int_as_float(q0) * scale));
+            atomicAdd(&acc64[at + dz + o], (unsigned long long)__double2ll_rn((double)__int_as_float(q1) * scale));
+          }
+        }
+      }
+    }
+  };
+  auto visits = [&](auto split_tag) {
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      // visits before segment k, record index = visit index + dk[k] (mod 2^32)
+      uint32_t pk[RX + 2], dk[RX + 1], bk[RX + 1];
+      pk[0] = 0;
+#pragma unroll
+      for (int k = 0; k <= RX; ++k) {
+        pk[k + 1] = pk[k] + s_cnt[pass][k];
+        dk[k] = s_beg[pass][k] - pk[k];
+        bk[k] = s_row[pass][k];
+      }
+#pragma unroll 1
+      for (uint32_t vi = tid; vi < pk[RX + 1]; vi += T) {
+        uint32_t i = vi + dk[0], b = bk[0];
+        int sx = -1;
+#pragma unroll
+        for (int k = 1; k <= RX; ++k)
+          if (vi >= pk[k]) {
+            i = vi + dk[k];
+            b = bk[k];
+            sx = k - 1;
+          }
+        const Rec r = rec[i];
+        const bool x0in = RX == 1 || sx >= 0, x1in = RX == 1 || sx + 1 < rxe;
+        if (EXACT) {
+          // cell counted from the tile's row 0 of this x: ly * NZP + cz
+          const int lin = (int)(r.key - b);
+          const bool low_y = lin < 0;
+          const bool top = (uint32_t)(lin + 1 + NZP) % (uint32_t)NZP == 0;
+          const int at = (RX == 1 ? 0 : sx * RY * NZP) + (RY == 1 && low_y ? lin + NZP : lin);
+          visit(r, i, at, top ? 1 - NZP : 1, sx, low_y, x0in, x1in, RY == 1 || !low_y,
+                RY == 1 || lin < (rye - 1) * NZP, split_tag);
+        } else {
+          const uint32_t rowk = div_by(r.key, by_nz);
+          const int ly = (int)(rowk - b), cz = (int)(r.key - rowk * (uint32_t)nz);
+          const int at = ((RX == 1 ? 0 : sx * RY) + (RY == 1 ? 0 : ly)) * NZP + cz;
+          visit(r, i, at, cz + 1 == nz ? 1 - nz : 1, sx, ly < 0, x0in, x1in, RY == 1 || ly >= 0,
+                RY == 1 || ly + 1 < rye, split_tag);
+        }
+      }
+    }
+  };
+  if (split)
+    visits(std::true_type{});
+  else
+    visits(std::false_type{});
   __syncthreads();
-  split_epilogue<C, 1, 1>(acc, cells, split, s, scale, A.two_s, m, x0, y0, mode, src_mul, out);
-}
 
-// Block shape of the split scatter for C channels, or false when the mesh
-// rows cannot take the vector epilogue or the accumulator does not fit.
-bool split_block_shape(Mesh3 m, int C, const float* out, int* RX, int* RY) {
-  if (m.nz % 4 != 0 || ((uintptr_t)out & 15) != 0) return false;
-  const int rx = C == 1 ? 2 : 1, ry = C <= 2 ? 2 : 1;
-  if ((int64_t)8 * rx * ry * C * m.nz > 200 * 1024) return false;
-  *RX = rx;
-  *RY = ry;
-  return true;
+  // Epilogue: (float)(sum / scale) as scatter_tile computes it; mode 0 the
+  // density, mode 1 the Poisson source (rho - 1) * src_mul
+  // (gravity.py:628-630).  Plane sums below 2^23 (signed: within 2^22)
+  // convert exactly through the bits of 2^23 + h and one fma forms h 2^s + l
+  // with a single rounding (|sum| < 2^53, so this equals the
+  // double-precision route, which the other cells take).
+  const double inv = __hiloint2double(0x7FE00000 - __double2hiint(scale), 0);  // 1 / scale, a power of two
+  const float invf = (float)inv, two_s = pow2f(split ? s : 0);
+  const bool fconv = split && invf >= 0x1p-126f;
+  constexpr int kOff = SIGNED ? 0x4B400000 : 0x4B000000;
+  const F2 near2 = f2_pack(-__int_as_float(kOff), -__int_as_float(kOff));
+  const F2 two_s2 = f2_pack(two_s, two_s), inv2 = f2_pack(invf, invf);
+  // exact integers in double precision through the bits of 2^52 + h (the
+  // 64-bit integer conversions are ten times as dear); one fma rounds the sum
+  // as the 64-bit conversion would
+  auto as_double = [](int h) {
+    return __hiloint2double(0x43300000, SIGNED ? h ^ (int)0x80000000 : h) - (SIGNED ? 0x1p52 + 0x1p31 : 0x1p52);
+  };
+  auto slow = [&](int a) -> float {
+    if (split) return (float)(fma(as_double(planes[a]), (double)two_s, as_double(planes[PLANE + a])) * inv);
+    return (float)((double)(long long)acc64[a] * inv);
+  };
+  auto pair = [&](int h0, int h1, int l0, int l1, float& a, float& b) {
+    const F2 h = f2_add(f2_pack(__int_as_float(kOff + h0), __int_as_float(kOff + h1)), near2);
+    const F2 l = f2_add(f2_pack(__int_as_float(kOff + l0), __int_as_float(kOff + l1)), near2);
+    int ia, ib;
+    f2_bits(f2_mul(f2_fma(h, two_s2, l), inv2), ia, ib);
+    a = __int_as_float(ia);
+    b = __int_as_float(ib);
+  };
+  auto finish = [&](float x) -> float { return mode == 1 ? __fmul_rn(__fsub_rn(x, 1.0f), src_mul) : x; };
+  const int64_t ystride = nz, xstride = (int64_t)m.ny * nz, cstride = (int64_t)m.nx * xstride;
+  float* const out0 = out + (int64_t)x0 * xstride + (int64_t)y0 * ystride;
+  // output row of accumulator row c * RX * RY + lx * RY + ly (null: not in the mesh)
+  auto row_out = [&](int row) -> float* {
+    const int c = row / (RX * RY), lx = row / RY % RX, ly = row % RY;
+    if (lx >= rxe || ly >= rye) return nullptr;
+    return out0 + c * cstride + lx * xstride + ly * ystride;
+  };
+  if (nz % 4 == 0 && ((uintptr_t)out & 15) == 0) {
+#pragma unroll 2
+    for (int g = tid; g < GROUPS; g += T) {
+      const int row = g / (NZP / 4), z4 = g % (NZP / 4);
+      float* o = row_out(row);
+      if ((!EXACT && z4 >= nz4) || o == nullptr) continue;
+      float res[4];
+      bool done = false;
+      if (fconv) {
+        const int4 hi = reinterpret_cast<const int4*>(acc)[g], lo = reinterpret_cast<const int4*>(acc)[GROUPS + g];
+        const unsigned top = ((kOff + hi.x) ^ 0x4B000000) | ((kOff + hi.y) ^ 0x4B000000) |
+                             ((kOff + hi.z) ^ 0x4B000000) | ((kOff + hi.w) ^ 0x4B000000) |
+                             ((kOff + lo.x) ^ 0x4B000000) | ((kOff + lo.y) ^ 0x4B000000) |
+                             ((kOff + lo.z) ^ 0x4B000000) | ((kOff + lo.w) ^ 0x4B000000);
+        if (top < 0x800000u) {
+          pair(hi.x, hi.y, lo.x, lo.y, res[0], res[1]);
+          pair(hi.z, hi.w, lo.z, lo.w, res[2], res[3]);
+          done = true;
+        }
+      }
+      if (!done) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) res[q] = slow(4 * g + q);
+      }
+      *reinterpret_cast<float4*>(o + 4 * z4) =
+          make_float4(finish(res[0]), finish(res[1]), finish(res[2]), finish(res[3]));
+    }
+  } else {
+    for (int a = tid; a < PLANE; a += T) {
+      const int row = a / NZP, z = a % NZP;
+      float* o = row_out(row);
+      if (z >= nz || o == nullptr) continue;
+      o[z] = finish(slow(a));
+    }
+  }
 }
 
 int fixed_point_exponent(int64_t n) {
@@ -800,76 +787,91 @@ int fixed_point_exponent(int64_t n) {
   return e;
 }
 
-void scatter_block_shape(Mesh3 m, int C, int* RX, int* RY) {
-  // First of 2x2, 1x2, 1x1 output rows whose accumulator fits the budget:
-  // 100 KB for one or two channels, 40 KB for three or four (more resident
-  // blocks beat the extra particle re-reads there; larger blocks measured
-  // slower everywhere).
-  const int64_t budget = (C >= 3 ? 40 : 100) * 1024;
-  static const int shapes[3][2] = {{2, 2}, {1, 2}, {1, 1}};
-  int rx = 1, ry = 1;
-  for (const auto& sh : shapes) {
-    if (ScatterSmem::acc_bytes(sh[0], sh[1], C, m.nz) <= budget) {
-      rx = sh[0];
-      ry = sh[1];
-      break;
-    }
-  }
-  *RX = rx < m.nx ? rx : m.nx;
-  *RY = ry < m.ny ? ry : m.ny;
+// Output rows of one block at row stride nzp: as many as keep the accumulator
+// within 33 KB (six or seven resident blocks).  More rows read each record
+// fewer times (9 / 4 visits per particle at 2 x 2 rows, 25 / 16 at 4 x 4) but
+// leave fewer blocks: one channel, us at 25 / 33 / 49 / 66 KB: 64^3 particles
+// on 128^3 cells 8.7 / 8.7 / 8.7 / 8.8, 256^3 on 512^3 333 / 281 / 280 / 298,
+// 512^3 on 1024^3 2209 / 2190 / 2189 / 2259; three channels on 512^3 822 / 822
+// / 1072 / 1071, five deposits on 256^3 553 / 554 / 667 / 667.
+constexpr int kTileBytes = 33 * 1024;
+constexpr int tile_x(int C, int nzp) {
+  const int row = 8 * C * nzp;
+  return 16 * row <= kTileBytes ? 4 : 4 * row <= kTileBytes ? 2 : 1;
+}
+constexpr int tile_y(int C, int nzp) {
+  const int rows = 8 * C * nzp * tile_x(C, nzp);
+  return 4 * rows <= kTileBytes ? 4 : 2 * rows <= kTileBytes ? 2 : 1;
 }
 
+template <int C, int NZP, bool EXACT, bool SIGNED>
+static int launch_rows(const Rec* rec, const uint32_t* perm, const uint32_t* offs, Mesh3 m, const float* val,
+                       int val_sorted, float val_const, const double* scale_dev, double scale_const, int E, int mode,
+                       float src_mul, float* out, uint32_t* status, cudaStream_t s) {
+  constexpr int RX = tile_x(C, NZP), RY = tile_y(C, NZP);
+  auto k = scatter_rows_kernel<C, RX, RY, NZP, EXACT, SIGNED>;
+  constexpr int smem = 8 * RX * RY * C * NZP;
+  PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
+  const int dup = (m.nx == 1 ? 2 : 1) * (m.ny == 1 ? 2 : 1) * (m.nz == 1 ? 2 : 1);
+  const int64_t nbx = (m.nx + RX - 1) / RX, nby = (m.ny + RY - 1) / RY;
+  k<<<(unsigned)(nbx * nby), kRowThreads, smem, s>>>(rec, perm, offs, m, fast_div((uint32_t)m.nz), fast_div((uint32_t)nby), val,
+                                           val_sorted, val_const, scale_dev, scale_const, E, dup, mode, src_mul, out,
+                                           status);
+  PMB_CUDA_CHECK(cudaGetLastError());
+  return kOk;
+}
+
+// A kernel for the row length itself (usual lengths, one and three channels),
+// else the one of the shortest row stride that holds nz cells.
+template <int C, bool SIGNED, class... Args>
+static int launch_rows_nz(Args... a) {
+  const int nz = std::get<3>(std::tie(a...)).nz;
+  if constexpr (C == 3 || (C == 1 && !SIGNED)) {
+    switch (nz) {
+      case 128: return launch_rows<C, 128, true, SIGNED>(a...);
+      case 192: return launch_rows<C, 192, true, SIGNED>(a...);
+      case 256: return launch_rows<C, 256, true, SIGNED>(a...);
+      case 384: return launch_rows<C, 384, true, SIGNED>(a...);
+      case 512: return launch_rows<C, 512, true, SIGNED>(a...);
+      case 768: return launch_rows<C, 768, true, SIGNED>(a...);
+      case 1024: return launch_rows<C, 1024, true, SIGNED>(a...);
+      default: break;
+    }
+  }
+#define PMB_ROWS(N) \
+  if (nz <= N) return launch_rows<C, N, false, SIGNED>(a...)
+  PMB_ROWS(64);
+  PMB_ROWS(128);
+  PMB_ROWS(192);
+  PMB_ROWS(256);
+  PMB_ROWS(384);
+  PMB_ROWS(512);
+  PMB_ROWS(768);
+  PMB_ROWS(1024);
+  PMB_ROWS(2048);
+  PMB_ROWS(4096);
+#undef PMB_ROWS
+  return kUnsupported;
+}
+
+// scale_dev null: the scale of the constant value val_const.
 int scatter_sorted(const Rec* rec, const uint32_t* perm, const uint32_t* offs, Mesh3 m, int C, const float* val,
                    int val_sorted, float val_const, const double* scale_dev, int mode, float src_mul, float* out,
                    cudaStream_t s, int64_t n, uint32_t* status) {
-  int RX, RY;
-  if (n >= 0 && C >= 1 && C <= 4 && split_block_shape(m, C, out, &RX, &RY)) {
-    const int E = fixed_point_exponent(n);
-    const int dup = (m.nx == 1 ? 2 : 1) * (m.ny == 1 ? 2 : 1) * (m.nz == 1 ? 2 : 1);
-    const int64_t smem = (int64_t)8 * RX * RY * C * m.nz;
-    const unsigned grid = (unsigned)((int64_t)((m.nx + RX - 1) / RX) * ((m.ny + RY - 1) / RY));
-#define PMB_LAUNCH_SPLIT(CC, X, Y)                                                                              \
-  do {                                                                                                          \
-    PMB_CUDA_CHECK(smem_optin((const void*)scatter_split_kernel<CC, X, Y>, 200 * 1024));                       \
-    scatter_split_kernel<CC, X, Y><<<grid, 256, (size_t)smem, s>>>(rec, perm, offs, m, val, val_sorted,         \
-                                                                   val_const, scale_dev, E, dup, mode, src_mul, \
-                                                                   out, status);                                \
-  } while (0)
-    switch (C) {
-      case 1: PMB_LAUNCH_SPLIT(1, 2, 2); break;
-      case 2: PMB_LAUNCH_SPLIT(2, 1, 2); break;
-      case 3:
-        PMB_CUDA_CHECK(smem_optin((const void*)scatter_flat_kernel<3>, 200 * 1024));
-        scatter_flat_kernel<3><<<grid, 256, (size_t)smem, s>>>(rec, perm, offs, m, val, val_sorted, val_const,
-                                                               scale_dev, E, dup, mode, src_mul, out, status);
-        break;
-      default: PMB_LAUNCH_SPLIT(4, 1, 1); break;
-    }
-#undef PMB_LAUNCH_SPLIT
-    PMB_CUDA_CHECK(cudaGetLastError());
-    return kOk;
-  }
-  scatter_block_shape(m, C, &RX, &RY);
-  const int64_t smem = ScatterSmem::acc_bytes(RX, RY, C, m.nz);
-  if (smem > 200 * 1024) return kUnsupported;
-  const int nbx = (m.nx + RX - 1) / RX, nby = (m.ny + RY - 1) / RY;
-  const unsigned grid = (unsigned)((int64_t)nbx * nby);
-#define PMB_LAUNCH_SCATTER(CC)                                                                                   \
-  do {                                                                                                           \
-    PMB_CUDA_CHECK(smem_optin((const void*)scatter_pull_kernel<CC>, 200 * 1024));                              \
-    scatter_pull_kernel<CC><<<grid, 256, (size_t)smem, s>>>(rec, perm, offs, m, RX, RY, val, val_sorted,         \
-                                                             val_const, scale_dev, mode, src_mul, out, status); \
-  } while (0)
+  const int E = fixed_point_exponent(n);
+  const double scale = fixed_point_scale(fixed_point_pow2(n), fabsf(val_const));
+  const bool uns = val == nullptr && val_const >= 0.f;
+#define PMB_SCATTER(CC, SG)                                                                                       \
+  launch_rows_nz<CC, SG>(rec, perm, offs, m, val, val_sorted, val_const, scale_dev, scale, E, mode, src_mul, out, \
+                         status, s)
   switch (C) {
-    case 1: PMB_LAUNCH_SCATTER(1); break;
-    case 2: PMB_LAUNCH_SCATTER(2); break;
-    case 3: PMB_LAUNCH_SCATTER(3); break;
-    case 4: PMB_LAUNCH_SCATTER(4); break;
+    case 1: return uns ? PMB_SCATTER(1, false) : PMB_SCATTER(1, true);
+    case 2: return PMB_SCATTER(2, true);
+    case 3: return PMB_SCATTER(3, true);
+    case 4: return PMB_SCATTER(4, true);
     default: return kUnsupported;
   }
-#undef PMB_LAUNCH_SCATTER
-  PMB_CUDA_CHECK(cudaGetLastError());
-  return kOk;
+#undef PMB_SCATTER
 }
 
 // ---------------------------------------------------------------------------

@@ -103,15 +103,12 @@ extern "C" int pmb_scatter_density_noalloc(const int16_t* pmid, const float* dis
   uint32_t* perm = (uint32_t*)(p + rec_bytes);
   uint32_t* offs = (uint32_t*)(p + rec_bytes + perm_bytes);
   void* bins = p + rec_bytes + perm_bytes + offs_bytes;
-  double* scale = (double*)(p + rec_bytes + perm_bytes + offs_bytes + bins_bytes);
   uint32_t* status = (uint32_t*)(p + rec_bytes + perm_bytes + offs_bytes + bins_bytes + 256);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // bin_particles zeroes the row counts itself; the scale word is rewritten
-  // below, so nothing left over from an earlier call is read.
+  // bin_particles zeroes the row counts itself, so nothing left over from an
+  // earlier call is read.
   st = bin_particles(pmid, const_cast<float*>(disp), nullptr, 0.f, n, m, cell, rec, perm, offs, bins, s, nullptr,
                      nullptr, status);
   if (st != kOk) return st;
-  st = set_double(scale, fixed_point_scale(fixed_point_pow2(n), fabsf(val)), s);
-  if (st != kOk) return st;
-  return scatter_sorted(rec, perm, offs, m, 1, nullptr, 0, val, scale, 0, 1.f, out, s, n, status);
+  return scatter_sorted(rec, perm, offs, m, 1, nullptr, 0, val, nullptr, 0, 1.f, out, s, n, status);
 }

@@ -22,7 +22,8 @@ int bin_particles(const int16_t* pmid, float* disp, const float* vel, float drif
                   const BinShift* shift = nullptr, const uint8_t* valid = nullptr, uint32_t* status = nullptr);
 double fixed_point_pow2(int64_t n);
 int compute_scale(const float* val, int64_t count, int64_t n, double* scale_dev, unsigned int* tmp, cudaStream_t s);
-// n: particles the sort placed (bounds the fixed-point sums)
+// n: particles the sort placed (bounds the fixed-point sums); scale_dev: the
+// fixed-point scale of val (null with a constant value, whose scale is known)
 int scatter_sorted(const Rec* rec, const uint32_t* perm, const uint32_t* offs, Mesh3 m, int C, const float* val,
                    int val_sorted, float val_const, const double* scale_dev, int mode, float src_mul, float* out,
                    cudaStream_t s, int64_t n, uint32_t* status);

@@ -362,14 +362,36 @@ int bin_particles(const int16_t* pmid, float* disp, const float* vel, float drif
 // of two scale = 2^e / 2^ceil(log2 max|val|), e = 62 - ceil(log2(n + 1)) (at
 // most 52), so that the sum of up to n contributions of magnitude <= max|val|
 // cannot overflow and val*w*scale is exact in float.
-__global__ void absmax_kernel(const float* __restrict__ v, int64_t count, unsigned int* __restrict__ out) {
+// Four values a load where they are aligned; one atomic a block, and only if
+// it raises the maximum (an atomic per warp on the one word was the bound: 24
+// us for 3.2 M values, now 5; 49 -> 36 us for 50 M).
+__global__ void __launch_bounds__(256) absmax_kernel(const float* __restrict__ v, int64_t count,
+                                                     unsigned int* __restrict__ out) {
+  __shared__ float sh[8];
+  const float inf = __int_as_float(0x7f800000);
   float mx = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-    float a = fabsf(v[i]);
-    if (a > mx || a != a) mx = (a != a) ? __int_as_float(0x7f800000) : a;
+  auto take = [&](float x) {
+    const float a = fabsf(x);
+    if (a > mx || a != a) mx = (a != a) ? inf : a;
+  };
+  const int64_t step = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t n4 = ((uintptr_t)v & 15) == 0 ? count >> 2 : 0;
+  for (int64_t i = t; i < n4; i += step) {
+    const float4 x = reinterpret_cast<const float4*>(v)[i];
+    take(x.x);
+    take(x.y);
+    take(x.z);
+    take(x.w);
   }
+  for (int64_t i = 4 * n4 + t; i < count; i += step) take(v[i]);
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(mx));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, sh[w]);
+    const unsigned int bits = __float_as_uint(mx);
+    if (bits > *reinterpret_cast<volatile unsigned int*>(out)) atomicMax(out, bits);
+  }
 }
 
 __global__ void scale_from_absmax_kernel(const unsigned int* __restrict__ bits, double pow2e, double* __restrict__ scale) {
@@ -395,9 +417,9 @@ double fixed_point_pow2(int64_t n) {
 int compute_scale(const float* val, int64_t count, int64_t n, double* scale_dev, unsigned int* tmp, cudaStream_t s) {
   PMB_CUDA_CHECK(cudaMemsetAsync(tmp, 0, sizeof(unsigned int), s));
   if (count > 0) {
-    int blocks = (int)((count + 255) / 256);
-    if (blocks > 4096) blocks = 4096;
-    absmax_kernel<<<blocks, 256, 0, s>>>(val, count, tmp);
+    int64_t blocks = (count + 1023) / 1024;
+    if (blocks > 148 * 8) blocks = 148 * 8;
+    absmax_kernel<<<(unsigned)blocks, 256, 0, s>>>(val, count, tmp);
   }
   scale_from_absmax_kernel<<<1, 1, 0, s>>>(tmp, fixed_point_pow2(n), scale_dev);
   PMB_CUDA_CHECK(cudaGetLastError());
@@ -1054,57 +1076,81 @@ __global__ void __launch_bounds__(256) gather_staged_kernel(const Rec* __restric
 // Direct gather with two particles per thread: both particles' 8C corner
 // loads are issued before either sum, doubling the loads in flight of this
 // latency-bound kernel (10% faster on clustered particles at 512^3, same
-// arithmetic per particle as gather_one).
+// arithmetic per particle as gather_one).  The results go through shared
+// memory, so that consecutive threads store consecutive components: the
+// stores follow the particles' own order, and a store per component from the
+// thread that computed it sends C partial sectors per particle to L2, which
+// this kernel keeps busiest: 522 -> 433 us (256^3 clustered particles on 512^3), 4.85
+// -> 4.11 ms (512^3 on 1024^3), 1.28 -> 0.90 ms (256^3 uniform).  A warp's
+// results through its own part, without the block's barrier, measured 452 us
+// and 4.46 ms.
+constexpr int kGatherThreads = 256;
+constexpr int kGatherTile = 2 * kGatherThreads;
+constexpr int kGatherWarps = kGatherThreads / 32;
+
 template <int C>
-__global__ void __launch_bounds__(256) gather_kernel_x2(const Rec* __restrict__ rec, const uint32_t* __restrict__ perm,
-                                                        int64_t n, Mesh3 m, const float* __restrict__ mesh,
-                                                        float* __restrict__ out, float* __restrict__ vel, float kick,
-                                                        float kick2, const uint32_t* __restrict__ status) {
-  const int64_t i0 = (int64_t)blockIdx.x * (2 * blockDim.x) + threadIdx.x;
-  const int64_t i1 = i0 + blockDim.x;
-  if (i0 >= n || flagged(status)) return;
-  const bool two = i1 < n;
-  // masked particles (trailing records) interpolate from cell 0 and write zero
-  bool mk0, mk1;
-  const Rec r0 = unmasked_or_origin(rec[i0], &mk0);
-  const Rec r1 = two ? unmasked_or_origin(rec[i1], &mk1) : r0;
-  if (!two) mk1 = mk0;
-  Corners k0, k1;
-  corners_of(r0, m, k0);
-  corners_of(r1, m, k1);
-  const uint32_t s0 = perm[i0], s1 = two ? perm[i1] : s0;
-  // velocities of the folded kicks, loaded ahead of the corner loads so their
-  // latency (particle-order addresses) overlaps them instead of following
-  // each channel's sum
-  float u0[C], u1[C];
-  if (vel != nullptr) {
+__global__ void __launch_bounds__(kGatherThreads)
+    gather_kernel_x2(const Rec* __restrict__ rec, const uint32_t* __restrict__ perm, int64_t n, Mesh3 m,
+                     const float* __restrict__ mesh, float* __restrict__ out, float* __restrict__ vel, float kick,
+                     float kick2, const uint32_t* __restrict__ status) {
+  __shared__ float s_val[kGatherTile * C];
+  __shared__ uint32_t s_dst[kGatherTile];
+  __shared__ bool s_masked[kGatherTile];
+  if (flagged(status)) return;
+  const int64_t base = (int64_t)blockIdx.x * kGatherTile;
+  const int cnt = n - base < kGatherTile ? (int)(n - base) : kGatherTile;
+  const int t0 = threadIdx.x, t1 = t0 + kGatherThreads;
+  const int64_t cells = m.cells();
+  if (t0 < cnt) {
+    const int64_t i0 = base + t0, i1 = t1 < cnt ? base + t1 : i0;
+    // masked particles (trailing records) interpolate from cell 0 and give zero
+    bool mk0, mk1;
+    const Rec r0 = unmasked_or_origin(rec[i0], &mk0);
+    const Rec r1 = unmasked_or_origin(rec[i1], &mk1);
+    Corners k0, k1;
+    corners_of(r0, m, k0);
+    corners_of(r1, m, k1);
+    s_dst[t0] = perm[i0];
+    s_dst[t1] = perm[i1];
+    s_masked[t0] = mk0;
+    s_masked[t1] = mk1;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-      u0[c] = vel[(int64_t)s0 * C + c];
-      u1[c] = vel[(int64_t)s1 * C + c];
+      const float* mc = mesh + (int64_t)c * cells;
+      float v0[8], v1[8];
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        v0[b] = __ldg(mc + k0.idx[b]);
+        v1[b] = __ldg(mc + k1.idx[b]);
+      }
+      float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        a0 = __fadd_rn(a0, __fmul_rn(v0[b], k0.w[b]));
+        a1 = __fadd_rn(a1, __fmul_rn(v1[b], k1.w[b]));
+      }
+      s_val[t0 * C + c] = mk0 ? 0.f : a0;
+      s_val[t1 * C + c] = mk1 ? 0.f : a1;
     }
   }
-  const int64_t cells = m.cells();
+  __syncthreads();
+  int64_t at[2 * C];
+  float u[2 * C];
 #pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const float* mc = mesh + (int64_t)c * cells;
-    float v0[8], v1[8];
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      v0[b] = __ldg(mc + k0.idx[b]);
-      v1[b] = __ldg(mc + k1.idx[b]);
+  for (int q = 0; q < 2 * C; ++q) {
+    const int j = t0 + q * kGatherThreads, p = j / C;
+    if (p < cnt) {
+      at[q] = (int64_t)s_dst[p] * C + (j - p * C);
+      if (vel != nullptr) u[q] = vel[at[q]];
     }
-    float a0 = 0.f, a1 = 0.f;
+  }
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      a0 = __fadd_rn(a0, __fmul_rn(v0[b], k0.w[b]));
-      a1 = __fadd_rn(a1, __fmul_rn(v1[b], k1.w[b]));
-    }
-    if (out != nullptr) out[(int64_t)s0 * C + c] = mk0 ? 0.f : a0;
-    if (vel != nullptr && !mk0) vel[(int64_t)s0 * C + c] = kicked(u0[c], a0, kick, kick2);
-    if (two) {
-      if (out != nullptr) out[(int64_t)s1 * C + c] = mk1 ? 0.f : a1;
-      if (vel != nullptr && !mk1) vel[(int64_t)s1 * C + c] = kicked(u1[c], a1, kick, kick2);
+  for (int q = 0; q < 2 * C; ++q) {
+    const int j = t0 + q * kGatherThreads, p = j / C;
+    if (p < cnt) {
+      const float a = s_val[j];
+      if (out != nullptr) out[at[q]] = a;
+      if (vel != nullptr && !s_masked[p]) vel[at[q]] = kicked(u[q], a, kick, kick2);
     }
   }
 }
@@ -1169,8 +1215,8 @@ int gather_sorted(const Rec* rec, const uint32_t* perm, const uint32_t* offs, in
   const int th = 256;
   const unsigned g = (unsigned)((n + th - 1) / th);
   if (C == 3) {
-    gather_kernel_x2<3><<<(unsigned)((n + 2 * th - 1) / (2 * th)), th, 0, s>>>(rec, perm, n, m, mesh, out, vel, kick,
-                                                                              kick2, status);
+    gather_kernel_x2<3><<<(unsigned)((n + kGatherTile - 1) / kGatherTile), kGatherThreads, 0, s>>>(
+        rec, perm, n, m, mesh, out, vel, kick, kick2, status);
     PMB_CUDA_CHECK(cudaGetLastError());
     return kOk;
   }
@@ -1212,16 +1258,50 @@ int wait_timeouts(unsigned int* count) {
 // adjoint's val cotangent, scatter.py:372-373) and u_sorted[i, c] =
 // u[src, c] (the weights in sorted order, so a following scatter of u reads
 // them coalesced instead of through the permutation).
-// Per-particle body shared by the direct and staged kernels; fetch(c, b)
-// returns channel c of corner b (bit a of b: +1 along axis a).  With
-// accumulate, dprev (if given) holds disp_cot[src] loaded by the caller ahead
-// of the corner loads.
-template <int C, class Fetch>
-__device__ __forceinline__ void interp_grad_one(const Rec& r, uint32_t src, int64_t i, const Fetch& fetch,
-                                                const float* __restrict__ u, float u_const, float cell, int accumulate,
-                                                float* __restrict__ disp_cot, float* __restrict__ wsum,
-                                                float* __restrict__ u_sorted, const float* dprev = nullptr,
-                                                bool masked = false) {
+// Raveled index of a record's corner b in 32-bit arithmetic modulo 2^32 (a mesh
+// has fewer cells than that): the lower cell and its steps to the upper one.
+struct Steps {
+  uint32_t key, dx, dy, dz;
+  __device__ __forceinline__ uint32_t at(int b) const {
+    return key + ((b & 1) ? dx : 0u) + ((b & 2) ? dy : 0u) + ((b & 4) ? dz : 0u);
+  }
+};
+
+__device__ __forceinline__ Steps steps_of(uint32_t key, Mesh3 m) {
+  const uint32_t nz = (uint32_t)m.nz, ny = (uint32_t)m.ny, plane = ny * nz;
+  uint32_t cx, cy, cz;
+  if (((nz & (nz - 1)) | (ny & (ny - 1))) == 0) {  // shifts instead of divisions
+    const int lz = __ffs(nz) - 1, ly = __ffs(ny) - 1;
+    cz = key & (nz - 1);
+    cy = (key >> lz) & (ny - 1);
+    cx = key >> (lz + ly);
+  } else {
+    const uint32_t row = key / nz;
+    cz = key - row * nz;
+    cx = row / ny;
+    cy = row - cx * ny;
+  }
+  Steps k;
+  k.key = key;
+  k.dx = cx + 1 == (uint32_t)m.nx ? 0u - cx * plane : plane;
+  k.dy = cy + 1 == ny ? 0u - cy * nz : nz;
+  k.dz = cz + 1 == nz ? 0u - cz : 1u;
+  return k;
+}
+
+// sum_b v_b w_b in the order of gather_one.
+__device__ __forceinline__ float corner_sum(const Rec& r, const float (&v)[8]) {
+  float a = 0.f;
+#pragma unroll
+  for (int b = 0; b < 8; ++b)
+    a = __fadd_rn(a, __fmul_rn(v[b], __fmul_rn(__fmul_rn(axis_weight(r.fx, b & 1), axis_weight(r.fy, (b >> 1) & 1)),
+                                               axis_weight(r.fz, (b >> 2) & 1))));
+  return a;
+}
+
+// (sum_b inner_b * grad w_b) / cell of one particle, inner_b the weighted sum
+// of the channels at corner b (bit a of b: +1 along axis a).
+__device__ __forceinline__ void position_term(const Rec& r, const float (&inner)[8], float cell, float (&g)[3]) {
   const float f[3] = {r.fx, r.fy, r.fz};
   float wa[3][2], sg[3][2];
 #pragma unroll
@@ -1231,61 +1311,71 @@ __device__ __forceinline__ void interp_grad_one(const Rec& r, uint32_t src, int6
     sg[a][0] = axis_sign(f[a], 0);
     sg[a][1] = axis_sign(f[a], 1);
   }
-  float uu[C];
+  g[0] = g[1] = g[2] = 0.f;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const int bx = b & 1, by = (b >> 1) & 1, bz = (b >> 2) & 1;
+    // grad_i = sign_i * w_{i+1} * w_{i+2} (enmesh.py:155-160)
+    const float gx = __fmul_rn(__fmul_rn(sg[0][bx], wa[1][by]), wa[2][bz]);
+    const float gy = __fmul_rn(__fmul_rn(sg[1][by], wa[2][bz]), wa[0][bx]);
+    const float gz = __fmul_rn(__fmul_rn(sg[2][bz], wa[0][bx]), wa[1][by]);
+    g[0] = __fadd_rn(g[0], __fmul_rn(inner[b], gx));
+    g[1] = __fadd_rn(g[1], __fmul_rn(inner[b], gy));
+    g[2] = __fadd_rn(g[2], __fmul_rn(inner[b], gz));
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) g[a] = __fdiv_rn(g[a], cell);
+}
+
+// Sums of one particle: g the position term, ws the interpolated values;
+// fetch(c, b) returns channel c of corner b.
+template <int C, class Fetch>
+__device__ __forceinline__ void interp_grad_sums(const Rec& r, const Fetch& fetch, const float (&uu)[C], float cell,
+                                                 float (&g)[3], float (&ws)[C]) {
+  float inner[8];
+#pragma unroll
+  for (int c = 0; c < C; ++c) ws[c] = 0.f;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const float w = __fmul_rn(__fmul_rn(axis_weight(r.fx, b & 1), axis_weight(r.fy, (b >> 1) & 1)),
+                              axis_weight(r.fz, (b >> 2) & 1));
+    inner[b] = 0.f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const float mv = fetch(c, b);
+      inner[b] = __fadd_rn(inner[b], __fmul_rn(uu[c], mv));
+      ws[c] = __fadd_rn(ws[c], __fmul_rn(mv, w));
+    }
+  }
+  position_term(r, inner, cell, g);
+}
+
+// One particle's loads, sums and stores in the kernels that handle one at a time.
+template <int C, class Fetch>
+__device__ __forceinline__ void interp_grad_one(const Rec& r, uint32_t src, int64_t i, const Fetch& fetch,
+                                                const float* __restrict__ u, float u_const, float cell, int accumulate,
+                                                float* __restrict__ disp_cot, float* __restrict__ wsum,
+                                                float* __restrict__ u_sorted, bool masked = false) {
+  float uu[C], g[3], ws[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) uu[c] = u ? u[(int64_t)src * C + c] : u_const;
   if (u_sorted != nullptr) {
 #pragma unroll
     for (int c = 0; c < C; ++c) u_sorted[i * C + c] = uu[c];
   }
-  float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-  float ws[C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) ws[c] = 0.f;
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const int bx = b & 1, by = (b >> 1) & 1, bz = (b >> 2) & 1;
-    float inner = 0.f;
-    const float w = __fmul_rn(__fmul_rn(wa[0][bx], wa[1][by]), wa[2][bz]);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const float mv = fetch(c, b);
-      inner = __fadd_rn(inner, __fmul_rn(uu[c], mv));
-      ws[c] = __fadd_rn(ws[c], __fmul_rn(mv, w));
-    }
-    // grad_i = sign_i * w_{i+1} * w_{i+2} (enmesh.py:155-160)
-    const float gx = __fmul_rn(__fmul_rn(sg[0][bx], wa[1][by]), wa[2][bz]);
-    const float gy = __fmul_rn(__fmul_rn(sg[1][by], wa[2][bz]), wa[0][bx]);
-    const float gz = __fmul_rn(__fmul_rn(sg[2][bz], wa[0][bx]), wa[1][by]);
-    g0 = __fadd_rn(g0, __fmul_rn(inner, gx));
-    g1 = __fadd_rn(g1, __fmul_rn(inner, gy));
-    g2 = __fadd_rn(g2, __fmul_rn(inner, gz));
-  }
-  g0 = __fdiv_rn(g0, cell);
-  g1 = __fdiv_rn(g1, cell);
-  g2 = __fdiv_rn(g2, cell);
+  interp_grad_sums<C>(r, fetch, uu, cell, g, ws);
   float* dc = disp_cot + 3 * (int64_t)src;
-  if (masked) {
-    // a masked particle takes no adjoint: zero, or unchanged when accumulating
-    if (!accumulate) dc[0] = dc[1] = dc[2] = 0.f;
-    if (wsum != nullptr) {
+  // a masked particle takes no adjoint: zero, or unchanged when accumulating
 #pragma unroll
-      for (int c = 0; c < C; ++c) wsum[(int64_t)src * C + c] = 0.f;
-    }
-    return;
-  }
-  if (accumulate) {
-    dc[0] = __fadd_rn(dprev ? dprev[0] : dc[0], g0);
-    dc[1] = __fadd_rn(dprev ? dprev[1] : dc[1], g1);
-    dc[2] = __fadd_rn(dprev ? dprev[2] : dc[2], g2);
-  } else {
-    dc[0] = g0;
-    dc[1] = g1;
-    dc[2] = g2;
+  for (int a = 0; a < 3; ++a) {
+    if (!accumulate)
+      dc[a] = masked ? 0.f : g[a];
+    else if (!masked)
+      dc[a] = __fadd_rn(dc[a], g[a]);
   }
   if (wsum != nullptr) {
 #pragma unroll
-    for (int c = 0; c < C; ++c) wsum[(int64_t)src * C + c] = ws[c];
+    for (int c = 0; c < C; ++c) wsum[(int64_t)src * C + c] = masked ? 0.f : ws[c];
   }
 }
 
@@ -1303,54 +1393,110 @@ __global__ void interp_grad_kernel(const Rec* __restrict__ rec, const uint32_t* 
   corners_of(r, m, k);
   const int64_t cells = m.cells();
   auto fetch = [&](int c, int b) { return __ldg(mesh + (int64_t)c * cells + k.idx[b]); };
-  interp_grad_one<C>(r, perm[i], i, fetch, u, u_const, cell, accumulate, disp_cot, wsum, u_sorted, nullptr, mk);
+  interp_grad_one<C>(r, perm[i], i, fetch, u, u_const, cell, accumulate, disp_cot, wsum, u_sorted, mk);
 }
 
-// Two particles per thread, as gather_kernel_x2.
+// Two particles per thread with the weights and the cotangents carried by
+// component through the warp's shared memory, as gather_kernel_x2; the channels
+// are summed one after another at each corner, so that one channel's corner
+// values are held at a time.  256^3 clustered particles on 512^3: three
+// channels 949 -> 721 us (80 registers, three blocks; 64 registers spill: 782),
+// one channel 805 -> 449 us accumulating and 360 -> 266 us not (64 registers).
 template <int C>
-__global__ void __launch_bounds__(256) interp_grad_kernel_x2(const Rec* __restrict__ rec,
-                                                             const uint32_t* __restrict__ perm, int64_t n, Mesh3 m,
-                                                             const float* __restrict__ mesh,
-                                                             const float* __restrict__ u, float u_const, float cell,
-                                                             int accumulate, float* __restrict__ disp_cot,
-                                                             float* __restrict__ wsum, float* __restrict__ u_sorted,
-                                                             const uint32_t* __restrict__ status) {
-  const int64_t i0 = (int64_t)blockIdx.x * (2 * blockDim.x) + threadIdx.x;
-  const int64_t i1 = i0 + blockDim.x;
-  if (i0 >= n || flagged(status)) return;
-  const bool two = i1 < n;
-  bool mk0, mk1;
-  const Rec r0 = unmasked_or_origin(rec[i0], &mk0);
-  const Rec r1 = two ? unmasked_or_origin(rec[i1], &mk1) : r0;
-  if (!two) mk1 = mk0;
-  Corners k0, k1;
-  corners_of(r0, m, k0);
-  corners_of(r1, m, k1);
-  const uint32_t s0 = perm[i0], s1 = two ? perm[i1] : s0;
-  // accumulated position cotangents, loaded ahead of the corner loads: read
-  // after each particle's sums, their particle-order latency ran in series
-  float d0[3] = {0.f, 0.f, 0.f}, d1[3] = {0.f, 0.f, 0.f};
-  if (accumulate) {
+__global__ void __launch_bounds__(kGatherThreads, C == 1 ? 4 : 3)
+    interp_grad_kernel_x2(const Rec* __restrict__ rec, const uint32_t* __restrict__ perm, int64_t n, Mesh3 m,
+                          const float* __restrict__ mesh, const float* __restrict__ u, float u_const, float cell,
+                          int accumulate, float* __restrict__ disp_cot, float* __restrict__ wsum,
+                          float* __restrict__ u_sorted, const uint32_t* __restrict__ status) {
+  __shared__ float s_val_all[kGatherWarps][64 * 3];  // weights (C of 3) in, cotangents out
+  __shared__ uint32_t s_dst_all[kGatherWarps][64];
+  __shared__ bool s_masked_all[kGatherWarps][64];
+  if (flagged(status)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* const s_val = s_val_all[warp];
+  uint32_t* const s_dst = s_dst_all[warp];
+  bool* const s_masked = s_masked_all[warp];
+  const int64_t base = (int64_t)blockIdx.x * kGatherTile + warp * 64;
+  if (base >= n) return;
+  const int cnt = n - base < 64 ? (int)(n - base) : 64;
+  const int t0 = lane, t1 = lane + 32;
+  if (t0 < cnt) s_dst[t0] = perm[base + t0];
+  if (t1 < cnt) s_dst[t1] = perm[base + t1];
+  __syncwarp();
+  // Loads in the order in which their results are needed: the accumulated
+  // cotangents (by the lanes that will store them) and the weights, which
+  // follow the permutation, then the first channel's corners; the weights are
+  // passed on once those are on their way.
+  float before[6], wgt[2 * C];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      d0[a] = disp_cot[3 * (int64_t)s0 + a];
-      d1[a] = disp_cot[3 * (int64_t)s1 + a];
-    }
+  for (int q = 0; q < 6; ++q) {
+    const int j = lane + q * 32, p = j / 3;
+    before[q] = accumulate && p < cnt ? disp_cot[(int64_t)s_dst[p] * 3 + (j - 3 * p)] : 0.f;
   }
-  const int64_t cells = m.cells();
-  float v0[C][8], v1[C][8];
 #pragma unroll
-  for (int c = 0; c < C; ++c)
+  for (int q = 0; q < 2 * C; ++q) {
+    const int j = lane + q * 32, p = j / C;
+    wgt[q] = u != nullptr && p < cnt ? u[(int64_t)s_dst[p] * C + (j - C * p)] : u_const;
+  }
+  const bool on = t0 < cnt;
+  const int e0 = on ? t0 : 0, e1 = t1 < cnt ? t1 : e0;
+  bool mk0, mk1;
+  const Rec r0 = unmasked_or_origin(rec[base + e0], &mk0);
+  const Rec r1 = unmasked_or_origin(rec[base + e1], &mk1);
+  const Steps k0 = steps_of(r0.key, m), k1 = steps_of(r1.key, m);
+  const int64_t cells = m.cells();
+  float in0[8], in1[8];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const float* mc = mesh + (int64_t)c * cells;
+    float v0[8], v1[8];
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
-      v0[c][b] = __ldg(mesh + (int64_t)c * cells + k0.idx[b]);
-      v1[c][b] = __ldg(mesh + (int64_t)c * cells + k1.idx[b]);
+      v0[b] = __ldg(mc + k0.at(b));
+      v1[b] = __ldg(mc + k1.at(b));
     }
-  auto f0 = [&](int c, int b) { return v0[c][b]; };
-  interp_grad_one<C>(r0, s0, i0, f0, u, u_const, cell, accumulate, disp_cot, wsum, u_sorted, d0, mk0);
-  if (two) {
-    auto f1 = [&](int c, int b) { return v1[c][b]; };
-    interp_grad_one<C>(r1, s1, i1, f1, u, u_const, cell, accumulate, disp_cot, wsum, u_sorted, d1, mk1);
+    if (c == 0) {
+#pragma unroll
+      for (int q = 0; q < 2 * C; ++q) {
+        const int j = lane + q * 32, p = j / C;
+        if (p < cnt) {
+          s_val[j] = wgt[q];
+          if (u_sorted != nullptr) u_sorted[base * C + j] = wgt[q];
+        }
+      }
+      __syncwarp();
+    }
+    const float u0 = s_val[e0 * C + c], u1 = s_val[e1 * C + c];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      in0[b] = __fadd_rn(c == 0 ? 0.f : in0[b], __fmul_rn(u0, v0[b]));
+      in1[b] = __fadd_rn(c == 0 ? 0.f : in1[b], __fmul_rn(u1, v1[b]));
+    }
+    if (wsum != nullptr && on) {
+      wsum[(int64_t)s_dst[t0] * C + c] = mk0 ? 0.f : corner_sum(r0, v0);
+      if (t1 < cnt) wsum[(int64_t)s_dst[t1] * C + c] = mk1 ? 0.f : corner_sum(r1, v1);
+    }
+  }
+  float g0[3], g1[3];
+  position_term(r0, in0, cell, g0);
+  position_term(r1, in1, cell, g1);
+  __syncwarp();  // the weights are read
+  if (on) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      s_val[t0 * 3 + a] = mk0 ? 0.f : g0[a];
+      s_val[t1 * 3 + a] = mk1 ? 0.f : g1[a];
+    }
+    s_masked[t0] = mk0;
+    s_masked[t1] = mk1;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const int j = lane + q * 32, p = j / 3;
+    // a masked particle takes no adjoint: zero, or unchanged when accumulating
+    if (p < cnt && !(accumulate && s_masked[p]))
+      disp_cot[(int64_t)s_dst[p] * 3 + (j - 3 * p)] = accumulate ? __fadd_rn(before[q], s_val[j]) : s_val[j];
   }
 }
 
@@ -1430,15 +1576,15 @@ int interp_grad_sorted(const Rec* rec, const uint32_t* perm, const uint32_t* off
   }
   const int th = 256;
   const unsigned g = (unsigned)((n + th - 1) / th);
-  const unsigned g2 = (unsigned)((n + 2 * th - 1) / (2 * th));
+  const unsigned g2 = (unsigned)((n + kGatherTile - 1) / kGatherTile);
   if (C == 1) {
-    interp_grad_kernel_x2<1><<<g2, th, 0, s>>>(rec, perm, n, m, mesh, u, u_const, cell, accumulate, disp_cot, wsum,
+    interp_grad_kernel_x2<1><<<g2, kGatherThreads, 0, s>>>(rec, perm, n, m, mesh, u, u_const, cell, accumulate, disp_cot, wsum,
                                                u_sorted, status);
     PMB_CUDA_CHECK(cudaGetLastError());
     return kOk;
   }
   if (C == 3) {
-    interp_grad_kernel_x2<3><<<g2, th, 0, s>>>(rec, perm, n, m, mesh, u, u_const, cell, accumulate, disp_cot, wsum,
+    interp_grad_kernel_x2<3><<<g2, kGatherThreads, 0, s>>>(rec, perm, n, m, mesh, u, u_const, cell, accumulate, disp_cot, wsum,
                                                u_sorted, status);
     PMB_CUDA_CHECK(cudaGetLastError());
     return kOk;

@@ -30,7 +30,7 @@
 // memory by TMA (a ring of S stages, one tile in flight while another is
 // transformed), R1-point DFTs run in registers, twiddles, a transpose through
 // shared memory, R2-point DFTs, and the results are stored from registers.
-// The z passes work on KR = 16 contiguous rows with a bulk copy per tile; the
+// The z passes work on KR contiguous rows with a bulk copy per tile; the
 // real transform of length nz is a complex transform of length nz/2 plus the
 // usual even/odd split.
 //
@@ -57,7 +57,6 @@ namespace {
 
 constexpr int KT = 8;   // columns per column tile
 constexpr int BY = 32;  // y rows per block of the spectral layout
-constexpr int KR = 16;  // rows per z-pass tile
 
 __device__ unsigned int g_fft_timeouts;
 
@@ -908,11 +907,20 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
 // ---------------------------------------------------------------------------
 // z passes (contiguous rows)
 // ---------------------------------------------------------------------------
+// KR rows per tile, T threads and CTAS resident CTAs per SM.  The phases of a
+// tile are separated by barriers, so other CTAs fill the gaps.  M = 512: one
+// CTA of 16 rows filled the shared memory, two of 8 rows take 5.12 -> 4.46 ms
+// (3-channel C2R, 1024^3) and 1.64 -> 1.50 ms (R2C).  M = 128: four CTAs of 8
+// rows and 128 threads against two of 16 and 256 take 703 -> 644 us (14 R2C of
+// a 128^3-particle run) and 902 -> 865 us (C2R); the same at M = 256 is slower
+// (507 -> 554 us) and at M = 64 no faster.
 template <int R1, int R2>
 struct ZGeom {
   static constexpr int M = R1 * R2;  // complex length = nz / 2
   static constexpr int P = M + 8;    // spectral row length
-  static constexpr int T = 256;
+  static constexpr int KR = M == 512 || M == 128 ? 8 : 16;
+  static constexpr int T = M == 128 ? 128 : 256;
+  static constexpr int CTAS = T == 128 ? 4 : 2;
   static constexpr int ROWZ = R2 + 1;
   static constexpr int XP = KR * R1 * ROWZ;  // transpose buffer (float2)
   static constexpr int TW = M + M + 8;       // W_M^k (k < M), W_N^k (k <= M), padded
@@ -953,9 +961,9 @@ __device__ __forceinline__ void load_z_twiddles(const ZArgs& a, float2* tw) {
 
 // Real-to-complex along z: KR rows of nz reals -> KR rows of P complex.
 template <int R1, int R2, int S>
-__global__ void __launch_bounds__(256, 1) z_r2c_kernel(const ZArgs a) {
+__global__ void __launch_bounds__(ZGeom<R1, R2>::T, ZGeom<R1, R2>::CTAS) z_r2c_kernel(const ZArgs a) {
   using G = ZGeom<R1, R2>;
-  constexpr int M = G::M, P = G::P;
+  constexpr int M = G::M, P = G::P, KR = G::KR;
   constexpr int STAGE = KR * M;  // float2
   extern __shared__ __align__(128) float2 smem[];
   float2* xp = smem + S * STAGE;
@@ -1051,9 +1059,9 @@ __global__ void __launch_bounds__(256, 1) z_r2c_kernel(const ZArgs a) {
 
 // Complex-to-real along z: KR rows of P complex -> KR rows of nz reals.
 template <int R1, int R2, int S, bool PR>
-__global__ void __launch_bounds__(256, 1) z_c2r_kernel(const ZArgs a) {
+__global__ void __launch_bounds__(ZGeom<R1, R2>::T, ZGeom<R1, R2>::CTAS) z_c2r_kernel(const ZArgs a) {
   using G = ZGeom<R1, R2>;
-  constexpr int M = G::M, P = G::P;
+  constexpr int M = G::M, P = G::P, KR = G::KR;
   constexpr int STAGE = KR * P;  // float2
   extern __shared__ __align__(128) float2 smem[];
   float2* xp = smem + S * STAGE;
@@ -1224,14 +1232,24 @@ int launch_col_ctas(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
   return kOk;
 }
 
-// One resident CTA per SM (255 registers, three stages) for every pass.  Two
-// CTAs of 128 registers spill in the fused x passes; with the multiplier's
-// tables in shared memory one CTA is faster (1024^3 on B200: x + multiplier
-// 4.07 against 4.53 ms, adjoint 4.02 against 4.45 ms).
+// Resident CTAs per SM of a pass of length L.  The passes that hold one
+// transform at a time fit 128 registers, so two CTAs share an SM and fill each
+// other's barriers: us with one / two, pruned: forward y 151 / 105 (512^3) and
+// 910 / 799 (1024^3), inverse y 140 / 131 (512^3) but 806 / 819 (1024^3), x +
+// multiplier 212 / 194 (512^3, though it spills).  The others spill too much:
+// x + multiplier 1082 / 1402 (1024^3), inverse y into two outputs 331 / 447
+// (512^3), y combine 310 / 437, adjoint x 222 / 302.  Lengths up to 256 run 128
+// threads a CTA, of which two share an SM at any register count.
+constexpr int col_ctas(int mode, int L) {
+  if (L == 1024) return mode == kYFwd ? 2 : 1;
+  if (L == 512) return mode == kYFwd || mode == kYInv || mode == kXGreen ? 2 : 1;
+  return 1;
+}
+
 template <int R1, int R2, int MODE, bool PR>
 int launch_col(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
-  return g_col_ctas == 2 ? launch_col_ctas<R1, R2, MODE, 2, PR>(map, a, s)
-                         : launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
+  const int ctas = g_col_ctas != 0 ? g_col_ctas : col_ctas(MODE, R1 * R2);
+  return ctas == 2 ? launch_col_ctas<R1, R2, MODE, 2, PR>(map, a, s) : launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
 }
 
 template <int MODE, bool PR = false>
@@ -1253,10 +1271,13 @@ int launch_col_len_pr(bool pr, int L, const CUtensorMap& map, const ColArgs& a, 
 }
 
 template <int R1, int R2, bool C2R, bool PR>
-int launch_z(const ZArgs& a, cudaStream_t s) {
+int launch_z(ZArgs a, int batch, cudaStream_t s) {
   using G = ZGeom<R1, R2>;
+  constexpr int KR = G::KR;
   constexpr int stage = C2R ? KR * G::P * 8 : KR * G::M * 8;
   constexpr int S = 2;
+  a.tiles_per_ch = (int)((int64_t)a.nx * a.ny / KR);
+  a.ntiles = a.tiles_per_ch * batch;
   constexpr int smem = S * stage + G::XP * 8 + G::TW * 8 + S * 8;
   auto k = C2R ? z_c2r_kernel<R1, R2, S, PR> : z_r2c_kernel<R1, R2, S>;
   PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
@@ -1267,12 +1288,12 @@ int launch_z(const ZArgs& a, cudaStream_t s) {
 }
 
 template <bool C2R, bool PR>
-int launch_z_len(int M, const ZArgs& a, cudaStream_t s) {
+int launch_z_len(int M, const ZArgs& a, int batch, cudaStream_t s) {
   switch (M) {
-    case 64: return launch_z<8, 8, C2R, PR>(a, s);
-    case 128: return launch_z<16, 8, C2R, PR>(a, s);
-    case 256: return launch_z<16, 16, C2R, PR>(a, s);
-    case 512: return launch_z<32, 16, C2R, PR>(a, s);
+    case 64: return launch_z<8, 8, C2R, PR>(a, batch, s);
+    case 128: return launch_z<16, 8, C2R, PR>(a, batch, s);
+    case 256: return launch_z<16, 16, C2R, PR>(a, batch, s);
+    case 512: return launch_z<32, 16, C2R, PR>(a, batch, s);
     default: set_last_error("pmfft: unsupported z length"); return kUnsupported;
   }
 }
@@ -1350,8 +1371,6 @@ int z_pass(Mesh3 m, int inverse, int batch, const float* in_r, const float2* in_
   a.nx = m.nx;
   a.ny = m.ny;
   a.nz = m.nz;
-  a.tiles_per_ch = (int)(m.rows() / KR);
-  a.ntiles = a.tiles_per_ch * batch;
   a.polls = wait_polls();
   a.prune_base = pr.base;
   a.prune_stride = pr.stride;
@@ -1362,8 +1381,8 @@ int z_pass(Mesh3 m, int inverse, int batch, const float* in_r, const float2* in_
   if (st != kOk) return st;
   // only the inverse reads a pruned spectrum (the forward pass stores whole
   // rows: storing the live columns alone measured slower)
-  if (inverse && pr.base != nullptr) return launch_z_len<true, true>(M, a, s);
-  return inverse ? launch_z_len<true, false>(M, a, s) : launch_z_len<false, false>(M, a, s);
+  if (inverse && pr.base != nullptr) return launch_z_len<true, true>(M, a, batch, s);
+  return inverse ? launch_z_len<true, false>(M, a, batch, s) : launch_z_len<false, false>(M, a, batch, s);
 }
 
 int col_pass(Mesh3 m, int mode, int nbatch, int ch_off, const float2* in, float2* out, SpecTables t, GreenParams g,

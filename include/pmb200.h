@@ -416,6 +416,14 @@ int64_t pmb_lpt_workspace_bytes(int gx, int gy, int gz);
 int pmb_lpt(const void* modes, int gx, int gy, int gz, float spacing, float cell_vol, const float* tables, int order,
             float D1, float V1, float D2, float V2, const int16_t* pmid, float* disp, float* vel, int64_t n,
             float cell, float* fields, int64_t* index_out, void* workspace, int64_t workspace_bytes, void* stream);
+/* pmb_lpt for the regular lattice itself: particle ((i gy) + j) gz + k has the
+ * anchors and offsets of the axis tables (x, y and z one after another, gx + gy
+ * + gz entries), so its anchors, displacement and velocity are written only;
+ * index_out (may be null) gets the particle's own number. */
+int pmb_lpt_lattice(const void* modes, int gx, int gy, int gz, float cell_vol, const float* tables, int order,
+                    float D1, float V1, float D2, float V2, const int16_t* axis_pmid, const float* axis_disp,
+                    int16_t* pmid, float* disp, float* vel, float* fields, int64_t* index_out, void* workspace,
+                    int64_t workspace_bytes, void* stream);
 /* Adjoint of pmb_lpt w.r.t. the modes (the hand-written transpose of
  * lpt.py:379-431; packed d/dRe + i d/dIm convention, the complex conjugate of
  * JAX's gradient convention).  amp (optional) chains through the linear-mode

@@ -95,6 +95,8 @@ _SIGS = {
     "pmb_lpt_workspace_bytes": (c_i64, [c_int, c_int, c_int]),
     "pmb_lpt": (c_int, [c_p, c_int, c_int, c_int, c_f, c_f, c_p, c_int, c_f, c_f, c_f, c_f, c_p, c_p, c_p, c_i64, c_f,
                         c_p, c_p, c_p, c_i64, c_p]),
+    "pmb_lpt_lattice": (c_int, [c_p, c_int, c_int, c_int, c_f, c_p, c_int, c_f, c_f, c_f, c_f, c_p, c_p, c_p, c_p, c_p,
+                                c_p, c_p, c_p, c_i64, c_p]),
     "pmb_lpt_vjp_workspace_bytes": (c_i64, [c_int, c_int, c_int]),
     "pmb_lpt_vjp": (c_int, [c_p, c_int, c_int, c_int, c_f, c_p, c_int, c_f, c_f, c_f, c_f, c_p, c_p, c_p, c_p, c_i64,
                             c_p, c_p, c_p, c_p, c_i64, c_p]),
@@ -194,7 +196,7 @@ def check(status, what):
 
 # Hand-written kernels launched per entry point (cuFFT's own kernels excluded).
 _KERNELS = {
-    "pmb_sort_rows": 5, "pmb_sort_rows_ex": 5, "pmb_cic_general_scatter": 3, "pmb_cic_general_gather": 1,
+    "pmb_sort_rows": 3, "pmb_sort_rows_ex": 3, "pmb_cic_general_scatter": 3, "pmb_cic_general_gather": 1,
     "pmb_cic_general_interp_grad": 1, "pmb_gather_rows": 1, "pmb_gather_rows2": 1, "pmb_interp_grad_rows": 1,
     "pmb_green_gradient": 1, "pmb_interlace_spectra": 1, "pmb_project_density": 1, "pmb_cnn_conv3d": 1,
     "pmb_cnn_conv3d_wgrad": 1, "pmb_cnn_stem_input": 1, "pmb_cnn_residual": 1, "pmb_cnn_residual_adjoint": 1,
@@ -203,7 +205,7 @@ _KERNELS = {
     "pmb_kick_adj": 1, "pmb_kick_adj2": 1, "pmb_kick_adj3": 1, "pmb_drift_cot_adj": 1, "pmb_drift_adj": 1, "pmb_dot": 1,
     "pmb_force": 9, "pmb_force2": 9, "pmb_force_streamed": 14, "pmb_force_vjp": 11, "pmb_force_vjp_presorted": 6, "pmb_sum": 1,
     "pmb_white_noise_nested": 1, "pmb_linear_modes": 1,
-    "pmb_lpt": 4, "pmb_lpt_vjp": 6, "pmb_pk_shells": 1, "pmb_shell_stats": 1, "pmb_pk_shells_adjoint": 1,
+    "pmb_lpt": 4, "pmb_lpt_lattice": 4, "pmb_lpt_vjp": 6, "pmb_pk_shells": 1, "pmb_shell_stats": 1, "pmb_pk_shells_adjoint": 1,
     "pmb_overdensity": 1, "pmb_ens_force": 7, "pmb_ens_step": 9, "pmb_ens_set_step": 1,
     "pmb_force64": 5, "pmb_force64_interlaced": 7, "pmb_force_vjp64_interlaced": 6, "pmb_deposit64": 1, "pmb_axpy64": 1, "pmb_sum64": 1, "pmb_force_vjp64": 4, "pmb_dot64": 1, "pmb_lpt64_ex": 4, "pmb_lpt_vjp64": 6,
     "pmb_scatter_vjp64": 1, "pmb_white_noise_nested64": 1,

@@ -254,6 +254,17 @@ class Configuration:
         d = ((f(8.0) * np.sin(phase)).astype(k.dtype) - np.sin(f(2.0) * phase)).astype(k.dtype)
         return (-(d / f(6.0 * spacing))).astype(k.dtype)
 
+    def lattice_tables(self, device=None):
+        """Device tables of the particle lattice's axes: anchors (int16) and
+        offsets of x, y and z one after another (Particles.lattice_axes)."""
+        device = self.device if device is None else torch.device(device)
+        key = ("lattice", str(device))
+        if key not in self._tables:
+            from .particles import Particles
+            pm, dp = Particles.lattice_axes(self, device)
+            self._tables[key] = (torch.cat(pm), torch.cat(dp))
+        return self._tables[key]
+
     def spectral_tables(self, which="mesh", device=None, green_kernel=0, gradient_kernel=0):
         """Device table [kx ky kz cx cy cz (mx my mz)] for pmb_green_gradient.
 

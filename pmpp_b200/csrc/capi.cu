@@ -801,9 +801,9 @@ int64_t pmb_lpt_workspace_bytes(int gx, int gy, int gz) {
   return lpt_layout(Mesh3{gx, gy, gz}, nullptr, 0, &a, &b, &r, &l, &d, &w);
 }
 
-int pmb_lpt(const void* modes, int gx, int gy, int gz, float spacing, float cell_vol, const float* tables, int order,
-            float D1, float V1, float D2, float V2, const int16_t* pmid, float* disp, float* vel, int64_t n,
-            float cell, float* fields, int64_t* index_out, void* workspace, int64_t workspace_bytes, void* stream) {
+// The gradient fields of both orders from the modes.
+static int lpt_fields(const void* modes, int gx, int gy, int gz, float cell_vol, const float* tables, int order,
+                      float* fields, void* workspace, int64_t workspace_bytes, void* stream) {
   Mesh3 g{gx, gy, gz};
   PMB_REQUIRE(gx > 0 && gy > 0 && gz > 0, "pmb_lpt: bad grid");
   PMB_REQUIRE(order >= 0 && order <= 2, "pmb_lpt: order must be 0, 1 or 2");
@@ -828,7 +828,26 @@ int pmb_lpt(const void* modes, int gx, int gy, int gz, float spacing, float cell
   }
   PMB_TRY(lpt_gradients(pot1, Lh, spec6, g, tables, inv_n, s));
   PMB_TRY(fft_c2r(g, 6, spec6, fields, work, s));
-  return lpt_displace(pmid, disp, vel, n, g, cell, spacing, fields, order, D1, V1, D2, V2, index_out, s);
+  return kOk;
+}
+
+int pmb_lpt(const void* modes, int gx, int gy, int gz, float spacing, float cell_vol, const float* tables, int order,
+            float D1, float V1, float D2, float V2, const int16_t* pmid, float* disp, float* vel, int64_t n,
+            float cell, float* fields, int64_t* index_out, void* workspace, int64_t workspace_bytes, void* stream) {
+  PMB_TRY(lpt_fields(modes, gx, gy, gz, cell_vol, tables, order, fields, workspace, workspace_bytes, stream));
+  return lpt_displace(pmid, disp, vel, n, Mesh3{gx, gy, gz}, cell, spacing, fields, order, D1, V1, D2, V2, index_out,
+                      S(stream));
+}
+
+int pmb_lpt_lattice(const void* modes, int gx, int gy, int gz, float cell_vol, const float* tables, int order,
+                    float D1, float V1, float D2, float V2, const int16_t* axis_pmid, const float* axis_disp,
+                    int16_t* pmid, float* disp, float* vel, float* fields, int64_t* index_out, void* workspace,
+                    int64_t workspace_bytes, void* stream) {
+  PMB_REQUIRE(axis_pmid != nullptr && axis_disp != nullptr && pmid != nullptr && disp != nullptr && vel != nullptr,
+              "pmb_lpt_lattice: null argument");
+  PMB_TRY(lpt_fields(modes, gx, gy, gz, cell_vol, tables, order, fields, workspace, workspace_bytes, stream));
+  return lpt_lattice(axis_pmid, axis_disp, Mesh3{gx, gy, gz}, fields, order, D1, V1, D2, V2, pmid, disp, vel,
+                     index_out, S(stream));
 }
 
 static int64_t lpt_vjp_layout(Mesh3 g, void* ws, int64_t cap, float** cot6, float2** F6, float2** Lhat, float** L,

@@ -25,6 +25,8 @@ int lpt_gradients(const float2* pot1, const float2* L_hat, float2* grads, Mesh3 
 int lpt_displace(const int16_t* pmid, float* disp, float* vel, int64_t n, Mesh3 g, float cell, float spacing,
                  const float* fields, int order, float D1, float V1, float D2, float V2, int64_t* index_out,
                  cudaStream_t s);
+int lpt_lattice(const int16_t* pm, const float* d0, Mesh3 g, const float* fields, int order, float D1, float V1,
+                float D2, float V2, int16_t* pmid, float* disp, float* vel, int64_t* index_out, cudaStream_t s);
 int lpt_field_cot(const int64_t* index, const float* disp_cot, const float* vel_cot, int64_t n, int64_t ng,
                   const float* fields, int order, float D1, float V1, float D2, float V2, float* cot, double* dots,
                   cudaStream_t s);

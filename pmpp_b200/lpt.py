@@ -2,9 +2,9 @@
 
 ``lpt(modes, cosmo, conf)`` builds 1LPT/2LPT displacements and canonical
 velocities on the Lagrangian lattice at conf.a_start from linear modes on the
-particle grid, entirely through the fused C-ABI call pmb_lpt (strain spectra,
-one batched C2R, the quadratic 2LPT source, R2C, six gradient C2Rs,
-sampling).  ``lpt_vjp`` is the hand-written adjoint w.r.t. the modes and the
+particle grid, entirely through the fused C-ABI call pmb_lpt_lattice (strain spectra,
+one batched C2R, the quadratic 2LPT source, R2C, six gradient C2Rs, the
+particles written at their lattice points).  ``lpt_vjp`` is the hand-written adjoint w.r.t. the modes and the
 growth factors.
 """
 from __future__ import annotations
@@ -36,18 +36,22 @@ def lpt_full(modes, cosmo, conf):
     gx, gy, gz = conf.ptcl_grid_shape
     dev = modes.device
     modes = modes.contiguous()
-    ptcl = Particles.gen_grid(conf, vel=True, device=dev)
+    n = conf.ptcl_num
+    axis_pmid, axis_disp = conf.lattice_tables(dev)
+    ptcl = Particles(conf, torch.empty((n, 3), dtype=torch.int16, device=dev),
+                     torch.empty((n, 3), dtype=torch.float32, device=dev),
+                     torch.empty((n, 3), dtype=torch.float32, device=dev))
     fac, dfac = cosmo.lpt_factors(conf.a_start)
     f32 = lambda x: float(np.float32(x))
     D1, V1, D2, V2 = f32(fac[0, 0]), f32(fac[0, 2]), f32(fac[1, 0]), f32(fac[1, 2])
     fields = torch.empty((6, gx, gy, gz), dtype=torch.float32, device=dev)
-    index = torch.empty(len(ptcl), dtype=torch.int64, device=dev)
+    index = torch.empty(n, dtype=torch.int64, device=dev)
     tables = conf.spectral_tables("particle", dev)
     ws = workspace(lib().pmb_lpt_workspace_bytes(gx, gy, gz), dev, "lpt")
-    call("pmb_lpt", modes.data_ptr(), gx, gy, gz, float(conf.ptcl_spacing), float(conf.ptcl_cell_vol),
-         tables.data_ptr(), int(conf.lpt_order), D1, V1, D2, V2, ptcl.pmid.data_ptr(), ptcl.disp.data_ptr(),
-         ptcl.vel.data_ptr(), len(ptcl), float(conf.cell_size), fields.data_ptr(), index.data_ptr(), ws.data_ptr(),
-         ws.numel(), stream_handle(dev))
+    call("pmb_lpt_lattice", modes.data_ptr(), gx, gy, gz, float(conf.ptcl_cell_vol), tables.data_ptr(),
+         int(conf.lpt_order), D1, V1, D2, V2, axis_pmid.data_ptr(), axis_disp.data_ptr(), ptcl.pmid.data_ptr(),
+         ptcl.disp.data_ptr(), ptcl.vel.data_ptr(), fields.data_ptr(), index.data_ptr(), ws.data_ptr(), ws.numel(),
+         stream_handle(dev))
     return LPTResult(ptcl, modes, fields, index, fac, dfac)
 
 

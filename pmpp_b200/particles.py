@@ -94,17 +94,23 @@ class Particles:
             pmid = torch.remainder(pmid, torch.tensor(conf.mesh_shape, dtype=torch.int16, device=pmid.device))
         return cls(conf, pmid, ptcl.disp.to(conf.float_dtype), ptcl.vel, ptcl.acc)
 
-    @classmethod
-    def gen_grid(cls, conf, vel=False, acc=False, device=None):
-        """Uniform Lagrangian lattice (particles.py:615-727, single device):
-        pmid = rint(linspace(0, Mx, nx)), disp = exact integer remainder * cell / n."""
-        device = conf.device if device is None else torch.device(device)
+    @staticmethod
+    def lattice_axes(conf, device):
+        """The lattice's anchors (int16) and offsets along each axis, on the device."""
         pm, dp = [], []
         for sp, sm in zip(conf.ptcl_grid_shape, conf.mesh_shape):
             p = torch.round(torch.linspace(0, sm, sp + 1, dtype=torch.float64, device=device)[:-1]).to(torch.int64)
             d = (torch.arange(sp, device=device, dtype=torch.int64) * sm - p * sp).to(torch.float64) * (conf.cell_size / sp)
             pm.append(p.to(torch.int16))
             dp.append(d.to(conf.float_dtype))
+        return pm, dp
+
+    @classmethod
+    def gen_grid(cls, conf, vel=False, acc=False, device=None):
+        """Uniform Lagrangian lattice (particles.py:615-727, single device):
+        pmid = rint(linspace(0, Mx, nx)), disp = exact integer remainder * cell / n."""
+        device = conf.device if device is None else torch.device(device)
+        pm, dp = cls.lattice_axes(conf, device)
         pmid = torch.stack(torch.meshgrid(*pm, indexing="ij"), dim=-1).reshape(-1, 3).contiguous()
         disp = torch.stack(torch.meshgrid(*dp, indexing="ij"), dim=-1).reshape(-1, 3).contiguous()
         z = torch.zeros_like(disp)

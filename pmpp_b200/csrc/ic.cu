@@ -663,134 +663,233 @@ int lpt_modes_adjoint64(const double2* F1, const double2* FS, const double* amp,
 // ---------------------------------------------------------------------------
 // Power spectrum shells (power_spectrum.py:120-143)
 // ---------------------------------------------------------------------------
-// shell = floor(sqrt(n^2) + 1e-9) clipped, weight = |d|^2 * W^-2p * mult in
-// float (W = product of per-axis sinc(n/M) tables), summed in FP64.
+// shell = floor(sqrt(n^2) + 1e-9) clipped, weight = |d|^2 * W^-2p * mult (W =
+// product of per-axis sinc(n/M) tables), summed in FP64.  n^2 is an integer, so
+// the shell is its integer square root.
+//
+// One warp per (x, y) row.  Along kz the shell never falls, so a warp's 32
+// consecutive modes form runs of equal shells: a segmented shuffle sum leaves
+// one addition per run, into the warp's own copy of the sums (no atomics).  The
+// window and multiplicity along z come from a table per block, the other two
+// axes' window from one quotient per row.  689 -> 395 us for a 512^3 mesh (a
+// power per mode and a shared atomic per mode before), 82 us for the bytes; now
+// bound by the shuffles of the segmented sums.
+constexpr int kPkThreads = 256;
+constexpr int kPkWarps = kPkThreads / 32;
+
+__device__ __forceinline__ int shell_of(long long n2, int num_shells) {
+  long long r;
+  if (n2 < (1ll << 31)) {
+    const unsigned n = (unsigned)n2;
+    unsigned q = (unsigned)sqrtf((float)n);  // off by one at most
+    if (q * q > n) --q;
+    if ((q + 1) * (q + 1) <= n) ++q;
+    r = q;
+  } else {
+    r = (long long)sqrt((double)n2);
+    while (r * r > n2) --r;
+    while ((r + 1) * (r + 1) <= n2) ++r;
+  }
+  return r < num_shells - 1 ? (int)r : num_shells - 1;
+}
+
+// w^-2p
+__device__ __forceinline__ double window_pow(double w, int p) {
+  double x = 1.0;
+  for (int i = 0; i < p; ++i) x *= w * w;
+  return 1.0 / x;
+}
+
+// Table of W_z^-2p (times the rFFT multiplicity with mult) for kz < nzh.
 template <class T>
-__global__ void pk_shells_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                                 int mas_power, int num_shells, double* __restrict__ sums,
-                                 const typename Real<T>::T2* __restrict__ spec_b, double* __restrict__ sums_b,
-                                 double* __restrict__ sums_x) {
-  using R = Real<T>;
-  extern __shared__ double sh[];
-  double* shA = sh;
-  double* shB = sh + num_shells;
-  double* shX = sh + 2 * num_shells;
-  const bool cross = spec_b != nullptr;
-  const int nsh = cross ? 3 * num_shells : num_shells;
-  for (int t = threadIdx.x; t < nsh; t += blockDim.x) sh[t] = 0.0;
-  __syncthreads();
+__device__ __forceinline__ void z_window(double* zf, const T* __restrict__ sz, int nz, int mas_power, bool mult) {
+  const int nzh = nz / 2 + 1;
+  for (int k = threadIdx.x; k < nzh; k += blockDim.x) {
+    const double f = window_pow((double)sz[k], mas_power);
+    zf[k] = mult && !(k == 0 || ((nz % 2 == 0) && k == nzh - 1)) ? 2.0 * f : f;
+  }
+}
+
+// Adds v to hist[shell] for the warp's 32 lanes; equal shells are neighbours.
+__device__ __forceinline__ void add_runs(double v, int shell, double* hist, bool own) {
+  const int lane = threadIdx.x & 31;
+  const int prev = __shfl_up_sync(0xFFFFFFFFu, shell, 1);
+  const unsigned heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || shell != prev);
+  const int head = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if (lane - o >= head) v += y;
+  }
+  if (lane == 31 || (heads >> (lane + 1)) & 1u) {
+    if (own)
+      hist[shell] += v;
+    else
+      atomicAdd(&hist[shell], v);
+  }
+  __syncwarp();
+}
+
+template <class T, bool CROSS>
+__global__ void __launch_bounds__(kPkThreads)
+    pk_shells_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
+                     int mas_power, int num_shells, int copies, double* __restrict__ sums,
+                     const typename Real<T>::T2* __restrict__ spec_b, double* __restrict__ sums_b,
+                     double* __restrict__ sums_x) {
+  using T2 = typename Real<T>::T2;
+  constexpr int NS = CROSS ? 3 : 1;
+  constexpr int UN = 4;  // chunks of 32 modes loaded together
+  extern __shared__ double sh[];  // copies x NS x num_shells, then the z table
+  double* zf = sh + (size_t)copies * NS * num_shells;
+  for (int t = threadIdx.x; t < copies * NS * num_shells; t += kPkThreads) sh[t] = 0.0;
   const T* sx = sinc_tab;
   const T* sy = sx + m.nx;
-  const T* sz = sy + m.ny;
-  const int64_t total = m.half_cells();
+  z_window(zf, sy + m.ny, m.nz, mas_power, true);
+  __syncthreads();
   const int nzh = m.nz / 2 + 1;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (int64_t)gridDim.x * blockDim.x) {
-    const Idx3 q = unravel_half(j, m);
-    const long long mx = fft_mode(q.ix, m.nx), my = fft_mode(q.iy, m.ny), mz = q.iz;
-    const long long n2 = mx * mx + my * my + mz * mz;
-    int shell = (int)floor(sqrt((double)n2) + 1e-9);
-    if (shell > num_shells - 1) shell = num_shells - 1;
-    const T mult = (q.iz == 0 || ((m.nz % 2 == 0) && q.iz == nzh - 1)) ? (T)1 : (T)2;
-    T deconv = (T)1;
-    if (mas_power > 0) {
-      const T w = R::mul(R::mul(sx[q.ix], sy[q.iy]), sz[q.iz]);
-      deconv = R::pow_(w, (T)(-2 * mas_power));
-    }
-    const typename R::T2 a = spec[j];
-    const T pa = R::add(R::mul(a.x, a.x), R::mul(a.y, a.y));
-    atomicAdd(&shA[shell], (double)R::mul(R::mul(pa, deconv), mult));
-    if (cross) {
-      const typename R::T2 b = spec_b[j];
-      const T pb = R::add(R::mul(b.x, b.x), R::mul(b.y, b.y));
-      const T px = R::add(R::mul(a.x, b.x), R::mul(a.y, b.y));
-      atomicAdd(&shB[shell], (double)R::mul(R::mul(pb, deconv), mult));
-      atomicAdd(&shX[shell], (double)R::mul(R::mul(px, deconv), mult));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* hist = sh + (size_t)(warp % copies) * NS * num_shells;
+  const bool own = copies == kPkWarps;
+  const int64_t rows = m.rows();
+  for (int64_t row = (int64_t)blockIdx.x * kPkWarps + warp; row < rows; row += (int64_t)gridDim.x * kPkWarps) {
+    const int ix = (int)(row / m.ny), iy = (int)(row - (int64_t)ix * m.ny);
+    const long long mx = fft_mode(ix, m.nx), my = fft_mode(iy, m.ny), r2 = mx * mx + my * my;
+    const double rf = mas_power > 0 ? window_pow((double)sx[ix] * (double)sy[iy], mas_power) : 1.0;
+    const T2* a = spec + row * nzh;
+    const T2* b = CROSS ? spec_b + row * nzh : nullptr;
+    for (int k0 = lane; k0 - lane < nzh; k0 += 32 * UN) {
+      T2 va[UN], vb[UN];
+#pragma unroll
+      for (int q = 0; q < UN; ++q) {
+        const int k = k0 + 32 * q;
+        va[q] = k < nzh ? a[k] : Real<T>::make2((T)0, (T)0);
+        if (CROSS) vb[q] = k < nzh ? b[k] : Real<T>::make2((T)0, (T)0);
+      }
+#pragma unroll
+      for (int q = 0; q < UN; ++q) {
+        const int k = k0 + 32 * q;
+        if (k - lane >= nzh) break;
+        const int shell = shell_of(r2 + (long long)k * k, num_shells);
+        const double f = k < nzh ? rf * zf[k] : 0.0;
+        const double ar = va[q].x, ai = va[q].y;
+        add_runs((ar * ar + ai * ai) * f, shell, hist, own);
+        if (CROSS) {
+          const double br = vb[q].x, bi = vb[q].y;
+          add_runs((br * br + bi * bi) * f, shell, hist + num_shells, own);
+          add_runs((ar * br + ai * bi) * f, shell, hist + 2 * num_shells, own);
+        }
+      }
     }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < num_shells; t += blockDim.x) {
-    if (shA[t] != 0.0) atomicAdd(&sums[t], shA[t]);
-    if (cross) {
-      if (shB[t] != 0.0) atomicAdd(&sums_b[t], shB[t]);
-      if (shX[t] != 0.0) atomicAdd(&sums_x[t], shX[t]);
-    }
+  for (int t = threadIdx.x; t < NS * num_shells; t += kPkThreads) {
+    double v = 0.0;
+    for (int c = 0; c < copies; ++c) v += sh[(size_t)c * NS * num_shells + t];
+    double* out = t < num_shells ? sums : t < 2 * num_shells ? sums_b : sums_x;
+    if (v != 0.0) atomicAdd(&out[t % num_shells], v);
   }
+}
+
+template <class T, bool CROSS>
+static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
+                            int num_shells, double* sums, const typename Real<T>::T2* spec_b, double* sums_b,
+                            double* sums_x, cudaStream_t s) {
+  // a copy of the sums per warp where that leaves room for two blocks on an SM
+  const int64_t table = 8 * (m.nz / 2 + 1), one = (int64_t)8 * (CROSS ? 3 : 1) * num_shells;
+  int copies = kPkWarps;
+  while (copies > 1 && table + copies * one > 100 * 1024) copies /= 2;
+  const int64_t smem = table + copies * one;
+  if (one > 200 * 1024 || smem > 220 * 1024) return kUnsupported;
+  auto k = pk_shells_kernel<T, CROSS>;
+  PMB_CUDA_CHECK(smem_optin((const void*)k, (int)smem));
+  int64_t per_sm = (220 * 1024) / (smem + 1024);
+  per_sm = per_sm > 8 ? 8 : per_sm < 1 ? 1 : per_sm;
+  int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
+  if (grid > 148 * per_sm) grid = 148 * per_sm;
+  k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, (size_t)smem, s>>>(spec, m, sinc_tab, mas_power, num_shells,
+                                                                      copies, sums, spec_b, sums_b, sums_x);
+  PMB_CUDA_CHECK(cudaGetLastError());
+  return kOk;
 }
 
 int pk_shells(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, double* sums,
               const float2* spec_b, double* sums_b, double* sums_x, cudaStream_t s) {
-  const int nsh = spec_b != nullptr ? 3 * num_shells : num_shells;
-  const size_t smem = sizeof(double) * nsh;
-  if (smem > 200 * 1024) return kUnsupported;
-  PMB_CUDA_CHECK(smem_optin((const void*)pk_shells_kernel<float>, 200 * 1024));
-  int64_t b = (m.half_cells() + 255) / 256;
-  if (b > 148 * 8) b = 148 * 8;
-  pk_shells_kernel<float><<<(unsigned)(b > 0 ? b : 1), 256, smem, s>>>(spec, m, sinc_tab, mas_power, num_shells, sums,
-                                                                       spec_b, sums_b, sums_x);
-  PMB_CUDA_CHECK(cudaGetLastError());
-  return kOk;
+  return spec_b != nullptr
+             ? launch_pk_shells<float, true>(spec, m, sinc_tab, mas_power, num_shells, sums, spec_b, sums_b, sums_x, s)
+             : launch_pk_shells<float, false>(spec, m, sinc_tab, mas_power, num_shells, sums, nullptr, nullptr,
+                                              nullptr, s);
 }
 
 int pk_shells64(const double2* spec, Mesh3 m, const double* sinc_tab, int mas_power, int num_shells, double* sums,
                 cudaStream_t s) {
-  const size_t smem = sizeof(double) * num_shells;
-  if (smem > 200 * 1024) return kUnsupported;
-  PMB_CUDA_CHECK(smem_optin((const void*)pk_shells_kernel<double>, 200 * 1024));
-  int64_t b = (m.half_cells() + 255) / 256;
-  if (b > 148 * 8) b = 148 * 8;
-  pk_shells_kernel<double><<<(unsigned)(b > 0 ? b : 1), 256, smem, s>>>(spec, m, sinc_tab, mas_power, num_shells,
-                                                                        sums, nullptr, nullptr, nullptr);
-  PMB_CUDA_CHECK(cudaGetLastError());
-  return kOk;
+  return launch_pk_shells<double, false>(spec, m, sinc_tab, mas_power, num_shells, sums, nullptr, nullptr, nullptr, s);
 }
 
 // Adjoint of the shell power: given dL/dP_shell (already divided by nmodes and
 // times the normalisation), out = 2 * spec * deconv * w_shell * (1/mult) so
 // that M * irfftn(out) is the real-field cotangent (rfftn^T for the
-// Hermitian-consistent spectrum).
-// T = double: the float64 build's form, with the same operations in double.
+// Hermitian-consistent spectrum; the multiplicity cancels against the 1/mult
+// of the rFFT transpose).  Rows and tables as in pk_shells_kernel: 506 -> 243 us
+// for a 512^3 mesh, 164 us for the bytes.
+// T = double: the float64 build's form.
 template <class T>
-__global__ void pk_shells_adjoint_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m,
-                                         const T* __restrict__ sinc_tab, int mas_power, int num_shells,
-                                         const double* __restrict__ wshell, T post,
-                                         typename Real<T>::T2* __restrict__ out) {
-  using R = Real<T>;
+__global__ void __launch_bounds__(kPkThreads)
+    pk_shells_adjoint_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
+                             int mas_power, int num_shells, const double* __restrict__ wshell, double post,
+                             typename Real<T>::T2* __restrict__ out) {
+  using T2 = typename Real<T>::T2;
+  constexpr int UN = 4;
+  extern __shared__ double zf[];
   const T* sx = sinc_tab;
   const T* sy = sx + m.nx;
-  const T* sz = sy + m.ny;
-  const int64_t total = m.half_cells();
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (int64_t)gridDim.x * blockDim.x) {
-    const Idx3 q = unravel_half(j, m);
-    const long long mx = fft_mode(q.ix, m.nx), my = fft_mode(q.iy, m.ny), mz = q.iz;
-    const long long n2 = mx * mx + my * my + mz * mz;
-    int shell = (int)floor(sqrt((double)n2) + 1e-9);
-    if (shell > num_shells - 1) shell = num_shells - 1;
-    T deconv = (T)1;
-    if (mas_power > 0) {
-      const T w = R::mul(R::mul(sx[q.ix], sy[q.iy]), sz[q.iz]);
-      deconv = R::pow_(w, (T)(-2 * mas_power));
+  z_window(zf, sy + m.ny, m.nz, mas_power, false);
+  __syncthreads();
+  const int nzh = m.nz / 2 + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t rows = m.rows();
+  for (int64_t row = (int64_t)blockIdx.x * kPkWarps + warp; row < rows; row += (int64_t)gridDim.x * kPkWarps) {
+    const int ix = (int)(row / m.ny), iy = (int)(row - (int64_t)ix * m.ny);
+    const long long mx = fft_mode(ix, m.nx), my = fft_mode(iy, m.ny), r2 = mx * mx + my * my;
+    const double rf = 2.0 * post * (mas_power > 0 ? window_pow((double)sx[ix] * (double)sy[iy], mas_power) : 1.0);
+    const T2* a = spec + row * nzh;
+    T2* o = out + row * nzh;
+    for (int k0 = lane; k0 < nzh; k0 += 32 * UN) {
+      T2 v[UN];
+#pragma unroll
+      for (int q = 0; q < UN; ++q)
+        if (k0 + 32 * q < nzh) v[q] = a[k0 + 32 * q];
+#pragma unroll
+      for (int q = 0; q < UN; ++q) {
+        const int k = k0 + 32 * q;
+        if (k < nzh) {
+          const double f = rf * zf[k] * wshell[shell_of(r2 + (long long)k * k, num_shells)];
+          o[k] = Real<T>::make2((T)(v[q].x * f), (T)(v[q].y * f));
+        }
+      }
     }
-    // the multiplicity cancels against the 1/mult of the rFFT transpose
-    const T f = R::mul(R::mul((T)2 * (T)wshell[shell], deconv), post);
-    const typename R::T2 a = spec[j];
-    out[j] = R::make2(R::mul(a.x, f), R::mul(a.y, f));
   }
+}
+
+template <class T>
+static int launch_pk_adjoint(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
+                             int num_shells, const double* wshell, double post, typename Real<T>::T2* out,
+                             cudaStream_t s) {
+  int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
+  if (grid > 148 * 8) grid = 148 * 8;
+  pk_shells_adjoint_kernel<T><<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, 8 * (m.nz / 2 + 1), s>>>(
+      spec, m, sinc_tab, mas_power, num_shells, wshell, post, out);
+  PMB_CUDA_CHECK(cudaGetLastError());
+  return kOk;
 }
 
 int pk_shells_adjoint(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells,
                       const double* wshell, float post, float2* out, cudaStream_t s) {
-  pk_shells_adjoint_kernel<float><<<grid_for(m.half_cells(), 256), 256, 0, s>>>(spec, m, sinc_tab, mas_power,
-                                                                                num_shells, wshell, post, out);
-  PMB_CUDA_CHECK(cudaGetLastError());
-  return kOk;
+  return launch_pk_adjoint<float>(spec, m, sinc_tab, mas_power, num_shells, wshell, (double)post, out, s);
 }
 
 int pk_shells_adjoint64(const double2* spec, Mesh3 m, const double* sinc_tab, int mas_power, int num_shells,
                         const double* wshell, double post, double2* out, cudaStream_t s) {
-  pk_shells_adjoint_kernel<double><<<grid_for(m.half_cells(), 256), 256, 0, s>>>(spec, m, sinc_tab, mas_power,
-                                                                                 num_shells, wshell, post, out);
-  PMB_CUDA_CHECK(cudaGetLastError());
-  return kOk;
+  return launch_pk_adjoint<double>(spec, m, sinc_tab, mas_power, num_shells, wshell, post, out, s);
 }
 
 // Shell mode counts and mean |n| (power_spectrum.py:46-74), FP64.
@@ -838,8 +937,32 @@ __global__ void overdensity_kernel(const T* __restrict__ rho, T* __restrict__ de
     delta[i] = R::sub(R::div(rho[i], mean), (T)1);
 }
 
+// Four cells a load and store, four of those a thread (n % 4 == 0, both
+// 16-byte aligned): 346 -> 213 us for 512^3 cells.
+__global__ void __launch_bounds__(256) overdensity4_kernel(const float4* __restrict__ rho, float4* __restrict__ delta,
+                                                           int64_t n4, const double* __restrict__ total) {
+  const float mean = (float)(*total / (double)(4 * n4));
+  const int64_t i0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+  float4 v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (i0 + q * 256 < n4) v[q] = rho[i0 + q * 256];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    v[q].x = __fsub_rn(__fdiv_rn(v[q].x, mean), 1.f);
+    v[q].y = __fsub_rn(__fdiv_rn(v[q].y, mean), 1.f);
+    v[q].z = __fsub_rn(__fdiv_rn(v[q].z, mean), 1.f);
+    v[q].w = __fsub_rn(__fdiv_rn(v[q].w, mean), 1.f);
+    if (i0 + q * 256 < n4) delta[i0 + q * 256] = v[q];
+  }
+}
+
 int overdensity(const float* rho, float* delta, int64_t n, const double* total, cudaStream_t s) {
-  overdensity_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(rho, delta, n, total);
+  if (n % 4 == 0 && n > 0 && (((uintptr_t)rho | (uintptr_t)delta) & 15) == 0)
+    overdensity4_kernel<<<(unsigned)((n / 4 + 1023) / 1024), 256, 0, s>>>((const float4*)rho, (float4*)delta, n / 4,
+                                                                        total);
+  else
+    overdensity_kernel<float><<<grid_for(n, 256), 256, 0, s>>>(rho, delta, n, total);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }

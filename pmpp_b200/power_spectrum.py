@@ -178,8 +178,8 @@ def pk_loss(ptcl, conf, pk_target, mas="CIC", grad=True, kmax=None):
     """L = mean_s (log P_s / P_target,s)^2 over shells with modes, and dL/d disp.
 
     Forward: scatter -> delta = rho/mean - 1 -> rFFT -> FP64 shell sums.
-    Backward: shell-power adjoint -> C2R -> overdensity adjoint (including the
-    mean) -> scatter adjoint (cic/scatter.py:386-437).  float64 particles take
+    Backward: shell-power adjoint -> C2R -> overdensity adjoint folded into the
+    scatter adjoint (cic/scatter.py:386-437).  float64 particles take
     the float64 build (x64.pk_loss)."""
     if ptcl.disp.dtype == torch.float64:
         from . import x64
@@ -214,14 +214,13 @@ def pk_loss(ptcl, conf, pk_target, mas="CIC", grad=True, kmax=None):
     gspec = torch.empty_like(spec)
     call("pmb_pk_shells_adjoint", spec.data_ptr(), nx, ny, nz, _sinc_tables(conf, dev).data_ptr(), mp, len(w),
          wd.data_ptr(), 1.0, gspec.data_ptr(), s)
-    fw = workspace(lib().pmb_fft_work_bytes(nx, ny, nz, 1), dev, "fft1")
-    dcot = torch.empty((nx, ny, nz), dtype=torch.float32, device=dev)
-    call("pmb_irfft3", nx, ny, nz, 1, gspec.data_ptr(), dcot.data_ptr(), fw.data_ptr(), s)
-    # delta = rho / m - 1 with m = sum(rho)/M:  rho_cot = dcot/m - sum(dcot*rho)/(m^2 M)
-    dd = torch.zeros(1, dtype=torch.float64, device=dev)
-    call("pmb_dot", dcot.data_ptr(), rho.data_ptr(), rho.numel(), dd.data_ptr(), s)
+    # delta = rho / m - 1 with m = sum(rho)/M: rho_cot = (dcot - sum(dcot delta)/M) / m.
+    # The sum is 2 sum_s w_s S_s over the shell sums S_s (gspec is 2 w_s times the
+    # spectrum), so the constant enters as the zero mode and 1 / m as the particle value
+    gspec.view(-1)[:1].fill_(-2.0 * float(np.dot(w, sums.cpu().numpy())) / rho.numel())
     m = float(tot.item()) / rho.numel()
-    shift = float(dd.item()) / (m * m * rho.numel())
-    rho_cot = dcot.mul_(np.float32(1.0 / m)).sub_(np.float32(shift)).unsqueeze(0)
-    disp_cot, _ = sp.interp_grad(rho_cot, u_const=float(conf.mesh_size / conf.ptcl_num))
+    fw = workspace(lib().pmb_fft_work_bytes(nx, ny, nz, 1), dev, "fft1")
+    dcot = torch.empty((1, nx, ny, nz), dtype=torch.float32, device=dev)
+    call("pmb_irfft3", nx, ny, nz, 1, gspec.data_ptr(), dcot.data_ptr(), fw.data_ptr(), s)
+    disp_cot, _ = sp.interp_grad(dcot, u_const=float(conf.mesh_size / conf.ptcl_num) / m)
     return loss, disp_cot

@@ -630,12 +630,19 @@ def gravity(a, ptcl, cosmo, conf, correction=None):
 
 def gravity_vjp(a, ptcl, cosmo, conf, acc_cot, correction=None):
     """Returns (disp_cot, Omega_m_cot) of gravity w.r.t. acc_cot."""
-    acc, F = force(ptcl.pmid, ptcl.disp.clone(), conf, cosmo.Omega_m, a=a, cosmo=cosmo, correction=correction)
+    acc, F = force(ptcl.pmid, ptcl.disp, conf, cosmo.Omega_m, a=a, cosmo=cosmo, correction=correction)
     om_out = []
-    dc = force_vjp(ptcl.pmid, ptcl.disp, conf, cosmo.Omega_m, F, acc_cot.contiguous(), a=a, cosmo=cosmo,
+    acc_cot = acc_cot.contiguous()
+    dc = force_vjp(ptcl.pmid, ptcl.disp, conf, cosmo.Omega_m, F, acc_cot, a=a, cosmo=cosmo,
                    correction=correction, om_out=om_out)
     if om_out:
         return dc, om_out[0]
     om = float(cosmo.Omega_m) if acc.dtype == torch.float64 else _om32(cosmo.Omega_m)
+    if acc.dtype == torch.float32 and acc_cot.dtype == torch.float32 and acc_cot.shape == acc.shape:
+        # products and sum in FP64 in one pass (the elementwise form makes two
+        # double copies first: 0.63 of 9.2 ms at 256^3 particles)
+        d = torch.zeros(1, dtype=torch.float64, device=acc.device)
+        call("pmb_dot", acc_cot.data_ptr(), acc.data_ptr(), acc.numel(), d.data_ptr(), stream_handle(acc.device))
+        return dc, float(d.item()) / om
     om_cot = float((acc_cot.double() * acc.double()).sum()) / om
     return dc, om_cot

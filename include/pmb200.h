@@ -255,7 +255,7 @@ int pmb_project_density(const float* mesh, int nx, int ny, int nz, int axis, int
 
 /* ---------------- hand-written PM FFT passes -------------------------------
  * For meshes whose sides are powers of two (nx, ny in 64..1024, nz in
- * 128..1024) the fused force and its adjoint run their spectral stages as a
+ * 128..1024) or three times one (96, 192, 384, 768) the fused force and its adjoint run their spectral stages as a
  * chain of hand-written passes over a y-blocked half-spectrum layout:
  * channel-major, then rows ((y/32)*nx + x)*32 + y%32 of P = nz/2 + 8 complex
  * values (columns above nz/2 zero).  pmb_pmfft_channel_elems gives the complex

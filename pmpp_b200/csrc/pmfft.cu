@@ -1,4 +1,4 @@
-// Particle-mesh FFT pipeline for power-of-two meshes.
+// Particle-mesh FFT pipeline for meshes of sides 2^a and 3 2^a.
 //
 // The force and its adjoint need, per evaluation, one real-to-complex 3D
 // transform, the Green x gradient multiplier and three complex-to-real
@@ -73,14 +73,16 @@ __device__ __forceinline__ float2 w32(int k) {
 }
 
 // Twiddle tables W_L^k = exp(-2 pi i k / L) (k < L) of every L = 32 .. 2048,
-// table L at offset L - 32, evaluated at compile time into a constant device
+// table L at offset L - 32, then of L = 48 .. 1536, table L at offset kTw3 +
+// L - 48, evaluated at compile time into a constant device
 // array (no fill at run time, so no first-use ordering between streams).
 // Each entry: the quadrant j = floor(4k / L) and the remainder are exact
 // integers, the remainder is folded to an angle b in [0, pi/4], and sin b /
 // cos b come from their Taylor series in double (13 terms; the first omitted
 // term is below 1e-28), then rounded once to float.  Exact zeros carry the
 // signs of sinpi / cospi of -2k/L: sine -0, cosine +0.
-constexpr int kTwTotal = 2048 * 2 - 32;
+constexpr int kTw3 = 2048 * 2 - 32;
+constexpr int kTwTotal = kTw3 + 1536 * 2 - 48;
 
 struct TwiddleTable {
   float2 v[kTwTotal];
@@ -119,6 +121,8 @@ constexpr TwiddleTable make_twiddles() {
   TwiddleTable t{};
   int i = 0;
   for (int L = 32; L <= 2048; L *= 2)
+    for (int k = 0; k < L; ++k) t.v[i++] = twiddle_entry(k, L);
+  for (int L = 48; L <= 1536; L *= 2)
     for (int k = 0; k < L; ++k) t.v[i++] = twiddle_entry(k, L);
   return t;
 }
@@ -176,21 +180,82 @@ __device__ __forceinline__ void dft_stage(float2 (&v)[R]) {
   if constexpr (LEN < R) dft_stage<R, 2 * LEN, INV>(v);
 }
 
-// In-register R-point DFT (R <= 32), natural order in and out; INV uses the
-// conjugate kernel (no scaling).
+// exp(-2 pi i k / R) of a small length as constants of the code.
+template <int R>
+struct SmallTwiddles {
+  float re[R], im[R];
+};
+
+template <int R>
+constexpr SmallTwiddles<R> make_small_twiddles() {
+  SmallTwiddles<R> t{};
+  for (int k = 0; k < R; ++k) {
+    const float2 w = twiddle_entry(k, R);
+    t.re[k] = w.x;
+    t.im[k] = w.y;
+  }
+  return t;
+}
+
+template <int R>
+__device__ __forceinline__ float2 w_small(int k) {
+  constexpr SmallTwiddles<R> t = make_small_twiddles<R>();
+  return make_float2(t.re[k], t.im[k]);
+}
+
+// In-register R-point DFT (R <= 32, 2^a or 3 2^a), natural order in and out;
+// INV uses the conjugate kernel (no scaling).  R = 3 Q: the Q-point DFTs of
+// the three interleaved thirds, twiddles W_R^(b k), and a three-point DFT for
+// every k.
 template <int R, bool INV>
 __device__ __forceinline__ void reg_dft(float2 (&v)[R]) {
-  constexpr int LB = Log2<R>::v;
+  if constexpr (R % 3 == 0) {
+    constexpr int Q = R / 3;
+    constexpr float kHalfSqrt3 = 0.866025403784438646763723170753f;
+    float2 y0[Q], y1[Q], y2[Q];
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int j = bit_reverse(i, LB);
-    if (j > i) {
-      const float2 t = v[i];
-      v[i] = v[j];
-      v[j] = t;
+    for (int i = 0; i < Q; ++i) {
+      y0[i] = v[3 * i];
+      y1[i] = v[3 * i + 1];
+      y2[i] = v[3 * i + 2];
     }
+    reg_dft<Q, INV>(y0);
+    reg_dft<Q, INV>(y1);
+    reg_dft<Q, INV>(y2);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+      float2 b = y1[k], c = y2[k];
+      if (k != 0) {
+        float2 w1 = w_small<R>(k), w2 = w_small<R>(2 * k);
+        if (INV) {
+          w1.y = -w1.y;
+          w2.y = -w2.y;
+        }
+        b = cmul(b, w1);
+        c = cmul(c, w2);
+      }
+      const float2 sum = cadd(b, c), dif = csub(b, c);
+      const float2 t = make_float2(y0[k].x - 0.5f * sum.x, y0[k].y - 0.5f * sum.y);
+      // -i sqrt(3)/2 (b - c), conjugated for the inverse
+      const float2 r = INV ? make_float2(-kHalfSqrt3 * dif.y, kHalfSqrt3 * dif.x)
+                           : make_float2(kHalfSqrt3 * dif.y, -kHalfSqrt3 * dif.x);
+      v[k] = cadd(y0[k], sum);
+      v[k + Q] = cadd(t, r);
+      v[k + 2 * Q] = csub(t, r);
+    }
+  } else {
+    constexpr int LB = Log2<R>::v;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int j = bit_reverse(i, LB);
+      if (j > i) {
+        const float2 t = v[i];
+        v[i] = v[j];
+        v[j] = t;
+      }
+    }
+    dft_stage<R, 2, INV>(v);
   }
-  dft_stage<R, 2, INV>(v);
 }
 
 // Four-step FFT of length A1*A2 over KT columns, first half: the job (n2, c)
@@ -222,6 +287,9 @@ __device__ __forceinline__ void four_step_b(float2 (&u)[A2], const float2* buf, 
   reg_dft<A2, INV>(u);
 }
 
+// Rows per TMA box of a column of length L: at most 256, a divisor of L.
+__host__ __device__ constexpr int col_box_rows(int L) { return L <= 256 ? L : L % 256 == 0 ? 256 : 192; }
+
 template <int R1, int R2>
 struct ColGeom {
   static constexpr int L = R1 * R2;
@@ -231,7 +299,7 @@ struct ColGeom {
   static constexpr int XB = R2 * (R1 * KT + 8);
   static constexpr int BUF0 = TILE > XA ? TILE : XA;
   static constexpr int BUF = BUF0 > XB ? BUF0 : XB;  // float2 per stage
-  static constexpr int BOX = L < 256 ? L : 256;      // rows per TMA box
+  static constexpr int BOX = col_box_rows(L);        // rows per TMA box
 };
 
 // Column pass modes.
@@ -918,7 +986,7 @@ template <int R1, int R2>
 struct ZGeom {
   static constexpr int M = R1 * R2;  // complex length = nz / 2
   static constexpr int P = M + 8;    // spectral row length
-  static constexpr int KR = M == 512 || M == 128 ? 8 : 16;
+  static constexpr int KR = M == 512 || M == 384 || M == 128 ? 8 : 16;
   static constexpr int T = M == 128 ? 128 : 256;
   static constexpr int CTAS = T == 128 ? 4 : 2;
   static constexpr int ROWZ = R2 + 1;
@@ -1176,7 +1244,8 @@ TwiddleState& twiddles() {
 }
 
 int twiddle_table(int L, const float2** out) {
-  if (L < 32 || L > 2048 || (L & (L - 1)) != 0) {
+  const bool p2 = pow2_in(L, 32, 2048), p3 = L % 3 == 0 && pow2_in(L / 3, 16, 512);
+  if (!p2 && !p3) {
     set_last_error("pmfft: unsupported twiddle table length");
     return kUnsupported;
   }
@@ -1190,7 +1259,7 @@ int twiddle_table(int L, const float2** out) {
     PMB_CUDA_CHECK(cudaGetSymbolAddress(&p, g_twiddles));
     it = t.base.emplace(dev, reinterpret_cast<const float2*>(p)).first;
   }
-  *out = it->second + (L - 32);
+  *out = it->second + (p2 ? L - 32 : kTw3 + L - 48);
   return kOk;
 }
 
@@ -1243,19 +1312,30 @@ int launch_col_ctas(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
 constexpr int col_ctas(int mode, int L) {
   if (L == 1024) return mode == kYFwd ? 2 : 1;
   if (L == 512) return mode == kYFwd || mode == kYInv || mode == kXGreen ? 2 : 1;
+  if (L == 384 || L == 768) return mode == kYFwd || mode == kYInv ? 2 : 1;
   return 1;
 }
 
 template <int R1, int R2, int MODE, bool PR>
 int launch_col(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
-  const int ctas = g_col_ctas != 0 ? g_col_ctas : col_ctas(MODE, R1 * R2);
-  return ctas == 2 ? launch_col_ctas<R1, R2, MODE, 2, PR>(map, a, s) : launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
+  constexpr int L = R1 * R2;
+  if constexpr (L == 512 || L == 1024) {  // the lengths at which the two differ
+    const int ctas = g_col_ctas != 0 ? g_col_ctas : col_ctas(MODE, L);
+    if (ctas == 2) return launch_col_ctas<R1, R2, MODE, 2, PR>(map, a, s);
+    return launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
+  } else {
+    return launch_col_ctas<R1, R2, MODE, col_ctas(MODE, L), PR>(map, a, s);
+  }
 }
 
 template <int MODE, bool PR = false>
 int launch_col_len(int L, const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
   switch (L) {
     case 64: return launch_col<8, 8, MODE, PR>(map, a, s);
+    case 96: return launch_col<16, 6, MODE, PR>(map, a, s);
+    case 192: return launch_col<16, 12, MODE, PR>(map, a, s);
+    case 384: return launch_col<32, 12, MODE, PR>(map, a, s);
+    case 768: return launch_col<32, 24, MODE, PR>(map, a, s);
     case 128: return launch_col<16, 8, MODE, PR>(map, a, s);
     case 256: return launch_col<16, 16, MODE, PR>(map, a, s);
     case 512: return launch_col<32, 16, MODE, PR>(map, a, s);
@@ -1290,6 +1370,10 @@ int launch_z(ZArgs a, int batch, cudaStream_t s) {
 template <bool C2R, bool PR>
 int launch_z_len(int M, const ZArgs& a, int batch, cudaStream_t s) {
   switch (M) {
+    case 48: return launch_z<8, 6, C2R, PR>(a, batch, s);
+    case 96: return launch_z<16, 6, C2R, PR>(a, batch, s);
+    case 192: return launch_z<16, 12, C2R, PR>(a, batch, s);
+    case 384: return launch_z<32, 12, C2R, PR>(a, batch, s);
     case 64: return launch_z<8, 8, C2R, PR>(a, batch, s);
     case 128: return launch_z<16, 8, C2R, PR>(a, batch, s);
     case 256: return launch_z<16, 16, C2R, PR>(a, batch, s);
@@ -1319,7 +1403,9 @@ int encode(CUtensorMap* map, int rank, const void* base, const cuuint64_t* dims,
 }  // namespace
 
 bool pmfft_supported(Mesh3 m) {
-  return pow2_in(m.nx, 64, 1024) && pow2_in(m.ny, 64, 1024) && pow2_in(m.nz, 128, 1024);
+  const auto third = [](int v) { return v % 3 == 0 && pow2_in(v / 3, 32, 256); };  // 96, 192, 384, 768
+  return (pow2_in(m.nx, 64, 1024) || third(m.nx)) && (pow2_in(m.ny, 64, 1024) || third(m.ny)) &&
+         (pow2_in(m.nz, 128, 1024) || third(m.nz));
 }
 
 int pmfft_row_len(Mesh3 m) { return m.nz / 2 + 8; }
@@ -1423,7 +1509,7 @@ int col_pass(Mesh3 m, int mode, int nbatch, int ch_off, const float2* in, float2
     L = m.ny;
     a.ncolt = P / KT;
     a.nouter = m.nx;
-    const int box_rows = L < 256 ? L : 256;
+    const int box_rows = col_box_rows(L);
     cuuint64_t dims[4] = {(cuuint64_t)P, (cuuint64_t)BY, (cuuint64_t)m.nx, (cuuint64_t)nyb * nch};
     cuuint64_t strides[3] = {(cuuint64_t)P * 8, (cuuint64_t)BY * P * 8, (cuuint64_t)a.sb * 8};
     cuuint32_t box[4] = {(cuuint32_t)KT, (cuuint32_t)BY, 1, (cuuint32_t)(box_rows / BY)};
@@ -1432,7 +1518,7 @@ int col_pass(Mesh3 m, int mode, int nbatch, int ch_off, const float2* in, float2
     L = m.nx;
     a.ncolt = BY * P / KT;
     a.nouter = nyb;
-    const int box_rows = L < 256 ? L : 256;
+    const int box_rows = col_box_rows(L);
     cuuint64_t dims[3] = {(cuuint64_t)BY * P, (cuuint64_t)m.nx, (cuuint64_t)nyb * nch};
     cuuint64_t strides[2] = {(cuuint64_t)BY * P * 8, (cuuint64_t)a.sb * 8};
     cuuint32_t box[3] = {(cuuint32_t)KT, (cuuint32_t)box_rows, 1};

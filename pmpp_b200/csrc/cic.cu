@@ -467,60 +467,6 @@ int compute_scale(const float* val, int64_t count, int64_t n, double* scale_dev,
 // rows it reaches.  NZP: the row stride of the accumulator (nz rounded up to
 // one of a few lengths), a constant so that every corner's address is one of
 // two registers plus an immediate.
-struct FastDiv {  // exact n / d for every 32-bit n
-  uint32_t mul;
-  int sh1, sh2;
-};
-
-inline FastDiv fast_div(uint32_t d) {
-  int l = 0;
-  while (l < 32 && (1ull << l) < d) ++l;
-  FastDiv f;
-  f.mul = (uint32_t)((((1ull << l) - d) << 32) / d + 1);
-  f.sh1 = l < 1 ? l : 1;
-  f.sh2 = l > 1 ? l - 1 : 0;
-  return f;
-}
-
-__device__ __forceinline__ uint32_t div_by(uint32_t n, FastDiv f) {
-  const uint32_t q = __umulhi(f.mul, n);
-  return (q + ((n - q) >> f.sh1)) >> f.sh2;
-}
-
-struct F2 {
-  unsigned long long v;
-};
-__device__ __forceinline__ F2 f2_pack(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void f2_bits(F2 x, int& a, int& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(x.v));
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_mul_rz(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }  // -126 <= e <= 127
-
 constexpr int kRowThreads = 256;
 
 template <int C, int RX, int RY, int NZP, bool EXACT, bool SIGNED>

@@ -36,6 +36,10 @@ namespace pmb {
 
 constexpr int kEnsMaxSims = 1024;
 
+// Tile shapes are limited to 200 KB at this many bytes per cell (the
+// accumulator takes two thirds of it).
+constexpr int64_t kTileBytesPerCell = 12;
+
 // Device descriptor of one member simulation.
 struct EnsSim {
   int64_t p0, n;     // particle range in the concatenated particle arrays
@@ -47,6 +51,8 @@ struct EnsSim {
   float src_mul;     // 1.5 Omega_m, the Poisson source factor
   float post;        // 1 / cells, the inverse-FFT normalisation
   double scale;      // fixed-point scale of the density deposit
+  int E;             // its exponent: contributions are at most 2^E units
+  FastDiv by_nz;     // division by m.nz
   float* rho;        // Poisson source mesh, (nx, ny, nz)
   float2* rho_hat;   // its half spectrum
   float2* grad_hat;  // three gradient spectra
@@ -131,16 +137,21 @@ __global__ void ens_bin_count_kernel(EnsDev d, int drift) {
       const Binned b = bin_particle(d.pmid, d0, d1, d2, i, m, d.sims[s].cell);
       row = (uint32_t)(d.sims[s].row0 + (int64_t)b.cx * m.ny + b.cy);
     }
-    const unsigned full = __ballot_sync(0xFFFFFFFFu, active);
+    // one atomic per run of equal rows, as the single-simulation sort
+    const int lane = threadIdx.x & 31;
+    const unsigned upto = 0xFFFFFFFFu >> (31 - lane);
+    const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, row, 1);
+    const unsigned heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || row != prev);
+    const int head = 31 - __clz(heads & upto);
+    uint32_t rb = 0;
+    if (head == lane && active) {
+      const unsigned after = heads & ~upto;
+      rb = atomicAdd(&d.counts[row], (uint32_t)((after ? __ffs(after) - 1 : 32) - lane));
+    }
+    rb = __shfl_sync(0xFFFFFFFFu, rb, head);
     if (active) {
-      const unsigned peers = __match_any_sync(full, row);
-      const int leader = __ffs(peers) - 1;
-      const int lane = threadIdx.x & 31;
-      uint32_t rb = 0;
-      if (lane == leader) rb = atomicAdd(&d.counts[row], (uint32_t)__popc(peers));
-      rb = __shfl_sync(peers, rb, leader);
       d.row_of[i] = row;
-      d.rank_of[i] = rb + __popc(peers & ((1u << lane) - 1u));
+      d.rank_of[i] = rb + (uint32_t)(lane - head);
     }
   }
 }
@@ -181,8 +192,8 @@ __global__ void __launch_bounds__(256) ens_scatter_kernel(EnsDev d) {
     const int64_t local = item - d.tile_start[s];
     const int nby = (m.ny + ry - 1) / ry;
     const int x0 = (int)(local / nby) * rx, y0 = (int)(local % nby) * ry;
-    scatter_tile<1>(d.rec, d.perm, d.offs + sim.row0, m, rx, ry, x0, y0, nullptr, 0, sim.val, sim.scale, 1,
-                    sim.src_mul, sim.rho, acc_smem, sm);
+    scatter_tile(d.rec, d.offs + sim.row0, m, sim.by_nz, rx, ry, x0, y0, sim.val, sim.scale, sim.E, sim.src_mul,
+                 sim.rho, acc_smem, sm);
   }
 }
 
@@ -351,10 +362,22 @@ void recount_tiles(Ensemble* e) {
   e->ntiles = e->tile_start[e->nsims];
 }
 
+// Tile shape until the tuner sets one: the largest of these whose accumulator
+// stays within 33 KB, as the single runs' deposit (24 members on 64^3 to 128^3
+// cells, five deposits: 1.91 ms in 2 x 2 rows, 1.07 in 4 x 4).
+void default_tile(Mesh3 m, int* rx, int* ry) {
+  static const int shapes[5][2] = {{4, 4}, {2, 4}, {2, 2}, {1, 2}, {1, 1}};
+  for (const auto& sh : shapes) {
+    *rx = sh[0] < m.nx ? sh[0] : m.nx;
+    *ry = sh[1] < m.ny ? sh[1] : m.ny;
+    if (ScatterSmem::acc_bytes(*rx, *ry, m.nz) <= 33 * 1024) return;
+  }
+}
+
 size_t scatter_smem_of(const Ensemble* e) {
   size_t mx = 0;
   for (const EnsSim& s : e->sims) {
-    const size_t b = (size_t)ScatterSmem::acc_bytes(s.rx, s.ry, 1, s.m.nz);
+    const size_t b = (size_t)ScatterSmem::acc_bytes(s.rx, s.ry, s.m.nz);
     if (b > mx) mx = b;
   }
   return mx;
@@ -584,10 +607,9 @@ int pmb_ens_create(int nsims, const int64_t* counts, const int32_t* mesh_shapes,
     q.post = (float)(1.0 / (double)q.m.cells());
     const float a = fabsf(vals[s]);
     q.scale = fixed_point_scale(fixed_point_pow2(q.n), a);
-    q.rx = 2;
-    q.ry = 2;
-    if (q.rx > q.m.nx) q.rx = q.m.nx;
-    if (q.ry > q.m.ny) q.ry = q.m.ny;
+    q.E = fixed_point_exponent(q.n);
+    q.by_nz = fast_div((uint32_t)q.m.nz);
+    default_tile(q.m, &q.rx, &q.ry);
     e->p_start[s + 1] = e->p_start[s] + counts[s];
     e->spec_start[s + 1] = e->spec_start[s] + q.m.half_cells();
     e->mesh_start[s + 1] = e->mesh_start[s] + q.m.cells();
@@ -727,7 +749,7 @@ int pmb_ens_set_tiles(void* handle, const int32_t* rx, const int32_t* ry) {
   for (int i = 0; i < e->nsims; ++i) {
     const EnsSim& q = e->sims[i];
     ENS_REQUIRE(rx[i] >= 1 && ry[i] >= 1 && (rx[i] + 1) * (ry[i] + 1) <= kMaxSrcRows && rx[i] <= q.m.nx &&
-                    ry[i] <= q.m.ny && ScatterSmem::acc_bytes(rx[i], ry[i], 1, q.m.nz) <= 200 * 1024,
+                    ry[i] <= q.m.ny && kTileBytesPerCell * rx[i] * ry[i] * q.m.nz <= 200 * 1024,
                 "pmb_ens_set_tiles: tile shape out of range");
   }
   for (int i = 0; i < e->nsims; ++i) {

@@ -77,151 +77,202 @@ __device__ __forceinline__ Rec unmasked_or_origin(const Rec& r, bool* masked) {
   return z;
 }
 
-constexpr int kMaxSrcRows = 25;  // (RX+1)*(RY+1) with RX, RY <= 4
-
-// Shared-memory bookkeeping of one scatter tile.
-struct ScatterSmem {
-  uint32_t seg_beg[kMaxSrcRows];
-  uint32_t seg_pre[kMaxSrcRows + 1];
-  // dynamic accumulator bytes of an RX x RY block with C channels
-  static constexpr int64_t acc_bytes(int RX, int RY, int C, int nz) { return (int64_t)12 * RX * RY * C * nz; }
+struct FastDiv {  // exact n / d for every 32-bit n
+  uint32_t mul;
+  int sh1, sh2;
 };
 
-// One RX x RY block of output rows at (x0, y0) of mesh m: pulls the
-// particles of the (RX+1) x (RY+1) source rows that reach the block
-// (offs[row] .. offs[row+1] in the sorted records; offs points at this
-// mesh's first row), accumulates val * w as 64-bit fixed-point integers
-// (units of 1/scale) in shared memory, and writes every output cell once:
-// mode 0 the deposit, mode 1 the Poisson source (rho - 1) * src_mul
-// (gravity.py:628-630).  val (C values per particle, may be null for the
-// constant val_const) is indexed by source particle (perm) or, with
-// val_sorted, by sorted position.
+inline FastDiv fast_div(uint32_t d) {
+  int l = 0;
+  while (l < 32 && (1ull << l) < d) ++l;
+  FastDiv f;
+  f.mul = (uint32_t)((((1ull << l) - d) << 32) / d + 1);
+  f.sh1 = l < 1 ? l : 1;
+  f.sh2 = l > 1 ? l - 1 : 0;
+  return f;
+}
+
+__device__ __forceinline__ uint32_t div_by(uint32_t n, FastDiv f) {
+  const uint32_t q = __umulhi(f.mul, n);
+  return (q + ((n - q) >> f.sh1)) >> f.sh2;
+}
+
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2_pack(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_bits(F2 x, int& a, int& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul_rz(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }  // -126 <= e <= 127
+
+constexpr int kMaxSrcRows = 25;  // (RX + 1) (RY + 1) of a tile
+constexpr int kMaxTile = 11;     // so RX, RY <= 11
+
+// Shared-memory bookkeeping of one scatter tile: per pass and source x the
+// records' range (as prefix sums of visits) and first row.
+struct ScatterSmem {
+  uint32_t pre[2][kMaxTile + 2], beg[2][kMaxTile + 1], row[2][kMaxTile + 1];
+  // dynamic accumulator bytes of an RX x RY block
+  static constexpr int64_t acc_bytes(int RX, int RY, int nz) { return (int64_t)8 * RX * RY * nz; }
+};
+
+// One RX x RY block of output rows at (x0, y0) of mesh m, shape known at run
+// time (cic.cu's scatter_rows_kernel has the constant shapes and explains the
+// arithmetic): pulls the particles of the (RX+1) x (RY+1) source rows that
+// reach the block (offs[row] .. offs[row+1] in the sorted records; offs points
+// at this mesh's first row), sums the constant val > 0 times the weights as
+// integers in units of 1/scale on two 32-bit planes in shared memory, and
+// writes every output cell once as the Poisson source (rho - 1) * src_mul
+// (gravity.py:628-630).  The sums are exact, so the result is independent of
+// the particle order and bit-identical to scatter_rows_kernel's.  Called by
+// all threads of the block; leaves it synchronised.  by_nz: m.nz.
 //
-// Integer sums do not depend on the order in which particles arrive, so the
-// result is bit-deterministic.  Accumulator: 12 bytes per output cell-channel
-// (ScatterSmem::acc_bytes).  When the block's source segments hold fewer
-// than 2^16 particles, each 64-bit contribution q = a*2^32 + b*2^16 + c (a
-// signed, 0 <= b, c < 2^16) is added as three 32-bit shared atomics on
-// separate planes: the b and c sums stay below 2^32 and the a sum below 2^31,
-// so the recombined total is exactly the 64-bit sum, while 32-bit atomics
-// tolerate many particles per cell (clustering) far better than 64-bit ones.
-// Larger blocks use one 64-bit atomic per contribution on the first 8 bytes
-// per cell.  Either way the result is the same exact sum.  Must be called by
-// all threads of the block; leaves the block synchronised.
-template <int C>
-__device__ __forceinline__ void scatter_tile(const Rec* __restrict__ rec, const uint32_t* __restrict__ perm,
-                                             const uint32_t* __restrict__ offs, Mesh3 m, int RX, int RY, int x0,
-                                             int y0, const float* __restrict__ val, int val_sorted, float val_const,
-                                             double scale, int mode, float src_mul, float* __restrict__ out,
-                                             unsigned int* acc, ScatterSmem& sm) {
-  const int nz = m.nz;
-  const int nsrc = (RX + 1) * (RY + 1);
-  const int cells = RX * RY * C * nz;
+// Three 16-bit planes with 64-bit conversions per corner, in 2 x 2 rows, took
+// 1.70 ms for five deposits of 24 members on 64^3 to 128^3 cells; this takes
+// 1.07 ms in 4 x 4 rows.
+__device__ __forceinline__ void scatter_tile(const Rec* __restrict__ rec, const uint32_t* __restrict__ offs, Mesh3 m,
+                                             FastDiv by_nz, int RX, int RY, int x0, int y0, float val, double scale,
+                                             int E, float src_mul, float* __restrict__ out, unsigned int* acc,
+                                             ScatterSmem& sm) {
+  const int nz = m.nz, cells = RX * RY * nz;
+  const int rxe = min(RX, m.nx - x0), rye = min(RY, m.ny - y0);
   {
     uint4* a4 = reinterpret_cast<uint4*>(acc);
-    const int n4 = (3 * cells) >> 2;
+    const int n4 = (2 * cells) >> 2;
     for (int t = threadIdx.x; t < n4; t += blockDim.x) a4[t] = make_uint4(0u, 0u, 0u, 0u);
-    for (int t = 4 * n4 + threadIdx.x; t < 3 * cells; t += blockDim.x) acc[t] = 0u;
+    for (int t = 4 * n4 + threadIdx.x; t < 2 * cells; t += blockDim.x) acc[t] = 0u;
   }
-  if (threadIdx.x < nsrc) {
-    const int k = threadIdx.x;
-    const int px = pmod(x0 + k / (RY + 1) - 1, m.nx), py = pmod(y0 + k % (RY + 1) - 1, m.ny);
-    const int64_t row = (int64_t)px * m.ny + py;
-    const uint32_t b = offs[row];
-    sm.seg_beg[k] = b;
-    sm.seg_pre[k + 1] = offs[row + 1] - b;
+  if (threadIdx.x < 2 * (kMaxTile + 1)) {
+    const int pass = threadIdx.x > kMaxTile, k = threadIdx.x - pass * (kMaxTile + 1);
+    uint32_t b = 0, c = 0, row = 0;
+    if (k <= rxe && (pass == 0 || y0 == 0)) {
+      const int x = k == 0 ? (x0 == 0 ? m.nx - 1 : x0 - 1) : x0 + k - 1;
+      row = (uint32_t)((int64_t)x * m.ny) + (uint32_t)(pass == 0 ? y0 : m.ny);
+      const int64_t lo = pass == 0 ? (int64_t)row - (y0 > 0) : (int64_t)row - 1;
+      const int64_t hi = pass == 0 ? (int64_t)row + rye : (int64_t)row;
+      b = offs[lo];
+      c = offs[hi] - b;
+    }
+    sm.beg[pass][k] = b;
+    sm.pre[pass][k + 1] = c;
+    sm.row[pass][k] = row;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  uint32_t kcell = 0;  // particles that may reach one cell: those of two neighbouring source x
+  for (int k = 0; k < RX; ++k)
+    kcell = max(kcell, sm.pre[0][k + 1] + sm.pre[1][k + 1] + sm.pre[0][k + 2] + sm.pre[1][k + 2]);
+  __syncthreads();
+  if (threadIdx.x < 2) {
     uint32_t run = 0;
-    for (int k = 0; k < nsrc; ++k) {
-      const uint32_t c = sm.seg_pre[k + 1];
-      sm.seg_pre[k] = run;
-      run += c;
+    sm.pre[threadIdx.x][0] = 0;
+    for (int k = 1; k <= kMaxTile + 1; ++k) {
+      run += sm.pre[threadIdx.x][k];
+      sm.pre[threadIdx.x][k] = run;
     }
-    sm.seg_pre[nsrc] = run;
   }
+  const int dup = (m.nx == 1 ? 2 : 1) * (m.ny == 1 ? 2 : 1) * (m.nz == 1 ? 2 : 1);
+  const uint64_t kmax = (uint64_t)kcell * (uint64_t)dup;
+  const int L = kmax ? 64 - __clzll((long long)kmax) : 0;
+  const int lo = max(max(E - 24, L + E - 32), 1), hi = min(24, 32 - L);
+  const int s = max(lo, min(hi, (E + 1) / 2));
+  const bool split = lo <= hi && scale >= 0x1p-50 && scale <= 0x1p100 && val >= 0.f;
+  const float v = split ? __fmul_rn(val, __fmul_rn((float)scale, pow2f(-s - 49))) : val;
+  const F2 v2 = f2_pack(v, v), to_h = f2_pack(pow2f(-100), pow2f(-100)), back = f2_pack(-pow2f(100), -pow2f(100));
+  const F2 to_l = f2_pack(pow2f(s - 100), pow2f(s - 100));
+  int* const planes = reinterpret_cast<int*>(acc);
+  unsigned long long* const acc64 = reinterpret_cast<unsigned long long*>(acc);
   __syncthreads();
-  const uint32_t ntot = sm.seg_pre[nsrc];
-  const bool split = ntot < 65536u;
-  unsigned long long* acc64 = reinterpret_cast<unsigned long long*>(acc);
-  // the scale is a power of two: contrib * scale is exact in float when the
-  // scale itself is a float (always, unless max|val| < 2^-74)
-  const bool fscale = scale < 0x1p126;
-  const float scalef = fscale ? (float)scale : 0.f;
-  int k = 0;  // source segment of idx; idx only grows, so the search resumes
-  const bool zpow2 = (nz & (nz - 1)) == 0;
-  for (uint32_t idx = threadIdx.x; idx < ntot; idx += blockDim.x) {
-    while (idx >= sm.seg_pre[k + 1]) ++k;
-    const int sx = k / (RY + 1) - 1, sy = k % (RY + 1) - 1;
-    const uint32_t i = sm.seg_beg[k] + (idx - sm.seg_pre[k]);
-    const Rec r = rec[i];
-    const int cz = zpow2 ? (int)(r.key & (uint32_t)(nz - 1)) : (int)(r.key % (uint32_t)nz);
-    float v[C];
-    if (val != nullptr) {
-      const int64_t src = val_sorted ? (int64_t)i : (int64_t)perm[i];
+  for (int pass = 0; pass < 2; ++pass) {
+    const uint32_t end = sm.pre[pass][kMaxTile + 1];
+    for (uint32_t vi = threadIdx.x; vi < end; vi += blockDim.x) {
+      int k = 0;
+      while (vi >= sm.pre[pass][k + 1]) ++k;
+      const Rec r = rec[sm.beg[pass][k] + (vi - sm.pre[pass][k])];
+      const uint32_t rowk = div_by(r.key, by_nz);
+      const int sx = k - 1, ly = (int)(rowk - sm.row[pass][k]), cz = (int)(r.key - rowk * (uint32_t)nz);
+      const int dz = cz + 1 == nz ? 1 - nz : 1;
+      const F2 wz = f2_pack(axis_weight(r.fz, 0), axis_weight(r.fz, 1));
 #pragma unroll
-      for (int c = 0; c < C; ++c) v[c] = val[src * C + c];
-    } else {
+      for (int bx = 0; bx < 2; ++bx) {
+        const int lx = sx + bx;
+        const float wx = axis_weight(r.fx, bx);
 #pragma unroll
-      for (int c = 0; c < C; ++c) v[c] = val_const;
-    }
-#pragma unroll
-    for (int bx = 0; bx < 2; ++bx) {
-      const int lx = sx + bx;
-      if (lx < 0 || lx >= RX || x0 + lx >= m.nx) continue;
-      const float wx = axis_weight(r.fx, bx);
-#pragma unroll
-      for (int by = 0; by < 2; ++by) {
-        const int ly = sy + by;
-        if (ly < 0 || ly >= RY || y0 + ly >= m.ny) continue;
-        const float wxy = __fmul_rn(wx, axis_weight(r.fy, by));
-#pragma unroll
-        for (int bz = 0; bz < 2; ++bz) {
-          int z = cz + bz;
-          if (z >= nz) z -= nz;
-          const float w = __fmul_rn(wxy, axis_weight(r.fz, bz));
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            const float contrib = __fmul_rn(v[c], w);
-            const long long q = fscale ? __float2ll_rn(__fmul_rn(contrib, scalef))
-                                       : __double2ll_rn((double)contrib * scale);
-            const int a = ((lx * RY + ly) * C + c) * nz + z;
-            if (split) {
-              atomicAdd(&acc[a], (unsigned int)(q >> 32));
-              atomicAdd(&acc[cells + a], (unsigned int)((q >> 16) & 0xFFFF));
-              atomicAdd(&acc[2 * cells + a], (unsigned int)(q & 0xFFFF));
-            } else {
-              atomicAdd(&acc64[a], (unsigned long long)q);
-            }
+        for (int by = 0; by < 2; ++by) {
+          if (lx < 0 || lx >= rxe || ly + by < 0 || ly + by >= rye) continue;
+          const float wxy = __fmul_rn(wx, axis_weight(r.fy, by));
+          const F2 q = f2_mul(v2, f2_mul(f2_pack(wxy, wxy), wz));
+          const int a0 = (lx * RY + ly + by) * nz + cz, a1 = a0 + dz;
+          int i0, i1, l0, l1;
+          if (split) {
+            const F2 t = f2_mul_rz(q, to_h);
+            f2_bits(t, i0, i1);
+            f2_bits(f2_mul(f2_fma(t, back, q), to_l), l0, l1);
+            atomicAdd(planes + a0, i0);
+            atomicAdd(planes + cells + a0, l0);
+            atomicAdd(planes + a1, i1);
+            atomicAdd(planes + cells + a1, l1);
+          } else {
+            f2_bits(q, i0, i1);
+            atomicAdd(&acc64[a0], (unsigned long long)__double2ll_rn((double)__int_as_float(i0) * scale));
+            atomicAdd(&acc64[a1], (unsigned long long)__double2ll_rn((double)__int_as_float(i1) * scale));
           }
         }
       }
     }
   }
   __syncthreads();
-  const double inv = 1.0 / scale;
-  const int64_t mcells = m.cells();
-  for (int lx = 0; lx < RX; ++lx) {
-    if (x0 + lx >= m.nx) break;
-    for (int ly = 0; ly < RY; ++ly) {
-      if (y0 + ly >= m.ny) break;
-      const int64_t row_off = ((int64_t)(x0 + lx) * m.ny + (y0 + ly)) * nz;
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int a0 = ((lx * RY + ly) * C + c) * nz;
-        float* o = out + (int64_t)c * mcells + row_off;
-        for (int z = threadIdx.x; z < nz; z += blockDim.x) {
-          const int a = a0 + z;
-          const long long sum = split ? (long long)(((unsigned long long)acc[a] << 32) +
-                                                    ((unsigned long long)acc[cells + a] << 16) +
-                                                    (unsigned long long)acc[2 * cells + a])
-                                      : (long long)acc64[a];
-          float rho = (float)((double)sum * inv);
-          if (mode == 1) rho = __fmul_rn(__fsub_rn(rho, 1.0f), src_mul);
-          o[z] = rho;
-        }
+  // (float)(sum / scale): sums below 2^23 on both planes in single precision
+  // with one rounding, the others exactly in double precision
+  const double inv = __hiloint2double(0x7FE00000 - __double2hiint(scale), 0);
+  const float invf = (float)inv, two_s = pow2f(split ? s : 0);
+  const bool fconv = split && invf >= 0x1p-126f;
+  for (int row = 0; row < RX * RY; ++row) {
+    const int lx = row / RY, ly = row - lx * RY;
+    if (lx >= rxe || ly >= rye) continue;
+    float* o = out + ((int64_t)(x0 + lx) * m.ny + (y0 + ly)) * nz;
+    for (int z = threadIdx.x; z < nz; z += blockDim.x) {
+      const int a = row * nz + z;
+      float rho;
+      if (split) {
+        const uint32_t h = acc[a], l = acc[cells + a];
+        if (fconv && (h | l) < 0x800000u)
+          rho = __fmul_rn(__fmaf_rn(__uint_as_float(0x4B000000u + h) - 0x1p23f, two_s,
+                                    __uint_as_float(0x4B000000u + l) - 0x1p23f),
+                          invf);
+        else
+          rho = (float)(fma(__hiloint2double(0x43300000, (int)h) - 0x1p52, (double)two_s,
+                            __hiloint2double(0x43300000, (int)l) - 0x1p52) *
+                        inv);
+      } else {
+        rho = (float)((double)(long long)acc64[a] * inv);
       }
+      o[z] = __fmul_rn(__fsub_rn(rho, 1.0f), src_mul);
     }
   }
   __syncthreads();

@@ -21,6 +21,7 @@ int bin_particles(const int16_t* pmid, float* disp, const float* vel, float drif
                   Rec* rec, uint32_t* perm, uint32_t* offs, void* scratch, cudaStream_t s,
                   const BinShift* shift = nullptr, const uint8_t* valid = nullptr, uint32_t* status = nullptr);
 double fixed_point_pow2(int64_t n);
+int fixed_point_exponent(int64_t n);  // its base-2 logarithm
 int compute_scale(const float* val, int64_t count, int64_t n, double* scale_dev, unsigned int* tmp, cudaStream_t s);
 // n: particles the sort placed (bounds the fixed-point sums); scale_dev: the
 // fixed-point scale of val (null with a constant value, whose scale is known)

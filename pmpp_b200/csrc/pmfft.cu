@@ -312,10 +312,16 @@ enum ColMode : int {
   kXInv = 5,     // x inverse, 1 -> 1
   kXGreen = 6,   // x, K(k), x^-1 of i c_x phi and phi: 1 -> 2
   kXGreenAdj = 7, // x of B_x and b, K(k) ((-i c_x) B_x + b), x^-1: 2 -> 1
-  kXFwdAdjK = 8   // x of B_x and b, K(k) ((-i c_x) B_x + b) (no inverse): 2 -> 1
+  kXFwdAdjK = 8,  // x of B_x and b, K(k) ((-i c_x) B_x + b) (no inverse): 2 -> 1
+  // y inverse of W, of i c_y Q, and i c_z y^-1(Q), one output a tile: 2 -> 3.
+  // kYInv and kYInvYZ in one launch for L <= 512; reading Q twice costs less
+  // than holding it through two transforms, since one transform at a time fits
+  // two CTAs per SM: 465 -> 352 us at 512^3, 30 -> 29 at 192^3, 16 -> 12 at
+  // 128^3, but 2.66 -> 2.97 ms at 1024^3.
+  kYInvAll = 9
 };
 
-__host__ __device__ constexpr bool is_y(int mode) { return mode <= kYFwdYZ; }
+__host__ __device__ constexpr bool is_y(int mode) { return mode <= kYFwdYZ || mode == kYInvAll; }
 __host__ __device__ constexpr int n_in(int mode) {
   return (mode == kYFwdYZ || mode == kXGreenAdj || mode == kXFwdAdjK) ? 2 : 1;
 }
@@ -323,7 +329,7 @@ __host__ __device__ constexpr int n_in(int mode) {
 // floats of per-axis tables a column pass keeps in shared memory
 __host__ __device__ constexpr int col_table_floats(int mode, int L) {
   return (mode == kXGreen || mode == kXGreenAdj || mode == kXFwdAdjK) ? 3 * L
-                                                                     : ((mode == kYInvYZ || mode == kYFwdYZ) ? L : 0);
+                                                                     : ((mode == kYInvYZ || mode == kYFwdYZ || mode == kYInvAll) ? L : 0);
 }
 
 struct ColArgs {
@@ -336,6 +342,7 @@ struct ColArgs {
   int nouter;      // x (y pass) or y blocks (x pass)
   int ntiles;      // ncolt * nouter * nbatch
   int ch_off;      // first input channel
+  int q_off;       // kYInvAll: input channel of Q relative to W's
   uint32_t polls;  // poll limit of the first wait on a stage (pmb_set_wait_limit)
   const float2* tw;
   SpecTables t;
@@ -502,7 +509,7 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
   // y passes run the column tiles kz < zs; x passes the live (ky, kz tile)
   // columns; the forward y pass stores live ky rows only and the inverse y
   // pass loads them only (PIN / POUT)
-  constexpr bool PIN = (MODE == kYInv || MODE == kYInvYZ);
+  constexpr bool PIN = (MODE == kYInv || MODE == kYInvYZ || MODE == kYInvAll);
   constexpr bool POUT = (MODE == kYFwd || MODE == kYFwdYZ);
   Live lv{a.ny, 0, a.P};
   if constexpr (PR) lv = live_extents(a.prune_base, a.prune_stride, a.prune_count, a.nx, a.ny, a.nz);
@@ -534,12 +541,14 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
       ct = (iy % BY) * (a.P / KT) + kt;
     }
   };
+  // table array of a batch (kYInvAll counts an output as a batch, three a member)
+  auto member_of = [](int batch) { return MODE == kYInvAll ? batch / 3 : batch; };
   // tables of the current batch (the configuration's for unbatched passes)
   SpecTables T = a.t;
   int tab_batch = 0;
   auto load_tables = [&]() {
     for (int i = t; i < L; i += G::T) {
-      if constexpr (MODE == kYInvYZ || MODE == kYFwdYZ) tab[i] = T.cy[i];
+      if constexpr (MODE == kYInvYZ || MODE == kYFwdYZ || MODE == kYInvAll) tab[i] = T.cy[i];
       if constexpr (MODE == kXGreen || MODE == kXGreenAdj || MODE == kXFwdAdjK) {
         const float kx = T.kx[i];
         tab[i] = kx * kx;                                  // kx^2
@@ -555,6 +564,7 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
     } else {
       tab_batch = (int)(blockIdx.x / (a.ncolt * a.nouter));
     }
+    tab_batch = member_of(tab_batch);
     T = tables_at(a.tab_base + (int64_t)tab_batch * a.tab_stride, a.nx, a.ny, a.nz, a.has_masks);
   }
   for (int i = t; i < L; i += G::T) stw[i] = a.tw[i];
@@ -575,7 +585,8 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
     const int tile = blockIdx.x + (i / NIN) * gridDim.x;
     int ct, outer, batch;
     decode(tile, ct, outer, batch);
-    const int ch = a.ch_off + batch * NIN + i % NIN;
+    const int ch = MODE == kYInvAll ? a.ch_off + member_of(batch) + (batch % 3 != 0 ? a.q_off : 0)
+                                    : a.ch_off + batch * NIN + i % NIN;
     const int s = i % S;
     float2* dst = smem + s * G::BUF;
     const int nyb = a.ny / BY;
@@ -655,12 +666,12 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
     const int tile = blockIdx.x + it * gridDim.x;
     int ct, outer, batch;
     decode(tile, ct, outer, batch);
-    if (a.tab_base != nullptr && batch != tab_batch) {
+    if (a.tab_base != nullptr && member_of(batch) != tab_batch) {
       // a new batch: its own tables (the previous tile released its stage
       // with a barrier, so no thread still reads them)
       __syncthreads();
-      tab_batch = batch;
-      T = tables_at(a.tab_base + (int64_t)batch * a.tab_stride, a.nx, a.ny, a.nz, a.has_masks);
+      tab_batch = member_of(batch);
+      T = tables_at(a.tab_base + (int64_t)tab_batch * a.tab_stride, a.nx, a.ny, a.nz, a.has_masks);
       load_tables();
       __syncthreads();
     }
@@ -683,6 +694,36 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
           else
             off = ob + (int64_t)outer * a.sb + (int64_t)r * BY * a.P + ct * KT + c;
           a.out[off] = u[k2];
+        }
+      }
+      release(i0);
+    } else if constexpr (MODE == kYInvAll) {
+      const int which = batch % 3;
+      const int kz = ct * KT + c;
+      const bool kv = kz_valid(kz, a.nz);
+      const float cz = kv ? T.cz[kz] : 0.f;
+      float2* buf = smem + (i0 % S) * G::BUF;
+      float2 v[R1];
+      if (ja) {
+#pragma unroll
+        for (int n1 = 0; n1 < R1; ++n1) {
+          v[n1] = ld(buf, R2 * n1 + q);
+          if (which == 1) v[n1] = i_times(tab[R2 * n1 + q], v[n1]);
+        }
+      }
+      __syncthreads();
+      if (ja) four_step_a<R1, R2, true>(v, buf, q, c, stw);
+      __syncthreads();
+      if (jb) {
+        four_step_b<R1, R2, true>(u, buf, q, c);
+        const int64_t ob = out_ch(batch, 0) + (int64_t)outer * BY * a.P + kz;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) {
+          const int y = q + R1 * k2;
+          float2 val = u[k2];
+          if (which == 1 && !kv) val = make_float2(0.f, 0.f);
+          if (which == 2) val = i_times(cz, val);
+          a.out[ob + (int64_t)(y / BY) * a.sb + (int64_t)(y % BY) * a.P] = val;
         }
       }
       release(i0);
@@ -1309,17 +1350,22 @@ int launch_col_ctas(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
 // x + multiplier 1082 / 1402 (1024^3), inverse y into two outputs 331 / 447
 // (512^3), y combine 310 / 437, adjoint x 222 / 302.  Lengths up to 256 run 128
 // threads a CTA, of which two share an SM at any register count.
+constexpr int kInvAllMax = 512;  // longest y of the joint inverse pass
+
 constexpr int col_ctas(int mode, int L) {
   if (L == 1024) return mode == kYFwd ? 2 : 1;
-  if (L == 512) return mode == kYFwd || mode == kYInv || mode == kXGreen ? 2 : 1;
-  if (L == 384 || L == 768) return mode == kYFwd || mode == kYInv ? 2 : 1;
+  if (L == 512) return mode == kYFwd || mode == kYInv || mode == kXGreen || mode == kYInvAll ? 2 : 1;
+  if (L == 384) return mode == kYFwd || mode == kYInv || mode == kYInvAll ? 2 : 1;
+  if (L == 768) return mode == kYFwd || mode == kYInv ? 2 : 1;
   return 1;
 }
 
 template <int R1, int R2, int MODE, bool PR>
 int launch_col(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
   constexpr int L = R1 * R2;
-  if constexpr (L == 512 || L == 1024) {  // the lengths at which the two differ
+  if constexpr (MODE == kYInvAll && L > kInvAllMax) {
+    return kUnsupported;
+  } else if constexpr (L == 512 || L == 1024) {  // the lengths at which the two differ
     const int ctas = g_col_ctas != 0 ? g_col_ctas : col_ctas(MODE, L);
     if (ctas == 2) return launch_col_ctas<R1, R2, MODE, 2, PR>(map, a, s);
     return launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
@@ -1474,13 +1520,13 @@ int z_pass(Mesh3 m, int inverse, int batch, const float* in_r, const float2* in_
 int col_pass(Mesh3 m, int mode, int nbatch, int ch_off, const float2* in, float2* out, SpecTables t, GreenParams g,
              const float* tab_base, int64_t tab_stride, int has_masks, int oofs, int ostride, int cstride, PruneSrc pr,
              cudaStream_t s) {
-  if (!pmfft_supported(m) || nbatch < 1 || mode < kYFwd || mode > kXFwdAdjK) {
+  if (!pmfft_supported(m) || nbatch < 1 || mode < kYFwd || mode > kYInvAll || (mode == kYInvAll && nbatch % 3 != 0)) {
     set_last_error("pmfft: unsupported mesh or mode");
     return kUnsupported;
   }
   const int P = pmfft_row_len(m);
   const int nyb = m.ny / BY;
-  const int nch = ch_off + nbatch * n_in(mode);
+  const int nch = ch_off + (mode == kYInvAll ? nbatch / 3 * 2 : nbatch * n_in(mode));
   ColArgs a{};
   a.out = out;
   a.ch = pmfft_channel_elems(m);
@@ -1490,6 +1536,7 @@ int col_pass(Mesh3 m, int mode, int nbatch, int ch_off, const float2* in, float2
   a.ny = m.ny;
   a.nz = m.nz;
   a.ch_off = ch_off;
+  a.q_off = nbatch / 3;
   a.polls = wait_polls();
   a.t = t;
   a.g = g;
@@ -1539,6 +1586,7 @@ int col_pass(Mesh3 m, int mode, int nbatch, int ch_off, const float2* in, float2
     case kYInv: return launch_col_len_pr<kYInv>(pr_on, L, map, a, s);
     case kYInvYZ: return launch_col_len_pr<kYInvYZ>(pr_on, L, map, a, s);
     case kYFwdYZ: return launch_col_len_pr<kYFwdYZ>(pr_on, L, map, a, s);
+    case kYInvAll: return launch_col_len_pr<kYInvAll>(pr_on, L, map, a, s);
     case kXFwd: return launch_col_len<kXFwd>(L, map, a, s);
     case kXInv: return launch_col_len<kXInv>(L, map, a, s);
     case kXGreen: return launch_col_len_pr<kXGreen>(pr_on, L, map, a, s);
@@ -1605,8 +1653,12 @@ int pmfft_force(Mesh3 m, const float* src, float* force_meshes, float2* work, Sp
   if (st != kOk) return st;
   if ((st = col_pass(m, kYFwd, 1, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
   if ((st = col_pass(m, kXGreen, 1, 0, fp, aq, t, g, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
-  if ((st = col_pass(m, kYInv, 1, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
-  if ((st = col_pass(m, kYInvYZ, 1, 1, aq, fp + C, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
+  if (m.ny <= kInvAllMax) {
+    if ((st = col_pass(m, kYInvAll, 3, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
+  } else {
+    if ((st = col_pass(m, kYInv, 1, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
+    if ((st = col_pass(m, kYInvYZ, 1, 1, aq, fp + C, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
+  }
   return z_pass(m, 1, 3, nullptr, fp, force_meshes, nullptr, pr, s);
 }
 
@@ -1628,10 +1680,14 @@ int pmfft_force_batched(Mesh3 m, int count, const float* src, float* force_meshe
   if ((st = col_pass(m, kYFwd, count, 0, aq, fp, t0, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
   if ((st = col_pass(m, kXGreen, count, 0, fp, aq, t0, g, tab_base, tab_stride, has_masks, 0, 1, count, pr, s)) != kOk)
     return st;
-  if ((st = col_pass(m, kYInv, count, 0, aq, fp, t0, none, nullptr, 0, 0, 0, 3, 1, pr, s)) != kOk) return st;
-  if ((st = col_pass(m, kYInvYZ, count, count, aq, fp, t0, none, tab_base, tab_stride, has_masks, 1, 3, 1, pr, s)) !=
-      kOk)
-    return st;
+  if (m.ny <= kInvAllMax) {
+    st = col_pass(m, kYInvAll, 3 * count, 0, aq, fp, t0, none, tab_base, tab_stride, has_masks, 0, 1, 1, pr, s);
+    if (st != kOk) return st;
+  } else {
+    if ((st = col_pass(m, kYInv, count, 0, aq, fp, t0, none, nullptr, 0, 0, 0, 3, 1, pr, s)) != kOk) return st;
+    st = col_pass(m, kYInvYZ, count, count, aq, fp, t0, none, tab_base, tab_stride, has_masks, 1, 3, 1, pr, s);
+    if (st != kOk) return st;
+  }
   return z_pass(m, 1, 3 * count, nullptr, fp, force_meshes, nullptr, pr, s);
 }
 

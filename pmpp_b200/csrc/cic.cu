@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kSortThreads) bin_place_kernel(const int16_t* 
 // launches saved on the host), else two launches over tiles of 4096 entries,
 // the second adding the sum of the tiles before its own.
 constexpr int kScanThreads = 1024;
-constexpr int kScanPer = 4;
+constexpr int kScanPer = 4;  // (scan_one_kernel moves these as one vector)
 constexpr int kScanTile = kScanThreads * kScanPer;
 constexpr int kScanOneTiles = 4;
 constexpr int64_t kScanOne = kScanOneTiles * kScanTile + 1;
@@ -209,17 +209,22 @@ __global__ void __launch_bounds__(kScanThreads) scan_one_kernel(const uint32_t* 
   hand_on_flag(flag, status);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t last = n - 1;
+  const bool vec = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
   uint32_t v[kScanOneTiles][kScanPer], x[kScanOneTiles], own[kScanOneTiles];
 #pragma unroll
   for (int c = 0; c < kScanOneTiles; ++c) {
     const int64_t base = (int64_t)c * kScanTile + (int64_t)threadIdx.x * kScanPer;
-    uint32_t s = 0;
+    if (vec && base + kScanPer <= last) {
+      const uint4 q = *reinterpret_cast<const uint4*>(in + base);
+      v[c][0] = q.x;
+      v[c][1] = q.y;
+      v[c][2] = q.z;
+      v[c][3] = q.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < kScanPer; ++j) {
-      v[c][j] = base + j < last ? in[base + j] : 0u;
-      s += v[c][j];
+      for (int j = 0; j < kScanPer; ++j) v[c][j] = base + j < last ? in[base + j] : 0u;
     }
-    own[c] = x[c] = s;
+    own[c] = x[c] = v[c][0] + v[c][1] + v[c][2] + v[c][3];
   }
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1)
@@ -245,11 +250,15 @@ __global__ void __launch_bounds__(kScanThreads) scan_one_kernel(const uint32_t* 
 #pragma unroll
   for (int c = 0; c < kScanOneTiles; ++c) {
     const int64_t base = (int64_t)c * kScanTile + (int64_t)threadIdx.x * kScanPer;
-    uint32_t off = carry + (warp ? sh[c][warp - 1] : 0u) + x[c] - own[c];
+    const uint32_t o0 = carry + (warp ? sh[c][warp - 1] : 0u) + x[c] - own[c];
+    const uint32_t o1 = o0 + v[c][0], o2 = o1 + v[c][1], o3 = o2 + v[c][2];
+    if (vec && base + kScanPer <= last) {
+      *reinterpret_cast<uint4*>(out + base) = make_uint4(o0, o1, o2, o3);
+    } else {
+      const uint32_t o[kScanPer] = {o0, o1, o2, o3};
 #pragma unroll
-    for (int j = 0; j < kScanPer; ++j) {
-      if (base + j < last) out[base + j] = off;
-      off += v[c][j];
+      for (int j = 0; j < kScanPer; ++j)
+        if (base + j < last) out[base + j] = o[j];
     }
     carry += sh[c][31];
   }

@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const int16_t* 
                                                                  uint32_t* __restrict__ row_of,
                                                                  uint32_t* __restrict__ rank_of,
                                                                  uint32_t* __restrict__ flag) {
+  wait_for_previous();
+  let_next_start();
   const int64_t base = (int64_t)blockIdx.x * (kSortThreads * kSortPer) + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const unsigned upto = 0xFFFFFFFFu >> (31 - lane);  // lanes 0 .. lane
@@ -140,6 +142,8 @@ __global__ void __launch_bounds__(kSortThreads) bin_place_kernel(const int16_t* 
                                                                  const uint32_t* __restrict__ row_of,
                                                                  const uint32_t* __restrict__ rank_of,
                                                                  Rec* __restrict__ rec, uint32_t* __restrict__ perm) {
+  wait_for_previous();
+  let_next_start();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t row = row_of[i];
@@ -206,6 +210,8 @@ __device__ __forceinline__ void hand_on_flag(const uint32_t* flag, uint32_t* sta
 __global__ void __launch_bounds__(kScanThreads) scan_one_kernel(const uint32_t* in, uint32_t* out, int64_t n,
                                                                 const uint32_t* flag, uint32_t* status) {
   __shared__ uint32_t sh[kScanOneTiles][33];
+  wait_for_previous();
+  let_next_start();
   hand_on_flag(flag, status);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t last = n - 1;
@@ -269,6 +275,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const uint32_t
                                                                   uint32_t* __restrict__ tile_sums,
                                                                   const uint32_t* flag, uint32_t* status) {
   __shared__ uint32_t sh[32];
+  wait_for_previous();
+  let_next_start();
   hand_on_flag(flag, status);
   int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanPer;
   uint32_t v[kScanPer];
@@ -290,6 +298,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const uint32_t
 __global__ void __launch_bounds__(kScanThreads) scan_add_kernel(uint32_t* __restrict__ out, int64_t n,
                                                                 const uint32_t* __restrict__ tile_sums) {
   __shared__ uint32_t sh[32];
+  wait_for_previous();
+  let_next_start();
   const int64_t tile = (int64_t)blockIdx.x + 1;
   uint32_t s = 0;
   for (int64_t t = threadIdx.x; t < tile; t += kScanThreads) s += tile_sums[t];
@@ -307,21 +317,22 @@ int64_t scan_tmp_elems(int64_t len) { return (len + kScanTile - 1) / kScanTile +
 // Exclusive scan of len uint32 values (in == out allowed); tile_sums needs
 // scan_tmp_elems(len) entries.  flag / status: hand_on_flag.
 static int exclusive_scan(const uint32_t* in, uint32_t* out, int64_t len, uint32_t* tile_sums, const uint32_t* flag,
-                          uint32_t* status, cudaStream_t s) {
+                          uint32_t* status, bool early, cudaStream_t s) {
   if (len <= 0) return kOk;
   if (len <= kScanOne) {
-    scan_one_kernel<<<1, kScanThreads, 0, s>>>(in, out, len, flag, status);
+    PMB_CUDA_CHECK(launch_dependent(early, scan_one_kernel, 1, kScanThreads, 0, s, in, out, len, flag, status));
   } else {
     const int64_t ntiles = (len + kScanTile - 1) / kScanTile;
-    scan_tiles_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, out, len, tile_sums, flag, status);
-    scan_add_kernel<<<(unsigned)(ntiles - 1), kScanThreads, 0, s>>>(out, len, tile_sums);
+    PMB_CUDA_CHECK(launch_dependent(early, scan_tiles_kernel, (int)ntiles, kScanThreads, 0, s, in, out, len, tile_sums,
+                                    flag, status));
+    PMB_CUDA_CHECK(launch_dependent(early, scan_add_kernel, (int)(ntiles - 1), kScanThreads, 0, s, out, len,
+                                    tile_sums));
   }
-  PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
 
 int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t len, uint32_t* tile_sums, cudaStream_t s) {
-  return exclusive_scan(in, out, len, tile_sums, nullptr, nullptr, s);
+  return exclusive_scan(in, out, len, tile_sums, nullptr, nullptr, false, s);
 }
 
 int64_t bin_scratch_bytes(int64_t n, Mesh3 m) {
@@ -352,15 +363,16 @@ int bin_particles(const int16_t* pmid, float* disp, const float* vel, float drif
   p += align_up(4 * n, 256);
   uint32_t* tile_sums = (uint32_t*)p;
   PMB_CUDA_CHECK(cudaMemsetAsync(counts, 0, align_up(4 * len, 256) + 4, s));
-  const auto grid_of = [n](int per) { return (unsigned)((n + kSortThreads * per - 1) / (kSortThreads * per)); };
+  const bool early = small_mesh(m.nx, m.ny, m.nz);
+  const auto grid_of = [n](int per) { return (int)((n + kSortThreads * per - 1) / (kSortThreads * per)); };
   if (n > 0)
-    bin_count_kernel<<<grid_of(kSortPer), kSortThreads, 0, s>>>(pmid, disp, vel, drift, n, m, cell, sh, valid, counts,
-                                                             row_of, rank_of, flag);
-  int st = exclusive_scan(counts, offs, len, tile_sums, flag, status, s);
+    PMB_CUDA_CHECK(launch_dependent(early, bin_count_kernel, grid_of(kSortPer), kSortThreads, 0, s, pmid, disp, vel,
+                                    drift, n, m, cell, sh, valid, counts, row_of, rank_of, flag));
+  int st = exclusive_scan(counts, offs, len, tile_sums, flag, status, early, s);
   if (st != kOk) return st;
   if (n > 0)
-    bin_place_kernel<<<grid_of(1), kSortThreads, 0, s>>>(pmid, disp, n, m, cell, sh, offs, row_of, rank_of, rec, perm);
-  PMB_CUDA_CHECK(cudaGetLastError());
+    PMB_CUDA_CHECK(launch_dependent(early, bin_place_kernel, grid_of(1), kSortThreads, 0, s, pmid, disp, n, m, cell, sh,
+                                    offs, row_of, rank_of, rec, perm));
   return kOk;
 }
 
@@ -490,6 +502,8 @@ __global__ void __launch_bounds__(kRowThreads)
   constexpr int GROUPS = PLANE / 4;   // groups of four cells per plane
   constexpr int T = kRowThreads;
   static_assert(NZP % 4 == 0, "rows of whole groups");
+  wait_for_previous();
+  let_next_start();
   if (flagged(status)) return;
   const double scale = scale_dev != nullptr ? *scale_dev : scale_const;
   if (!(scale == scale)) {  // NaN scale: a non-finite value
@@ -791,10 +805,9 @@ static int launch_rows(const Rec* rec, const uint32_t* perm, const uint32_t* off
   PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
   const int dup = (m.nx == 1 ? 2 : 1) * (m.ny == 1 ? 2 : 1) * (m.nz == 1 ? 2 : 1);
   const int64_t nbx = (m.nx + RX - 1) / RX, nby = (m.ny + RY - 1) / RY;
-  k<<<(unsigned)(nbx * nby), kRowThreads, smem, s>>>(rec, perm, offs, m, fast_div((uint32_t)m.nz), fast_div((uint32_t)nby), val,
-                                           val_sorted, val_const, scale_dev, scale_const, E, dup, mode, src_mul, out,
-                                           status);
-  PMB_CUDA_CHECK(cudaGetLastError());
+  PMB_CUDA_CHECK(launch_dependent(small_mesh(m.nx, m.ny, m.nz), k, (int)(nbx * nby), kRowThreads, smem, s, rec, perm, offs, m,
+                                  fast_div((uint32_t)m.nz), fast_div((uint32_t)nby), val, val_sorted, val_const,
+                                  scale_dev, scale_const, E, dup, mode, src_mul, out, status));
   return kOk;
 }
 
@@ -1051,6 +1064,8 @@ __global__ void __launch_bounds__(kGatherThreads)
   __shared__ float s_val[kGatherTile * C];
   __shared__ uint32_t s_dst[kGatherTile];
   __shared__ bool s_masked[kGatherTile];
+  wait_for_previous();
+  let_next_start();
   if (flagged(status)) return;
   const int64_t base = (int64_t)blockIdx.x * kGatherTile;
   const int cnt = n - base < kGatherTile ? (int)(n - base) : kGatherTile;
@@ -1170,9 +1185,8 @@ int gather_sorted(const Rec* rec, const uint32_t* perm, const uint32_t* offs, in
   const int th = 256;
   const unsigned g = (unsigned)((n + th - 1) / th);
   if (C == 3) {
-    gather_kernel_x2<3><<<(unsigned)((n + kGatherTile - 1) / kGatherTile), kGatherThreads, 0, s>>>(
-        rec, perm, n, m, mesh, out, vel, kick, kick2, status);
-    PMB_CUDA_CHECK(cudaGetLastError());
+    PMB_CUDA_CHECK(launch_dependent(small_mesh(m.nx, m.ny, m.nz), gather_kernel_x2<3>,
+                                    (int)((n + kGatherTile - 1) / kGatherTile), kGatherThreads, 0, s, rec, perm, n, m, mesh, out, vel, kick, kick2, status));
     return kOk;
   }
   switch (C) {

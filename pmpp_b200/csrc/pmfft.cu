@@ -509,6 +509,9 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
   // y passes run the column tiles kz < zs; x passes the live (ky, kz tile)
   // columns; the forward y pass stores live ky rows only and the inverse y
   // pass loads them only (PIN / POUT)
+  for (int i = t; i < L; i += G::T) stw[i] = a.tw[i];
+  wait_for_previous();
+  let_next_start();
   constexpr bool PIN = (MODE == kYInv || MODE == kYInvYZ || MODE == kYInvAll);
   constexpr bool POUT = (MODE == kYFwd || MODE == kYFwdYZ);
   Live lv{a.ny, 0, a.P};
@@ -567,7 +570,6 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
     tab_batch = member_of(tab_batch);
     T = tables_at(a.tab_base + (int64_t)tab_batch * a.tab_stride, a.nx, a.ny, a.nz, a.has_masks);
   }
-  for (int i = t; i < L; i += G::T) stw[i] = a.tw[i];
   load_tables();
   __syncthreads();
   auto out_ch = [&](int batch, int chan) -> int64_t {
@@ -1083,6 +1085,8 @@ __global__ void __launch_bounds__(ZGeom<R1, R2>::T, ZGeom<R1, R2>::CTAS) z_r2c_k
   if (t == 0)
     for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
   load_z_twiddles<M>(a, tw);
+  wait_for_previous();
+  let_next_start();
   __syncthreads();
   auto issue = [&](int i) {
     if (i >= tiles_mine) return;
@@ -1181,6 +1185,8 @@ __global__ void __launch_bounds__(ZGeom<R1, R2>::T, ZGeom<R1, R2>::CTAS) z_c2r_k
   if (t == 0)
     for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
   load_z_twiddles<M>(a, tw);
+  wait_for_previous();
+  let_next_start();
   int zs = P;
   if constexpr (PR) zs = live_extents(a.prune_base, a.prune_stride, a.prune_count, a.nx, a.ny, a.nz).zs;
   __syncthreads();
@@ -1337,8 +1343,7 @@ int launch_col_ctas(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
   auto k = col_pass_kernel<R1, R2, S, MODE, CTAS, PR>;
   PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
   const int grid = persistent_grid(k, G::T, smem, a.ntiles);
-  k<<<grid, G::T, smem, s>>>(map, a);
-  PMB_CUDA_CHECK(cudaGetLastError());
+  PMB_CUDA_CHECK(launch_dependent(small_mesh(a.nx, a.ny, a.nz), k, grid, G::T, smem, s, map, a));
   return kOk;
 }
 
@@ -1408,8 +1413,7 @@ int launch_z(ZArgs a, int batch, cudaStream_t s) {
   auto k = C2R ? z_c2r_kernel<R1, R2, S, PR> : z_r2c_kernel<R1, R2, S>;
   PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
   const int grid = persistent_grid(k, G::T, smem, a.ntiles);
-  k<<<grid, G::T, smem, s>>>(a);
-  PMB_CUDA_CHECK(cudaGetLastError());
+  PMB_CUDA_CHECK(launch_dependent(small_mesh(a.nx, a.ny, a.nz), k, grid, G::T, smem, s, a));
   return kOk;
 }
 

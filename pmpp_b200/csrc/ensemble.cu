@@ -321,7 +321,7 @@ struct Ensemble {
   uint32_t* tile_sums = nullptr;
   void* fft_work = nullptr;
   int64_t fft_bytes = 0;
-  // the hand-written FFT pass chain (member meshes it supports): one work
+  // the hand-written FFT pass chain (power-of-two member meshes): one work
   // area of five blocked spectral channels, reused member after member
   void* pm_work = nullptr;
   int64_t pm_bytes = 0;

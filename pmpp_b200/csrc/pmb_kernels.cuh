@@ -96,7 +96,7 @@ int project_window(const float* mesh, Mesh3 m, int axis, int start, int stop, in
 // acc (n,3) from three planar (3,n) channels
 int interleave3(const float* planar, float* acc, int64_t n, cudaStream_t s);
 
-// pmfft.cu: hand-written FFT passes (sides 2^a or 3 2^a) over the
+// pmfft.cu: hand-written FFT passes for power-of-two meshes over the
 // y-blocked half-spectrum layout (see pmfft.cu for the layout and modes).
 bool pmfft_supported(Mesh3 m);
 int pmfft_row_len(Mesh3 m);

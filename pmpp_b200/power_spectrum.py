@@ -68,12 +68,14 @@ def shell_statistics(conf, device=None):
 def _spectrum(delta, conf):
     """rFFT of delta: (spectrum, blocked).  Meshes of the hand-written pass chain
     take its z, y and x passes and keep its blocked layout (blocked = 1, a flat
-    tensor), the others (and fields that are not 16-byte aligned) cuFFT."""
+    tensor), the others cuFFT."""
     nx, ny, nz = conf.mesh_shape
     dev = delta.device
     s = stream_handle(dev)
     x = delta.to(torch.float32).contiguous()
-    if pmfft_active(nx, ny, nz) and x.data_ptr() % 16 == 0:
+    if pmfft_active(nx, ny, nz):
+        if x.data_ptr() % 16:  # the z pass loads whole 16-byte words
+            x = x.clone()
         n = lib().pmb_pmfft_channel_elems(nx, ny, nz)
         spec = torch.empty(n, dtype=torch.complex64, device=dev)
         tmp = workspace(8 * n, dev, "pk_pm")

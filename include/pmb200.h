@@ -441,18 +441,11 @@ int pmb_lpt_vjp(const void* modes, int gx, int gy, int gz, float cell_vol, const
  * [nx ny nz/2+1].  With spec_b, also the auto sums of b and the cross sums. */
 int pmb_pk_shells(const void* spec, int nx, int ny, int nz, const float* sinc_tab, int mas_power, int num_shells,
                   double* sums, const void* spec_b, double* sums_b, double* sums_x, void* stream);
-/* pmb_pk_shells of a spectrum in the pass chain's blocked layout (blocked != 0,
- * meshes of pmb_pmfft_supported) or in order. */
-int pmb_pk_shells2(const void* spec, int nx, int ny, int nz, int blocked, const float* sinc_tab, int mas_power,
-                   int num_shells, double* sums, const void* spec_b, double* sums_b, double* sums_x, void* stream);
 /* Mode counts and sum of |n| * mult per shell (power_spectrum.py:46-74). */
 int pmb_shell_stats(int nx, int ny, int nz, int num_shells, double* counts, double* ksum, void* stream);
 /* Adjoint of the shell power: out = 2 spec W^-2p wshell[shell] * post. */
 int pmb_pk_shells_adjoint(const void* spec, int nx, int ny, int nz, const float* sinc_tab, int mas_power,
                           int num_shells, const double* wshell, float post, void* out, void* stream);
-/* ... in the blocked layout (padding columns written as zeros) or in order. */
-int pmb_pk_shells_adjoint2(const void* spec, int nx, int ny, int nz, int blocked, const float* sinc_tab,
-                           int mas_power, int num_shells, const double* wshell, float post, void* out, void* stream);
 /* delta = rho / (total / n) - 1 (power_spectrum.py:371-374). */
 int pmb_overdensity(const float* rho, float* delta, int64_t n, const double* total, void* stream);
 

@@ -100,8 +100,6 @@ _SIGS = {
     "pmb_lpt_vjp_workspace_bytes": (c_i64, [c_int, c_int, c_int]),
     "pmb_lpt_vjp": (c_int, [c_p, c_int, c_int, c_int, c_f, c_p, c_int, c_f, c_f, c_f, c_f, c_p, c_p, c_p, c_p, c_i64,
                             c_p, c_p, c_p, c_p, c_i64, c_p]),
-    "pmb_pk_shells2": (c_int, [c_p, c_int, c_int, c_int, c_int, c_p, c_int, c_int, c_p, c_p, c_p, c_p, c_p]),
-    "pmb_pk_shells_adjoint2": (c_int, [c_p, c_int, c_int, c_int, c_int, c_p, c_int, c_int, c_p, c_f, c_p, c_p]),
     "pmb_pk_shells": (c_int, [c_p, c_int, c_int, c_int, c_p, c_int, c_int, c_p, c_p, c_p, c_p, c_p]),
     "pmb_shell_stats": (c_int, [c_int, c_int, c_int, c_int, c_p, c_p, c_p]),
     "pmb_pk_shells_adjoint": (c_int, [c_p, c_int, c_int, c_int, c_p, c_int, c_int, c_p, c_f, c_p, c_p]),
@@ -207,7 +205,7 @@ _KERNELS = {
     "pmb_kick_adj": 1, "pmb_kick_adj2": 1, "pmb_kick_adj3": 1, "pmb_drift_cot_adj": 1, "pmb_drift_adj": 1, "pmb_dot": 1,
     "pmb_force": 9, "pmb_force2": 9, "pmb_force_streamed": 14, "pmb_force_vjp": 11, "pmb_force_vjp_presorted": 6, "pmb_sum": 1,
     "pmb_white_noise_nested": 1, "pmb_linear_modes": 1,
-    "pmb_lpt": 4, "pmb_lpt_lattice": 4, "pmb_lpt_vjp": 6, "pmb_pk_shells": 1, "pmb_pk_shells2": 1, "pmb_pk_shells_adjoint2": 1, "pmb_shell_stats": 1, "pmb_pk_shells_adjoint": 1,
+    "pmb_lpt": 4, "pmb_lpt_lattice": 4, "pmb_lpt_vjp": 6, "pmb_pk_shells": 1, "pmb_shell_stats": 1, "pmb_pk_shells_adjoint": 1,
     "pmb_overdensity": 1, "pmb_ens_force": 7, "pmb_ens_step": 9, "pmb_ens_set_step": 1,
     "pmb_force64": 5, "pmb_force64_interlaced": 7, "pmb_force_vjp64_interlaced": 6, "pmb_deposit64": 1, "pmb_axpy64": 1, "pmb_sum64": 1, "pmb_force_vjp64": 4, "pmb_dot64": 1, "pmb_lpt64_ex": 4, "pmb_lpt_vjp64": 6,
     "pmb_scatter_vjp64": 1, "pmb_white_noise_nested64": 1,

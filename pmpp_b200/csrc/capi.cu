@@ -915,14 +915,9 @@ int pmb_lpt_vjp(const void* modes, int gx, int gy, int gz, float cell_vol, const
 // ---------------------------------------------------------------------------
 // Power spectrum
 // ---------------------------------------------------------------------------
-// Row length of a spectrum given in the pass chain's blocked layout (0: rows in order).
-static int spec_pitch(Mesh3 m, int blocked) { return blocked ? pmfft_row_len(m) : 0; }
-
-int pmb_pk_shells2(const void* spec, int nx, int ny, int nz, int blocked, const float* sinc_tab, int mas_power,
-                   int num_shells, double* sums, const void* spec_b, double* sums_b, double* sums_x, void* stream) {
-  Mesh3 m{nx, ny, nz};
+int pmb_pk_shells(const void* spec, int nx, int ny, int nz, const float* sinc_tab, int mas_power, int num_shells,
+                  double* sums, const void* spec_b, double* sums_b, double* sums_x, void* stream) {
   PMB_REQUIRE(nx > 0 && ny > 0 && nz > 0 && num_shells > 0, "pmb_pk_shells: bad arguments");
-  PMB_REQUIRE(!blocked || pmfft_supported(m), "pmb_pk_shells: no blocked layout for this mesh");
   PMB_REQUIRE(spec_b == nullptr || (sums_b != nullptr && sums_x != nullptr), "pmb_pk_shells: cross sums missing");
   cudaStream_t s = S(stream);
   PMB_CUDA_CHECK(cudaMemsetAsync(sums, 0, sizeof(double) * num_shells, s));
@@ -930,13 +925,8 @@ int pmb_pk_shells2(const void* spec, int nx, int ny, int nz, int blocked, const 
     PMB_CUDA_CHECK(cudaMemsetAsync(sums_b, 0, sizeof(double) * num_shells, s));
     PMB_CUDA_CHECK(cudaMemsetAsync(sums_x, 0, sizeof(double) * num_shells, s));
   }
-  return pk_shells((const float2*)spec, m, sinc_tab, mas_power, num_shells, spec_pitch(m, blocked), sums,
+  return pk_shells((const float2*)spec, Mesh3{nx, ny, nz}, sinc_tab, mas_power, num_shells, sums,
                    (const float2*)spec_b, sums_b, sums_x, s);
-}
-
-int pmb_pk_shells(const void* spec, int nx, int ny, int nz, const float* sinc_tab, int mas_power, int num_shells,
-                  double* sums, const void* spec_b, double* sums_b, double* sums_x, void* stream) {
-  return pmb_pk_shells2(spec, nx, ny, nz, 0, sinc_tab, mas_power, num_shells, sums, spec_b, sums_b, sums_x, stream);
 }
 
 int pmb_shell_stats(int nx, int ny, int nz, int num_shells, double* counts, double* ksum, void* stream) {
@@ -947,18 +937,11 @@ int pmb_shell_stats(int nx, int ny, int nz, int num_shells, double* counts, doub
   return shell_stats(Mesh3{nx, ny, nz}, num_shells, counts, ksum, s);
 }
 
-int pmb_pk_shells_adjoint2(const void* spec, int nx, int ny, int nz, int blocked, const float* sinc_tab,
-                           int mas_power, int num_shells, const double* wshell, float post, void* out, void* stream) {
-  Mesh3 m{nx, ny, nz};
-  PMB_REQUIRE(nx > 0 && ny > 0 && nz > 0 && num_shells > 0, "pmb_pk_shells_adjoint: bad arguments");
-  PMB_REQUIRE(!blocked || pmfft_supported(m), "pmb_pk_shells_adjoint: no blocked layout for this mesh");
-  return pk_shells_adjoint((const float2*)spec, m, sinc_tab, mas_power, num_shells, spec_pitch(m, blocked), wshell,
-                           post, (float2*)out, S(stream));
-}
-
 int pmb_pk_shells_adjoint(const void* spec, int nx, int ny, int nz, const float* sinc_tab, int mas_power,
                           int num_shells, const double* wshell, float post, void* out, void* stream) {
-  return pmb_pk_shells_adjoint2(spec, nx, ny, nz, 0, sinc_tab, mas_power, num_shells, wshell, post, out, stream);
+  PMB_REQUIRE(nx > 0 && ny > 0 && nz > 0 && num_shells > 0, "pmb_pk_shells_adjoint: bad arguments");
+  return pk_shells_adjoint((const float2*)spec, Mesh3{nx, ny, nz}, sinc_tab, mas_power, num_shells, wshell, post,
+                           (float2*)out, S(stream));
 }
 
 int pmb_overdensity(const float* rho, float* delta, int64_t n, const double* total, void* stream) {

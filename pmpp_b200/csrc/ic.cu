@@ -693,13 +693,6 @@ __device__ __forceinline__ int shell_of(long long n2, int num_shells) {
   return r < num_shells - 1 ? (int)r : num_shells - 1;
 }
 
-// First value of spectral row (x, y): rows of nz / 2 + 1 in order, or (pitch >
-// 0) the pass chain's layout of blocks of 32 y rows with that pitch (pmfft.cu).
-__device__ __forceinline__ int64_t spec_row_at(int ix, int iy, Mesh3 m, int pitch) {
-  return pitch > 0 ? (((int64_t)(iy >> 5) * m.nx + ix) * 32 + (iy & 31)) * pitch
-                   : ((int64_t)ix * m.ny + iy) * (m.nz / 2 + 1);
-}
-
 // w^-2p
 __device__ __forceinline__ double window_pow(double w, int p) {
   double x = 1.0;
@@ -740,7 +733,7 @@ __device__ __forceinline__ void add_runs(double v, int shell, double* hist, bool
 template <class T, bool CROSS>
 __global__ void __launch_bounds__(kPkThreads)
     pk_shells_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                     int mas_power, int num_shells, int copies, int pitch, double* __restrict__ sums,
+                     int mas_power, int num_shells, int copies, double* __restrict__ sums,
                      const typename Real<T>::T2* __restrict__ spec_b, double* __restrict__ sums_b,
                      double* __restrict__ sums_x) {
   using T2 = typename Real<T>::T2;
@@ -762,9 +755,8 @@ __global__ void __launch_bounds__(kPkThreads)
     const int ix = (int)(row / m.ny), iy = (int)(row - (int64_t)ix * m.ny);
     const long long mx = fft_mode(ix, m.nx), my = fft_mode(iy, m.ny), r2 = mx * mx + my * my;
     const double rf = mas_power > 0 ? window_pow((double)sx[ix] * (double)sy[iy], mas_power) : 1.0;
-    const int64_t at = spec_row_at(ix, iy, m, pitch);
-    const T2* a = spec + at;
-    const T2* b = CROSS ? spec_b + at : nullptr;
+    const T2* a = spec + row * nzh;
+    const T2* b = CROSS ? spec_b + row * nzh : nullptr;
     for (int k0 = lane; k0 - lane < nzh; k0 += 32 * UN) {
       T2 va[UN], vb[UN];
 #pragma unroll
@@ -800,8 +792,8 @@ __global__ void __launch_bounds__(kPkThreads)
 
 template <class T, bool CROSS>
 static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
-                            int num_shells, int pitch, double* sums, const typename Real<T>::T2* spec_b,
-                            double* sums_b, double* sums_x, cudaStream_t s) {
+                            int num_shells, double* sums, const typename Real<T>::T2* spec_b, double* sums_b,
+                            double* sums_x, cudaStream_t s) {
   // a copy of the sums per warp where that leaves room for two blocks on an SM
   const int64_t table = 8 * (m.nz / 2 + 1), one = (int64_t)8 * (CROSS ? 3 : 1) * num_shells;
   int copies = kPkWarps;
@@ -815,37 +807,36 @@ static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* 
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * per_sm) grid = 148 * per_sm;
   k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, (size_t)smem, s>>>(spec, m, sinc_tab, mas_power, num_shells,
-                                                                      copies, pitch, sums, spec_b, sums_b, sums_x);
+                                                                      copies, sums, spec_b, sums_b, sums_x);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
 
-int pk_shells(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, int pitch,
-              double* sums, const float2* spec_b, double* sums_b, double* sums_x, cudaStream_t s) {
-  return spec_b != nullptr ? launch_pk_shells<float, true>(spec, m, sinc_tab, mas_power, num_shells, pitch, sums,
-                                                           spec_b, sums_b, sums_x, s)
-                           : launch_pk_shells<float, false>(spec, m, sinc_tab, mas_power, num_shells, pitch, sums,
-                                                            nullptr, nullptr, nullptr, s);
+int pk_shells(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, double* sums,
+              const float2* spec_b, double* sums_b, double* sums_x, cudaStream_t s) {
+  return spec_b != nullptr
+             ? launch_pk_shells<float, true>(spec, m, sinc_tab, mas_power, num_shells, sums, spec_b, sums_b, sums_x, s)
+             : launch_pk_shells<float, false>(spec, m, sinc_tab, mas_power, num_shells, sums, nullptr, nullptr,
+                                              nullptr, s);
 }
 
 int pk_shells64(const double2* spec, Mesh3 m, const double* sinc_tab, int mas_power, int num_shells, double* sums,
                 cudaStream_t s) {
-  return launch_pk_shells<double, false>(spec, m, sinc_tab, mas_power, num_shells, 0, sums, nullptr, nullptr, nullptr,
-                                         s);
+  return launch_pk_shells<double, false>(spec, m, sinc_tab, mas_power, num_shells, sums, nullptr, nullptr, nullptr, s);
 }
 
 // Adjoint of the shell power: given dL/dP_shell (already divided by nmodes and
 // times the normalisation), out = 2 * spec * deconv * w_shell * (1/mult) so
 // that M * irfftn(out) is the real-field cotangent (rfftn^T for the
 // Hermitian-consistent spectrum; the multiplicity cancels against the 1/mult
-// of the rFFT transpose); out may be spec.  Rows and tables as in pk_shells_kernel: 506 -> 243 us
+// of the rFFT transpose).  Rows and tables as in pk_shells_kernel: 506 -> 243 us
 // for a 512^3 mesh, 164 us for the bytes.
 // T = double: the float64 build's form.
 template <class T>
 __global__ void __launch_bounds__(kPkThreads)
-    pk_shells_adjoint_kernel(const typename Real<T>::T2* spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                             int mas_power, int num_shells, int pitch, const double* __restrict__ wshell,
-                             double post, typename Real<T>::T2* out) {
+    pk_shells_adjoint_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
+                             int mas_power, int num_shells, const double* __restrict__ wshell, double post,
+                             typename Real<T>::T2* __restrict__ out) {
   using T2 = typename Real<T>::T2;
   constexpr int UN = 4;
   extern __shared__ double zf[];
@@ -860,10 +851,8 @@ __global__ void __launch_bounds__(kPkThreads)
     const int ix = (int)(row / m.ny), iy = (int)(row - (int64_t)ix * m.ny);
     const long long mx = fft_mode(ix, m.nx), my = fft_mode(iy, m.ny), r2 = mx * mx + my * my;
     const double rf = 2.0 * post * (mas_power > 0 ? window_pow((double)sx[ix] * (double)sy[iy], mas_power) : 1.0);
-    const int64_t at = spec_row_at(ix, iy, m, pitch);
-    const T2* a = spec + at;
-    T2* o = out + at;
-    if (lane < pitch - nzh) o[nzh + lane] = Real<T>::make2((T)0, (T)0);  // padding columns (seven)
+    const T2* a = spec + row * nzh;
+    T2* o = out + row * nzh;
     for (int k0 = lane; k0 < nzh; k0 += 32 * UN) {
       T2 v[UN];
 #pragma unroll
@@ -883,24 +872,24 @@ __global__ void __launch_bounds__(kPkThreads)
 
 template <class T>
 static int launch_pk_adjoint(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
-                             int num_shells, int pitch, const double* wshell, double post,
-                             typename Real<T>::T2* out, cudaStream_t s) {
+                             int num_shells, const double* wshell, double post, typename Real<T>::T2* out,
+                             cudaStream_t s) {
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * 8) grid = 148 * 8;
   pk_shells_adjoint_kernel<T><<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, 8 * (m.nz / 2 + 1), s>>>(
-      spec, m, sinc_tab, mas_power, num_shells, pitch, wshell, post, out);
+      spec, m, sinc_tab, mas_power, num_shells, wshell, post, out);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
 
-int pk_shells_adjoint(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, int pitch,
+int pk_shells_adjoint(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells,
                       const double* wshell, float post, float2* out, cudaStream_t s) {
-  return launch_pk_adjoint<float>(spec, m, sinc_tab, mas_power, num_shells, pitch, wshell, (double)post, out, s);
+  return launch_pk_adjoint<float>(spec, m, sinc_tab, mas_power, num_shells, wshell, (double)post, out, s);
 }
 
 int pk_shells_adjoint64(const double2* spec, Mesh3 m, const double* sinc_tab, int mas_power, int num_shells,
                         const double* wshell, double post, double2* out, cudaStream_t s) {
-  return launch_pk_adjoint<double>(spec, m, sinc_tab, mas_power, num_shells, 0, wshell, post, out, s);
+  return launch_pk_adjoint<double>(spec, m, sinc_tab, mas_power, num_shells, wshell, post, out, s);
 }
 
 // Shell mode counts and mean |n| (power_spectrum.py:46-74), FP64.

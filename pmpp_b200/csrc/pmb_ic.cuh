@@ -34,10 +34,9 @@ int lpt_grad2_adjoint(const float2* F2, float2* out, Mesh3 m, const float* tab, 
 int lpt_source_adjoint(const float* s6, const float* Lc, float* c6, int64_t n, cudaStream_t s);
 int lpt_modes_adjoint(const float2* F1, const float2* FS, const float* amp, float2* out, Mesh3 m, const float* tab,
                       float scale, cudaStream_t s);
-// pitch: 0 for rows of nz / 2 + 1, or the pass chain's row length
-int pk_shells(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, int pitch,
-              double* sums, const float2* spec_b, double* sums_b, double* sums_x, cudaStream_t s);
-int pk_shells_adjoint(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, int pitch,
+int pk_shells(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells, double* sums,
+              const float2* spec_b, double* sums_b, double* sums_x, cudaStream_t s);
+int pk_shells_adjoint(const float2* spec, Mesh3 m, const float* sinc_tab, int mas_power, int num_shells,
                       const double* wshell, float post, float2* out, cudaStream_t s);
 int overdensity(const float* rho, float* delta, int64_t n, const double* total, cudaStream_t s);
 int shell_stats(Mesh3 m, int num_shells, double* counts, double* ksum, cudaStream_t s);

@@ -16,7 +16,7 @@ import math
 import numpy as np
 import torch
 
-from ._lib import call, lib, pmfft_active
+from ._lib import call, lib
 from .cic import SortedParticles
 from .runtime import stream_handle, workspace
 
@@ -66,56 +66,23 @@ def shell_statistics(conf, device=None):
 
 
 def _spectrum(delta, conf):
-    """rFFT of delta: (spectrum, blocked).  Meshes of the hand-written pass chain
-    take its z, y and x passes and keep its blocked layout (blocked = 1, a flat
-    tensor), the others cuFFT."""
     nx, ny, nz = conf.mesh_shape
     dev = delta.device
-    s = stream_handle(dev)
     x = delta.to(torch.float32).contiguous()
-    if pmfft_active(nx, ny, nz):
-        if x.data_ptr() % 16:  # the z pass loads whole 16-byte words
-            x = x.clone()
-        n = lib().pmb_pmfft_channel_elems(nx, ny, nz)
-        spec = torch.empty(n, dtype=torch.complex64, device=dev)
-        tmp = workspace(8 * n, dev, "pk_pm")
-        call("pmb_pmfft_z", nx, ny, nz, 0, 1, x.data_ptr(), spec.data_ptr(), s)
-        call("pmb_pmfft_col", nx, ny, nz, 0, 1, 0, spec.data_ptr(), tmp.data_ptr(), None, 0, None, None, 0, 1.0, s)
-        call("pmb_pmfft_col", nx, ny, nz, 4, 1, 0, tmp.data_ptr(), spec.data_ptr(), None, 0, None, None, 0, 1.0, s)
-        return spec, 1
     spec = torch.empty((nx, ny, nz // 2 + 1), dtype=torch.complex64, device=dev)
     w = workspace(lib().pmb_fft_work_bytes(nx, ny, nz, 1), dev, "fft1")
-    call("pmb_rfft3", nx, ny, nz, 1, x.data_ptr(), spec.data_ptr(), w.data_ptr(), s)
-    return spec, 0
+    call("pmb_rfft3", nx, ny, nz, 1, x.data_ptr(), spec.data_ptr(), w.data_ptr(), stream_handle(dev))
+    return spec
 
 
-def _field(spec, blocked, conf):
-    """Unnormalised inverse of _spectrum's result (overwritten), a real mesh (1, nx, ny, nz)."""
-    nx, ny, nz = conf.mesh_shape
-    dev = spec.device
-    s = stream_handle(dev)
-    out = torch.empty((1, nx, ny, nz), dtype=torch.float32, device=dev)
-    if blocked:
-        tmp = workspace(8 * spec.numel(), dev, "pk_pm")
-        call("pmb_pmfft_col", nx, ny, nz, 5, 1, 0, spec.data_ptr(), tmp.data_ptr(), None, 0, None, None, 0, 1.0, s)
-        call("pmb_pmfft_col", nx, ny, nz, 1, 1, 0, tmp.data_ptr(), spec.data_ptr(), None, 0, None, None, 0, 1.0, s)
-        call("pmb_pmfft_z", nx, ny, nz, 1, 1, spec.data_ptr(), out.data_ptr(), s)
-    else:
-        w = workspace(lib().pmb_fft_work_bytes(nx, ny, nz, 1), dev, "fft1")
-        call("pmb_irfft3", nx, ny, nz, 1, spec.data_ptr(), out.data_ptr(), w.data_ptr(), s)
-    return out
-
-
-def _shell_sums(spectrum, conf, mas_power, spectrum_b=None):
-    spec, blocked = spectrum
-    spec_b = None if spectrum_b is None else spectrum_b[0]
+def _shell_sums(spec, conf, mas_power, spec_b=None):
     nx, ny, nz = conf.mesh_shape
     dev = spec.device
     ns = num_shells(conf)
     sums = torch.empty(ns, dtype=torch.float64, device=dev)
     sb = torch.empty(ns, dtype=torch.float64, device=dev) if spec_b is not None else None
     sx = torch.empty(ns, dtype=torch.float64, device=dev) if spec_b is not None else None
-    call("pmb_pk_shells2", spec.data_ptr(), nx, ny, nz, blocked, _sinc_tables(conf, dev).data_ptr(), mas_power, ns,
+    call("pmb_pk_shells", spec.data_ptr(), nx, ny, nz, _sinc_tables(conf, dev).data_ptr(), mas_power, ns,
          sums.data_ptr(), None if spec_b is None else spec_b.data_ptr(), None if sb is None else sb.data_ptr(),
          None if sx is None else sx.data_ptr(), stream_handle(dev))
     return sums, sb, sx
@@ -227,8 +194,8 @@ def pk_loss(ptcl, conf, pk_target, mas="CIC", grad=True, kmax=None):
     call("pmb_sum", rho.data_ptr(), rho.numel(), tot.data_ptr(), s)
     delta = torch.empty_like(rho)
     call("pmb_overdensity", rho.data_ptr(), delta.data_ptr(), rho.numel(), tot.data_ptr(), s)
-    spectrum = _spectrum(delta, conf)
-    sums, _, _ = _shell_sums(spectrum, conf, mp)
+    spec = _spectrum(delta, conf)
+    sums, _, _ = _shell_sums(spec, conf, mp)
     k, pk, nmodes = _finalize(sums, conf)
     tgt = np.asarray(pk_target, dtype=np.float64)
     valid = (nmodes > 0) & (pk > 0) & (tgt > 0)
@@ -244,15 +211,16 @@ def pk_loss(ptcl, conf, pk_target, mas="CIC", grad=True, kmax=None):
     w = np.zeros(num_shells(conf))
     w[1:] = np.where(valid, 2 * lr / nv / np.where(valid, pk, 1.0), 0.0) * norm / np.maximum(nmodes, 1)
     wd = torch.from_numpy(w).to(dev)
-    spec, blocked = spectrum
-    gspec = spec  # in place: every mode is read once, by the thread that writes it
-    call("pmb_pk_shells_adjoint2", spec.data_ptr(), nx, ny, nz, blocked, _sinc_tables(conf, dev).data_ptr(), mp,
-         len(w), wd.data_ptr(), 1.0, gspec.data_ptr(), s)
+    gspec = torch.empty_like(spec)
+    call("pmb_pk_shells_adjoint", spec.data_ptr(), nx, ny, nz, _sinc_tables(conf, dev).data_ptr(), mp, len(w),
+         wd.data_ptr(), 1.0, gspec.data_ptr(), s)
     # delta = rho / m - 1 with m = sum(rho)/M: rho_cot = (dcot - sum(dcot delta)/M) / m.
     # The sum is 2 sum_s w_s S_s over the shell sums S_s (gspec is 2 w_s times the
     # spectrum), so the constant enters as the zero mode and 1 / m as the particle value
     gspec.view(-1)[:1].fill_(-2.0 * float(np.dot(w, sums.cpu().numpy())) / rho.numel())
     m = float(tot.item()) / rho.numel()
-    dcot = _field(gspec, blocked, conf)
+    fw = workspace(lib().pmb_fft_work_bytes(nx, ny, nz, 1), dev, "fft1")
+    dcot = torch.empty((1, nx, ny, nz), dtype=torch.float32, device=dev)
+    call("pmb_irfft3", nx, ny, nz, 1, gspec.data_ptr(), dcot.data_ptr(), fw.data_ptr(), s)
     disp_cot, _ = sp.interp_grad(dcot, u_const=float(conf.mesh_size / conf.ptcl_num) / m)
     return loss, disp_cot

@@ -1,11 +1,11 @@
 """Shell sums, their adjoint and the overdensity at the edges of their loops:
-odd and tiny row lengths, meshes of the FFT pass chain (blocked rows) against
-rows in order, cross sums, lengths with remainders, NaN and misaligned fields.
+odd and tiny row lengths, cross sums, lengths with remainders, NaN and misaligned
+fields.
 
 Bars: against float64 transforms 1e-5 of each shell's power (float32
-transforms); between the layouts the same float64 terms in another order, 1e-12;
-the adjoint is element by element, so exact; the overdensity within one rounding
-of each of its two operations (2^-22 of rho / mean + 1)."""
+transforms); the overdensity within one rounding of each of its two operations
+(2^-22 of rho / mean + 1).
+"""
 import numpy as np
 import pytest
 import torch
@@ -18,81 +18,62 @@ def _conf(shape):
     return pb.Configuration(2.0, shape, 1, device="cuda")
 
 
-def _reference(a, b, shape, ns, power):
+def _shells(shape, ns):
     nx, ny, nz = shape
     md = lambda n: np.where(np.arange(n) < (n + 1) // 2, np.arange(n), np.arange(n) - n).astype(np.int64)
-    mx, my, mz = np.meshgrid(md(nx), md(ny), np.arange(nz // 2 + 1), indexing="ij")
-    shell = np.minimum(np.floor(np.sqrt(mx * mx + my * my + mz * mz) + 1e-9).astype(int), ns - 1)
+    n = np.meshgrid(md(nx), md(ny), np.arange(nz // 2 + 1), indexing="ij")
+    return np.minimum(np.floor(np.sqrt(n[0]**2 + n[1]**2 + n[2]**2) + 1e-9).astype(int), ns - 1), n
+
+
+def _reference(a, b, shape, ns, power):
+    shell, (mx, my, mz) = _shells(shape, ns)
+    nx, ny, nz = shape
     w = (np.sinc(mx / nx) * np.sinc(my / ny) * np.sinc(mz / nz))**-(2.0 * power)
     mult = np.where((mz == 0) | ((nz % 2 == 0) & (mz == nz // 2)), 1.0, 2.0)
     t = (a.real * b.real + a.imag * b.imag) * w * mult
-    add = lambda v: np.bincount(shell.ravel(), v.ravel(), minlength=ns)[:ns]
-    return add(t)
+    return np.bincount(shell.ravel(), t.ravel(), minlength=ns)[:ns]
 
 
 @pytest.mark.parametrize("shape", [(4, 4, 4), (5, 3, 7), (9, 8, 65), (3, 2, 1), (2, 70, 130), (64, 64, 128),
                                    (64, 96, 128)])
 @pytest.mark.parametrize("mas", [None, "CIC"])
-def test_shell_sums_both_layouts_and_cross(shape, mas):
-    from pmpp_b200 import _lib, power_spectrum as ps
+def test_shell_sums_and_cross(shape, mas):
+    from pmpp_b200 import power_spectrum as ps
     conf = _conf(shape)
     g = torch.Generator(device="cuda").manual_seed(3)
     x, y = (torch.randn(shape, generator=g, device="cuda") for _ in range(2))
     p = ps._mas(mas)
-    res = {}
-    try:
-        for on in (True, False):
-            _lib.set_pmfft(on)
-            res[on] = [s.cpu().numpy() for s in ps._shell_sums(ps._spectrum(x, conf), conf, p, ps._spectrum(y, conf))]
-    finally:
-        _lib.set_pmfft(True)
+    got = [s.cpu().numpy() for s in ps._shell_sums(ps._spectrum(x, conf), conf, p, ps._spectrum(y, conf))]
     fa, fb = (np.fft.rfftn(t.cpu().numpy().astype(np.float64)) for t in (x, y))
     ns = ps.num_shells(conf)
     auto = [_reference(u, u, shape, ns, p) for u in (fa, fb)]
     bars = [1e-5 * v for v in (auto[0], auto[1], np.sqrt(auto[0] * auto[1]))]  # float32 transforms
     for i, ref in enumerate(auto + [_reference(fa, fb, shape, ns, p)]):
-        for on in (True, False):
-            assert np.all(np.abs(res[on][i] - ref) <= bars[i])
+        assert np.all(np.abs(got[i] - ref) <= bars[i])
 
 
-@pytest.mark.parametrize("shape", [(64, 64, 128), (96, 64, 128)])
-def test_blocked_layout_equals_rows_in_order(shape):
+@pytest.mark.parametrize("shape", [(4, 4, 4), (5, 3, 7), (9, 8, 65), (3, 2, 1), (2, 70, 130)])
+def test_adjoint_rows(shape):
+    """out = spec * 2 post W^-2p w[shell], in float64 and rounded once (bar 2^-22)."""
     from pmpp_b200 import power_spectrum as ps
     from pmpp_b200._lib import call
     from pmpp_b200.runtime import stream_handle
-    nx, ny, nz = shape
-    nzh = nz // 2 + 1
     conf = _conf(shape)
-    x = torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda")
-    spec, blocked = ps._spectrum(x, conf)
-    assert blocked
-    rows = lambda t: t.view(ny // 32, nx, 32, -1).permute(1, 0, 2, 3).reshape(nx, ny, -1)
-    flat = rows(spec)[..., :nzh].contiguous()
-    a, _, _ = ps._shell_sums((spec, 1), conf, 2)
-    b, _, _ = ps._shell_sums((flat, 0), conf, 2)
-    np.testing.assert_allclose(a.cpu().numpy(), b.cpu().numpy(), rtol=1e-12)
     ns = ps.num_shells(conf)
-    w = torch.randn(ns, dtype=torch.float64, device="cuda")
+    rng = np.random.default_rng(7)
+    nzh = shape[2] // 2 + 1
+    spec = (rng.normal(size=shape[:2] + (nzh, )) + 1j * rng.normal(size=shape[:2] + (nzh, ))).astype(np.complex64)
+    w = rng.normal(size=ns)
+    x, wd = torch.from_numpy(spec).cuda(), torch.from_numpy(w).cuda()
+    out = torch.full_like(x, float("nan"))
     tab = ps._sinc_tables(conf, x.device)
-    s = stream_handle(x.device)
-    out = [torch.full_like(t, float("nan")) for t in (spec, flat)]
-    for t, o, blk in ((spec, out[0], 1), (flat, out[1], 0)):
-        call("pmb_pk_shells_adjoint2", t.data_ptr(), nx, ny, nz, blk, tab.data_ptr(), 2, ns, w.data_ptr(), 0.5,
-             o.data_ptr(), s)
-    got = rows(out[0])
-    assert torch.equal(got[..., :nzh], out[1]) and not bool(got[..., nzh:].abs().sum())
-    call("pmb_pk_shells_adjoint2", spec.data_ptr(), nx, ny, nz, 1, tab.data_ptr(), 2, ns, w.data_ptr(), 0.5,
-         spec.data_ptr(), s)  # in place
-    assert torch.equal(rows(spec), got)
-
-
-def test_misaligned_field_stays_refused():
-    from pmpp_b200 import power_spectrum as ps
-    from pmpp_b200._lib import PMBError
-    conf = _conf((64, 64, 128))
-    buf = torch.zeros(64 * 64 * 128 + 1, device="cuda")
-    with pytest.raises(PMBError):
-        ps.delta_to_pk(buf[1:].view(64, 64, 128), conf)
+    call("pmb_pk_shells_adjoint", x.data_ptr(), *shape, tab.data_ptr(), 2, ns, wd.data_ptr(), 0.5, out.data_ptr(),
+         stream_handle(x.device))
+    t = np.split(tab.cpu().numpy().astype(np.float64), np.cumsum(shape[:2]))
+    shell, _ = _shells(shape, ns)
+    ref = spec.astype(complex) * (t[0][:, None, None] * t[1][:, None] * t[2])**-4.0 * w[shell]
+    got = out.cpu().numpy()
+    assert np.all(np.abs(got - ref) <= 2.0**-22 * np.abs(ref))
 
 
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4097, 100003])

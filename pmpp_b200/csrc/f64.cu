@@ -143,8 +143,8 @@ __global__ void green64_kernel(const double2* __restrict__ src, double2* __restr
 }
 
 // acc = CIC gather of the three force meshes; optional vel += acc * kick.  A
-// thread per component, so that a particle's 24 loads are in flight in three
-// warps and neighbouring lanes store neighbouring values (29.7 -> 24.5 us for
+// thread per component, so that three threads have a particle's 24 loads in flight
+// and neighbouring lanes store neighbouring values (29.7 -> 24.5 us for
 // 64^3 particles on 128^3 cells; bound by the L2 sectors of the corners).
 __global__ void gather64_kernel(const int16_t* __restrict__ pmid, const double* __restrict__ disp, int64_t n, Mesh3 m,
                                 double cell, const double* __restrict__ mesh, double* __restrict__ acc,

@@ -548,8 +548,8 @@ static int force_vjp64_impl(const int16_t* pmid, const double* disp, int64_t n, 
     deposit64v_kernel<3><<<grid_for(n, 256), 256, 0, s>>>(pmid, disp, n, m, cell, acc_cot, mesh3);
   PMB_CUDA_CHECK(cudaGetLastError());
   F64_TRY(fft_d2z(m, 3, mesh3, spec3, work, s));
-  green64_adjoint_kernel<<<grid_for(m.half_cells(), 256), 256, 0, s>>>(spec3, spec1, m, tables64(tables, m, has_masks),
-                                                                       src_mul / (double)m.cells(), transfer, mode_div(m));
+  green64_adjoint_kernel<<<grid_for(m.half_cells(), 256), 256, 0, s>>>(
+      spec3, spec1, m, tables64(tables, m, has_masks), src_mul / (double)m.cells(), transfer, mode_div(m));
   // interlaced: split the source cotangent between the two deposits
   if (il) interlace64_kernel<<<grid_for(m.half_cells(), 256), 256, 0, s>>>(spec1, spec1 + m.half_cells(), m, 1,
                                                                          mode_div(m));

@@ -676,6 +676,7 @@ int lpt_modes_adjoint64(const double2* F1, const double2* FS, const double* amp,
 // bound by the shuffles of the segmented sums.
 constexpr int kPkThreads = 256;
 constexpr int kPkWarps = kPkThreads / 32;
+constexpr int kPkSmem = 220 * 1024;  // dynamic shared memory of these kernels at most
 
 __device__ __forceinline__ int shell_of(long long n2, int num_shells) {
   long long r;
@@ -700,14 +701,16 @@ __device__ __forceinline__ double window_pow(double w, int p) {
   return 1.0 / x;
 }
 
-// Table of W_z^-2p (times the rFFT multiplicity with mult) for kz < nzh.
+// W_z^-2p of column k (times the rFFT multiplicity with mult); read from a table
+// in shared memory, filled by z_window, where that fits (kPkSmem).
+__device__ __forceinline__ double z_factor(double w, int k, int nz, int mas_power, bool mult) {
+  const double f = window_pow(w, mas_power);
+  return mult && !(k == 0 || (nz % 2 == 0 && k == nz / 2)) ? 2.0 * f : f;
+}
+
 template <class T>
 __device__ __forceinline__ void z_window(double* zf, const T* __restrict__ sz, int nz, int mas_power, bool mult) {
-  const int nzh = nz / 2 + 1;
-  for (int k = threadIdx.x; k < nzh; k += blockDim.x) {
-    const double f = window_pow((double)sz[k], mas_power);
-    zf[k] = mult && !(k == 0 || ((nz % 2 == 0) && k == nzh - 1)) ? 2.0 * f : f;
-  }
+  for (int k = threadIdx.x; k < nz / 2 + 1; k += blockDim.x) zf[k] = z_factor((double)sz[k], k, nz, mas_power, mult);
 }
 
 // Adds v to hist[shell] for the warp's 32 lanes; equal shells are neighbours.
@@ -733,18 +736,19 @@ __device__ __forceinline__ void add_runs(double v, int shell, double* hist, bool
 template <class T, bool CROSS>
 __global__ void __launch_bounds__(kPkThreads)
     pk_shells_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                     int mas_power, int num_shells, int copies, double* __restrict__ sums,
+                     int mas_power, int num_shells, int copies, int tabulated, double* __restrict__ sums,
                      const typename Real<T>::T2* __restrict__ spec_b, double* __restrict__ sums_b,
                      double* __restrict__ sums_x) {
   using T2 = typename Real<T>::T2;
   constexpr int NS = CROSS ? 3 : 1;
   constexpr int UN = 4;  // chunks of 32 modes loaded together
-  extern __shared__ double sh[];  // copies x NS x num_shells, then the z table
+  extern __shared__ double sh[];  // copies x NS x num_shells, then the z table if tabulated
   double* zf = sh + (size_t)copies * NS * num_shells;
   for (int t = threadIdx.x; t < copies * NS * num_shells; t += kPkThreads) sh[t] = 0.0;
   const T* sx = sinc_tab;
   const T* sy = sx + m.nx;
-  z_window(zf, sy + m.ny, m.nz, mas_power, true);
+  const T* sz = sy + m.ny;
+  if (tabulated) z_window(zf, sz, m.nz, mas_power, true);
   __syncthreads();
   const int nzh = m.nz / 2 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -770,7 +774,8 @@ __global__ void __launch_bounds__(kPkThreads)
         const int k = k0 + 32 * q;
         if (k - lane >= nzh) break;
         const int shell = shell_of(r2 + (long long)k * k, num_shells);
-        const double f = k < nzh ? rf * zf[k] : 0.0;
+        double f = 0.0;
+        if (k < nzh) f = rf * (tabulated ? zf[k] : z_factor((double)sz[k], k, m.nz, mas_power, true));
         const double ar = va[q].x, ai = va[q].y;
         add_runs((ar * ar + ai * ai) * f, shell, hist, own);
         if (CROSS) {
@@ -794,20 +799,24 @@ template <class T, bool CROSS>
 static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
                             int num_shells, double* sums, const typename Real<T>::T2* spec_b, double* sums_b,
                             double* sums_x, cudaStream_t s) {
-  // a copy of the sums per warp where that leaves room for two blocks on an SM
-  const int64_t table = 8 * (m.nz / 2 + 1), one = (int64_t)8 * (CROSS ? 3 : 1) * num_shells;
+  // a copy of the sums per warp where that leaves room for two blocks on an SM;
+  // no z table where it does not fit beside one copy
+  const int64_t one = (int64_t)8 * (CROSS ? 3 : 1) * num_shells;
+  if (one > 200 * 1024) return kUnsupported;
+  int64_t table = 8 * ((int64_t)m.nz / 2 + 1);
+  const int tabulated = table + one <= kPkSmem;
+  if (!tabulated) table = 0;
   int copies = kPkWarps;
   while (copies > 1 && table + copies * one > 100 * 1024) copies /= 2;
   const int64_t smem = table + copies * one;
-  if (one > 200 * 1024 || smem > 220 * 1024) return kUnsupported;
   auto k = pk_shells_kernel<T, CROSS>;
   PMB_CUDA_CHECK(smem_optin((const void*)k, (int)smem));
-  int64_t per_sm = (220 * 1024) / (smem + 1024);
+  int64_t per_sm = kPkSmem / (smem + 1024);
   per_sm = per_sm > 8 ? 8 : per_sm < 1 ? 1 : per_sm;
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * per_sm) grid = 148 * per_sm;
   k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, (size_t)smem, s>>>(spec, m, sinc_tab, mas_power, num_shells,
-                                                                      copies, sums, spec_b, sums_b, sums_x);
+                                                                      copies, tabulated, sums, spec_b, sums_b, sums_x);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
@@ -835,14 +844,15 @@ int pk_shells64(const double2* spec, Mesh3 m, const double* sinc_tab, int mas_po
 template <class T>
 __global__ void __launch_bounds__(kPkThreads)
     pk_shells_adjoint_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                             int mas_power, int num_shells, const double* __restrict__ wshell, double post,
-                             typename Real<T>::T2* __restrict__ out) {
+                             int mas_power, int num_shells, int tabulated, const double* __restrict__ wshell,
+                             double post, typename Real<T>::T2* __restrict__ out) {
   using T2 = typename Real<T>::T2;
   constexpr int UN = 4;
   extern __shared__ double zf[];
   const T* sx = sinc_tab;
   const T* sy = sx + m.nx;
-  z_window(zf, sy + m.ny, m.nz, mas_power, false);
+  const T* sz = sy + m.ny;
+  if (tabulated) z_window(zf, sz, m.nz, mas_power, false);
   __syncthreads();
   const int nzh = m.nz / 2 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -862,7 +872,8 @@ __global__ void __launch_bounds__(kPkThreads)
       for (int q = 0; q < UN; ++q) {
         const int k = k0 + 32 * q;
         if (k < nzh) {
-          const double f = rf * zf[k] * wshell[shell_of(r2 + (long long)k * k, num_shells)];
+          const double z = tabulated ? zf[k] : z_factor((double)sz[k], k, m.nz, mas_power, false);
+          const double f = rf * z * wshell[shell_of(r2 + (long long)k * k, num_shells)];
           o[k] = Real<T>::make2((T)(v[q].x * f), (T)(v[q].y * f));
         }
       }
@@ -876,8 +887,13 @@ static int launch_pk_adjoint(const typename Real<T>::T2* spec, Mesh3 m, const T*
                              cudaStream_t s) {
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * 8) grid = 148 * 8;
-  pk_shells_adjoint_kernel<T><<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, 8 * (m.nz / 2 + 1), s>>>(
-      spec, m, sinc_tab, mas_power, num_shells, wshell, post, out);
+  const int64_t table = 8 * ((int64_t)m.nz / 2 + 1);
+  const int tabulated = table <= kPkSmem;
+  const size_t smem = tabulated ? (size_t)table : 0;
+  auto k = pk_shells_adjoint_kernel<T>;
+  PMB_CUDA_CHECK(smem_optin((const void*)k, (int)smem));
+  k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, smem, s>>>(spec, m, sinc_tab, mas_power, num_shells, tabulated,
+                                                              wshell, post, out);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }

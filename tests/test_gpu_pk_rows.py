@@ -52,7 +52,39 @@ def test_shell_sums_and_cross(shape, mas):
         assert np.all(np.abs(got[i] - ref) <= bars[i])
 
 
-@pytest.mark.parametrize("shape", [(4, 4, 4), (5, 3, 7), (9, 8, 65), (3, 2, 1), (2, 70, 130)])
+# rows whose window table along z is above 48 KB, and above all of shared memory
+LONG = [(2, 3, 12288), (4, 1, 40001), (2, 1, 57344)]
+
+
+@pytest.mark.parametrize("shape,cross,ns", [(LONG[0], True, 40), (LONG[1], False, 40), (LONG[2], False, 40),
+                                            (LONG[2], True, 40), ((4, 2, 8192), True, 8533), ((2, 2, 40001), False, 25600)])
+@pytest.mark.parametrize("mas", [0, 2])
+def test_shell_sums_of_long_rows(shape, cross, ns, mas):
+    """Rows up to and beyond the length whose table fits beside the sums: FP64 products and sums of at most
+    2^18 terms (bar 2^-34 of the sum of their magnitudes)."""
+    from pmpp_b200 import power_spectrum as ps
+    from pmpp_b200._lib import call
+    from pmpp_b200.runtime import stream_handle
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a, b = (torch.randn(shape[:2] + (shape[2] // 2 + 1, 2), generator=g, device="cuda") for _ in range(2))
+    tab = ps._sinc_tables(_conf(shape), a.device)
+    out = torch.empty((3, ns), dtype=torch.float64, device="cuda")
+    ptr = lambda t: t.data_ptr() if cross else None
+    call("pmb_pk_shells", a.data_ptr(), *shape, tab.data_ptr(), mas, ns, out[0].data_ptr(), ptr(b), ptr(out[1]),
+         ptr(out[2]), stream_handle(a.device))
+    t = np.split(tab.cpu().numpy().astype(np.float64), np.cumsum(shape[:2]))
+    shell, (_, _, mz) = _shells(shape, ns)
+    w = (t[0][:, None, None] * t[1][:, None] * t[2])**(-2.0 * mas)
+    w = w * np.where((mz == 0) | ((shape[2] % 2 == 0) & (mz == shape[2] // 2)), 1.0, 2.0)
+    ca, cb = (x.cpu().numpy().astype(np.float64) for x in (a, b))
+    pairs = [(ca, ca)] + ([(cb, cb), (ca, cb)] if cross else [])
+    for i, (x, y) in enumerate(pairs):
+        v = (x[..., 0] * y[..., 0] + x[..., 1] * y[..., 1]) * w
+        ref, mag = (np.bincount(shell.ravel(), z.ravel(), minlength=ns) for z in (v, np.abs(v)))
+        assert np.all(np.abs(out[i].cpu().numpy() - ref) <= 2.0**-34 * mag)
+
+
+@pytest.mark.parametrize("shape", [(4, 4, 4), (5, 3, 7), (9, 8, 65), (3, 2, 1), (2, 70, 130)] + LONG)
 def test_adjoint_rows(shape):
     """out = spec * 2 post W^-2p w[shell], in float64 and rounded once (bar 2^-22)."""
     from pmpp_b200 import power_spectrum as ps

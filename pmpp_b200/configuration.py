@@ -256,14 +256,24 @@ class Configuration:
 
     def lattice_tables(self, device=None):
         """Device tables of the particle lattice's axes: anchors (int16) and
-        offsets of x, y and z one after another (Particles.lattice_axes)."""
+        offsets of x, y and z one after another (Particles.lattice_axes).
+
+        Made by kernels of the caller's stream, so they are kept only once these
+        have run (any stream may read them afterwards); under graph capture, where
+        that cannot be waited for, each call makes its own."""
         device = self.device if device is None else torch.device(device)
         key = ("lattice", str(device))
-        if key not in self._tables:
+        got = self._tables.get(key)
+        if got is None:
             from .particles import Particles
             pm, dp = Particles.lattice_axes(self, device)
-            self._tables[key] = (torch.cat(pm), torch.cat(dp))
-        return self._tables[key]
+            got = torch.cat(pm), torch.cat(dp)
+            if device.type == "cuda":
+                if torch.cuda.is_current_stream_capturing():
+                    return got
+                torch.cuda.current_stream(device).synchronize()
+            self._tables[key] = got
+        return got
 
     def spectral_tables(self, which="mesh", device=None, green_kernel=0, gradient_kernel=0):
         """Device table [kx ky kz cx cy cz (mx my mz)] for pmb_green_gradient.

@@ -36,3 +36,37 @@ def test_lattice_particles_bitwise(shape, order, mesh):
     assert torch.equal(res.index, index)
     for m in range(3 * order):  # the fields of the orders in use
         assert torch.equal(res.fields[m], fields[m]), m
+
+
+def _conf():
+    import pmpp_b200 as pb
+    return pb.Configuration(4.0, (7, 6, 5), 2, a_start=0.1, device="cuda")
+
+
+def _same(tables, conf):
+    from pmpp_b200 import Particles
+    pm, dp = Particles.lattice_axes(conf, torch.device("cuda"))
+    return torch.equal(tables[0], torch.cat(pm)) and torch.equal(tables[1], torch.cat(dp))
+
+
+def test_axis_tables_are_complete_when_kept():
+    """Another stream may read the kept tables at once, so the work that makes them has ended."""
+    conf = _conf()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+        tables = conf.lattice_tables("cuda")
+        assert side.query()
+    assert conf.lattice_tables("cuda")[0] is tables[0]
+    assert _same(tables, conf)
+
+
+def test_axis_tables_of_a_capture_are_its_own():
+    conf = _conf()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = conf.lattice_tables("cuda")
+    assert held[0] is not conf.lattice_tables("cuda")[0]  # nothing that only a replay fills is kept
+    assert _same(conf.lattice_tables("cuda"), conf)
+    graph.replay()
+    assert _same(held, conf)

@@ -733,22 +733,22 @@ __device__ __forceinline__ void add_runs(double v, int shell, double* hist, bool
   __syncwarp();
 }
 
-template <class T, bool CROSS>
+template <class T, bool CROSS, bool TAB>
 __global__ void __launch_bounds__(kPkThreads)
     pk_shells_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                     int mas_power, int num_shells, int copies, int tabulated, double* __restrict__ sums,
+                     int mas_power, int num_shells, int copies, double* __restrict__ sums,
                      const typename Real<T>::T2* __restrict__ spec_b, double* __restrict__ sums_b,
                      double* __restrict__ sums_x) {
   using T2 = typename Real<T>::T2;
   constexpr int NS = CROSS ? 3 : 1;
   constexpr int UN = 4;  // chunks of 32 modes loaded together
-  extern __shared__ double sh[];  // copies x NS x num_shells, then the z table if tabulated
+  extern __shared__ double sh[];  // copies x NS x num_shells, then the z table (TAB)
   double* zf = sh + (size_t)copies * NS * num_shells;
   for (int t = threadIdx.x; t < copies * NS * num_shells; t += kPkThreads) sh[t] = 0.0;
   const T* sx = sinc_tab;
   const T* sy = sx + m.nx;
   const T* sz = sy + m.ny;
-  if (tabulated) z_window(zf, sz, m.nz, mas_power, true);
+  if (TAB) z_window(zf, sz, m.nz, mas_power, true);
   __syncthreads();
   const int nzh = m.nz / 2 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kPkThreads)
         if (k - lane >= nzh) break;
         const int shell = shell_of(r2 + (long long)k * k, num_shells);
         double f = 0.0;
-        if (k < nzh) f = rf * (tabulated ? zf[k] : z_factor((double)sz[k], k, m.nz, mas_power, true));
+        if (k < nzh) f = rf * (TAB ? zf[k] : z_factor((double)sz[k], k, m.nz, mas_power, true));
         const double ar = va[q].x, ai = va[q].y;
         add_runs((ar * ar + ai * ai) * f, shell, hist, own);
         if (CROSS) {
@@ -804,19 +804,19 @@ static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* 
   const int64_t one = (int64_t)8 * (CROSS ? 3 : 1) * num_shells;
   if (one > 200 * 1024) return kUnsupported;
   int64_t table = 8 * ((int64_t)m.nz / 2 + 1);
-  const int tabulated = table + one <= kPkSmem;
+  const bool tabulated = table + one <= kPkSmem;
   if (!tabulated) table = 0;
   int copies = kPkWarps;
   while (copies > 1 && table + copies * one > 100 * 1024) copies /= 2;
   const int64_t smem = table + copies * one;
-  auto k = pk_shells_kernel<T, CROSS>;
+  auto k = tabulated ? pk_shells_kernel<T, CROSS, true> : pk_shells_kernel<T, CROSS, false>;
   PMB_CUDA_CHECK(smem_optin((const void*)k, (int)smem));
   int64_t per_sm = kPkSmem / (smem + 1024);
   per_sm = per_sm > 8 ? 8 : per_sm < 1 ? 1 : per_sm;
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * per_sm) grid = 148 * per_sm;
   k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, (size_t)smem, s>>>(spec, m, sinc_tab, mas_power, num_shells,
-                                                                      copies, tabulated, sums, spec_b, sums_b, sums_x);
+                                                                      copies, sums, spec_b, sums_b, sums_x);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
@@ -841,18 +841,18 @@ int pk_shells64(const double2* spec, Mesh3 m, const double* sinc_tab, int mas_po
 // of the rFFT transpose).  Rows and tables as in pk_shells_kernel: 506 -> 243 us
 // for a 512^3 mesh, 164 us for the bytes.
 // T = double: the float64 build's form.
-template <class T>
+template <class T, bool TAB>
 __global__ void __launch_bounds__(kPkThreads)
     pk_shells_adjoint_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, const T* __restrict__ sinc_tab,
-                             int mas_power, int num_shells, int tabulated, const double* __restrict__ wshell,
-                             double post, typename Real<T>::T2* __restrict__ out) {
+                             int mas_power, int num_shells, const double* __restrict__ wshell, double post,
+                             typename Real<T>::T2* __restrict__ out) {
   using T2 = typename Real<T>::T2;
   constexpr int UN = 4;
   extern __shared__ double zf[];
   const T* sx = sinc_tab;
   const T* sy = sx + m.nx;
   const T* sz = sy + m.ny;
-  if (tabulated) z_window(zf, sz, m.nz, mas_power, false);
+  if (TAB) z_window(zf, sz, m.nz, mas_power, false);
   __syncthreads();
   const int nzh = m.nz / 2 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(kPkThreads)
       for (int q = 0; q < UN; ++q) {
         const int k = k0 + 32 * q;
         if (k < nzh) {
-          const double z = tabulated ? zf[k] : z_factor((double)sz[k], k, m.nz, mas_power, false);
+          const double z = TAB ? zf[k] : z_factor((double)sz[k], k, m.nz, mas_power, false);
           const double f = rf * z * wshell[shell_of(r2 + (long long)k * k, num_shells)];
           o[k] = Real<T>::make2((T)(v[q].x * f), (T)(v[q].y * f));
         }
@@ -888,12 +888,12 @@ static int launch_pk_adjoint(const typename Real<T>::T2* spec, Mesh3 m, const T*
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * 8) grid = 148 * 8;
   const int64_t table = 8 * ((int64_t)m.nz / 2 + 1);
-  const int tabulated = table <= kPkSmem;
+  const bool tabulated = table <= kPkSmem;
   const size_t smem = tabulated ? (size_t)table : 0;
-  auto k = pk_shells_adjoint_kernel<T>;
+  auto k = tabulated ? pk_shells_adjoint_kernel<T, true> : pk_shells_adjoint_kernel<T, false>;
   PMB_CUDA_CHECK(smem_optin((const void*)k, (int)smem));
-  k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, smem, s>>>(spec, m, sinc_tab, mas_power, num_shells, tabulated,
-                                                              wshell, post, out);
+  k<<<(unsigned)(grid > 0 ? grid : 1), kPkThreads, smem, s>>>(spec, m, sinc_tab, mas_power, num_shells, wshell,
+                                                              post, out);
   PMB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }

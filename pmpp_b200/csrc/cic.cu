@@ -795,11 +795,49 @@ constexpr int tile_y(int C, int nzp) {
   return 4 * rows <= kTileBytes ? 4 : 2 * rows <= kTileBytes ? 2 : 1;
 }
 
-template <int C, int NZP, bool EXACT, bool SIGNED>
+// Crowded meshes take one output row per block (ROW) instead of a tile, although
+// a record is then read four times instead of 25 / 16 or 9 / 4:
+//  * where the tiles are too few to share the work out evenly;
+//  * where a tile would hold too many particles for the two-plane sums and a row
+//    does not (at the mean density and four standard deviations);
+//  * where neither fits, with three or four channels and tiles of more than four
+//    rows.
+// Deposits in us, tile / row (constant value | one, two, three, four channels of
+// values): 16^3 cells with 32 particles each 131 / 20 | 145 / 29, 227 / 37, 304 / 45,
+// 383 / 52; 64^3 with 4: 50 / 20 | 61 / 32, 95 / 39, 126 / 48, 160 / 60; 96^3 with 32,
+// where neither fits: 867 / 963 | 787 / 1002, 1389 / 1668, 2486 / 2296, 3339 / 3067;
+// 128^3 with 4, where the tile of a constant fits: 89 / 98 | 300 / 132, 550 / 188, 702 /
+// 249, 845 / 350; 32 x 32 x 256 with 8, whose tiles of three and four channels
+// are enough: 224 / 71 | 262 / 77, 226 / 180, 192 / 249, 250 / 320.
+constexpr int kRowMaxNz = 512;  // longer rows have tiles of at most four
+
+static bool planes_fit(double particles, int E, bool sgn) {
+  const double k = particles + 4.0 * sqrt(particles);
+  int L = 0;  // k < 2^L, as in the kernel
+  while (ldexp(1.0, L) <= k) ++L;
+  const int lo = E - 24 > L + E - (sgn ? 31 : 32) ? E - 24 : L + E - (sgn ? 31 : 32);
+  return lo <= (32 - L < (sgn ? 23 : 24) ? 32 - L : (sgn ? 23 : 24));
+}
+
+static bool row_per_block(Mesh3 m, int C, bool sgn, int64_t n, int E) {
+  if (m.nz > kRowMaxNz) return false;
+  static const int strides[6] = {64, 128, 192, 256, 384, 512};
+  int q = 0;
+  while (strides[q] < m.nz) ++q;
+  const int tx = tile_x(C, strides[q]), ty = tile_y(C, strides[q]);
+  const double tiles = (double)((m.nx + tx - 1) / tx) * (double)((m.ny + ty - 1) / ty);
+  if (tiles < (tx * ty > 4 ? 3 * 148 : 148) && (double)n > 5.0 * tiles * tiles) return true;
+  if (n <= m.cells()) return false;
+  const double line = (double)n / (double)m.cells() * (double)m.nz;  // particles in a row of the mesh
+  if (planes_fit(2 * (ty + 1) * line, E, sgn)) return false;
+  return planes_fit(4 * line, E, sgn) || (C >= 3 && tx * ty > 4);
+}
+
+template <int C, int NZP, bool EXACT, bool SIGNED, bool ROW = false>
 static int launch_rows(const Rec* rec, const uint32_t* perm, const uint32_t* offs, Mesh3 m, const float* val,
                        int val_sorted, float val_const, const double* scale_dev, double scale_const, int E, int mode,
                        float src_mul, float* out, uint32_t* status, cudaStream_t s) {
-  constexpr int RX = tile_x(C, NZP), RY = tile_y(C, NZP);
+  constexpr int RX = ROW ? 1 : tile_x(C, NZP), RY = ROW ? 1 : tile_y(C, NZP);
   auto k = scatter_rows_kernel<C, RX, RY, NZP, EXACT, SIGNED>;
   constexpr int smem = 8 * RX * RY * C * NZP;
   PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
@@ -811,11 +849,18 @@ static int launch_rows(const Rec* rec, const uint32_t* perm, const uint32_t* off
   return kOk;
 }
 
-// A kernel for the row length itself (usual lengths, one and three channels),
-// else the one of the shortest row stride that holds nz cells.
+// A kernel for the row length itself (usual lengths; one channel of a constant
+// value and three channels, the deposits of a force and its adjoint), else the
+// one of the shortest row stride that holds nz cells.  row: one row per block.
 template <int C, bool SIGNED, class... Args>
-static int launch_rows_nz(Args... a) {
+static int launch_rows_nz(bool row, Args... a) {
   const int nz = std::get<3>(std::tie(a...)).nz;
+  if (row) {
+    if (nz <= 64) return launch_rows<C, 64, false, SIGNED, true>(a...);
+    if (nz <= 128) return launch_rows<C, 128, false, SIGNED, true>(a...);
+    if (nz <= 256) return launch_rows<C, 256, false, SIGNED, true>(a...);
+    return launch_rows<C, kRowMaxNz, false, SIGNED, true>(a...);
+  }
   if constexpr (C == 3 || (C == 1 && !SIGNED)) {
     switch (nz) {
       case 128: return launch_rows<C, 128, true, SIGNED>(a...);
@@ -852,8 +897,8 @@ int scatter_sorted(const Rec* rec, const uint32_t* perm, const uint32_t* offs, M
   const double scale = fixed_point_scale(fixed_point_pow2(n), fabsf(val_const));
   const bool uns = val == nullptr && val_const >= 0.f;
 #define PMB_SCATTER(CC, SG)                                                                                       \
-  launch_rows_nz<CC, SG>(rec, perm, offs, m, val, val_sorted, val_const, scale_dev, scale, E, mode, src_mul, out, \
-                         status, s)
+  launch_rows_nz<CC, SG>(row_per_block(m, CC, SG, n, E), rec, perm, offs, m, val, val_sorted, val_const, scale_dev, \
+                         scale, E, mode, src_mul, out, status, s)
   switch (C) {
     case 1: return uns ? PMB_SCATTER(1, false) : PMB_SCATTER(1, true);
     case 2: return PMB_SCATTER(2, true);

@@ -1,5 +1,6 @@
 """Deposit at the edges of its tiles and row strides: row lengths on and beside
-the instantiated strides, meshes with remainders of the tile's rows, the
+the instantiated strides, meshes with remainders of the tile's rows, meshes of few
+rows (one row per block once they are crowded) and of many, the
 smallest meshes (a particle reaching one cell twice), values of every scale, an
 output that is not 16-byte aligned, and one cell holding so many particles that
 the 64-bit sums are taken.  The arithmetic is restated exactly
@@ -16,6 +17,9 @@ pytestmark = pytest.mark.gpu
 MESHES = [(1, 1, 1), (2, 1, 3), (1, 2, 64), (3, 5, 65), (5, 2, 127), (9, 6, 128), (4, 7, 129), (6, 5, 192),
           (5, 5, 250), (7, 9, 256), (3, 6, 384), (5, 3, 512), (3, 3, 600), (2, 5, 768), (5, 2, 1024), (2, 2, 1500),
           (1, 3, 4096)]
+# rows enough that 40000 particles are not a crowd
+WIDE = [(37, 43, 3), (40, 37, 64), (37, 42, 65), (38, 40, 128), (41, 39, 192), (37, 41, 250), (39, 38, 256),
+        (38, 39, 384), (41, 50, 512)]
 
 
 def _particles(mesh, n, seed, crowd):
@@ -35,7 +39,7 @@ def _check(got, ref):
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
 
 
-@pytest.mark.parametrize("mesh", MESHES)
+@pytest.mark.parametrize("mesh", MESHES + WIDE)
 @pytest.mark.parametrize("n,crowd", [(300, False), (40000, False), (40000, True)])
 def test_density_bit_exact(mesh, n, crowd):
     from pmpp_b200.cic import SortedParticles
@@ -46,7 +50,7 @@ def test_density_bit_exact(mesh, n, crowd):
         _check(sp.scatter(val_const=val)[0].cpu().numpy(), ref)
 
 
-@pytest.mark.parametrize("mesh", MESHES)
+@pytest.mark.parametrize("mesh", MESHES + WIDE)
 @pytest.mark.parametrize("channels,scale", [(1, 1.0), (2, 1e-28), (3, 1.0), (3, 1e27), (4, 1e-5)])
 def test_values_bit_exact_and_misaligned_output(mesh, channels, scale):
     from pmpp_b200.cic import SortedParticles

@@ -55,3 +55,30 @@ def test_unsynchronised_calls_bitwise(shape, mesh):
         assert torch.equal(other[i], ref[i % 3][0])
     for k in range(3):
         assert torch.equal(held[k], ref[k][0])
+
+
+@pytest.mark.parametrize("mesh,n", [((16, 16, 16), 1 << 17), ((16, 16, 16), 1 << 18), ((32, 8, 64), 300000),
+                                    ((8, 8, 8), 200000)])
+def test_crowded_small_mesh_bitwise(mesh, n):
+    """Deposits of many particles on few rows, early and plain, right after their sort and before a gather
+    of what they wrote: no synchronisation in between against one after each."""
+    import pmpp_b200 as pb
+    from pmpp_b200.cic import SortedParticles
+    conf = pb.Configuration(2.0, mesh, 1, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(2)
+    side = torch.tensor(mesh, device="cuda")
+    sets = [((torch.rand((n, 3), generator=g, device="cuda") * side).to(torch.int16),
+             torch.randn((n, 3), generator=g, device="cuda")) for _ in range(2)]
+
+    def run(k, sync):
+        wait = torch.cuda.synchronize if sync else lambda: None
+        sp = SortedParticles(*sets[k], conf)
+        wait()
+        rho = sp.scatter(val_const=0.25)
+        wait()
+        return rho, sp.gather(rho.expand(3, *mesh).contiguous())
+
+    ref = [run(k, True) for k in range(2)]
+    got = [run(i % 2, False) for i in range(8)]
+    for i, (rho, v) in enumerate(got):
+        assert torch.equal(rho, ref[i % 2][0]) and torch.equal(v, ref[i % 2][1])

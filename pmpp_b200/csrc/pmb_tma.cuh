@@ -54,7 +54,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 // blocks have all called let_next_start or ended); from wait_for_previous on,
 // all that the stream did before is complete and visible.  Every thread calls
 // wait_for_previous before it touches anything but its own shared memory and
-// constants of the module.
+// constants of the module.  Such a kernel is resident while its inputs are still
+// being written, so it reads them by ordinary loads: no __ldg and no const
+// __restrict__ parameters, which would let the compiler take the non-coherent path
+// or move a load above the wait.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -57,8 +57,14 @@ __device__ __forceinline__ bool flagged(const uint32_t* status) { return status 
 // bound: 342 us for 256^3 and 2.71 ms for 512^3 clustered particles, 174 us
 // and 1.26 ms by runs; the bytes take 0.07 and 0.6 ms.)  kSortPer particles a
 // thread, a block apart, so that their loads overlap.
+//
+// On meshes of few rows (FEW) a warp of particles in no order, more than eight
+// runs of rows that repeat, groups equal rows all the same: the atomics on those
+// rows are the bound there (sorts of 2^22 shuffled particles by runs / grouped, us:
+// 4^3 cells 730 / 243, 8^3 1146 / 770, 16^3 1056 / 980, 24^3 631 / 617, 32^3 434 / 432).
 constexpr int kSortThreads = 256;
 constexpr int kSortPer = 4;
+constexpr int64_t kFewRows = 1024;
 
 __device__ __forceinline__ uint32_t row_bin(const int16_t* __restrict__ pmid, float d0, float d1, float d2, int64_t i,
                                             Mesh3 m, float cell, const BinShift& sh,
@@ -68,6 +74,7 @@ __device__ __forceinline__ uint32_t row_bin(const int16_t* __restrict__ pmid, fl
   return (uint32_t)b.cx * (uint32_t)m.ny + (uint32_t)b.cy;
 }
 
+template <bool FEW>
 __global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const int16_t* pmid,
                                                                  float* __restrict__ disp,
                                                                  const float* vel, float drift, int64_t n,
@@ -103,7 +110,7 @@ __global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const int16_t* 
     }
   }
   uint32_t head_base[kSortPer];
-  int head[kSortPer];
+  int head[kSortPer], after_head[kSortPer];
   bool bad = false;
 #pragma unroll
   for (int k = 0; k < kSortPer; ++k) {
@@ -114,19 +121,24 @@ __global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const int16_t* 
     const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, row, 1);
     const unsigned heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || row != prev);
     head[k] = 31 - __clz(heads & upto);
-    head_base[k] = 0;
-    if (head[k] == lane && i < n) {
-      const unsigned after = heads & ~upto;
-      const int len = (after ? __ffs(after) - 1 : 32) - lane;
-      head_base[k] = atomicAdd(&counts[row], (uint32_t)len);
+    after_head[k] = lane - head[k];
+    const unsigned after = heads & ~upto;
+    int len = (after ? __ffs(after) - 1 : 32) - lane;
+    if (FEW && __popc(heads) > 8) {
+      const unsigned equal = __match_any_sync(0xFFFFFFFFu, row);
+      head[k] = __ffs(equal) - 1;
+      after_head[k] = __popc(equal & upto) - 1;
+      len = __popc(equal);
     }
+    head_base[k] = 0;
+    if (head[k] == lane && i < n) head_base[k] = atomicAdd(&counts[row], (uint32_t)len);
   }
   if (bad) raise_flag(flag, kFlagNonFiniteDisp);
 #pragma unroll
   for (int k = 0; k < kSortPer; ++k) {
     const int64_t i = base + k * kSortThreads;
     const uint32_t b = __shfl_sync(0xFFFFFFFFu, head_base[k], head[k]);
-    if (i < n) rank_of[i] = b + (uint32_t)(lane - head[k]);
+    if (i < n) rank_of[i] = b + (uint32_t)after_head[k];
   }
 }
 
@@ -365,9 +377,11 @@ int bin_particles(const int16_t* pmid, float* disp, const float* vel, float drif
   PMB_CUDA_CHECK(cudaMemsetAsync(counts, 0, align_up(4 * len, 256) + 4, s));
   const bool early = small_mesh(m.nx, m.ny, m.nz);
   const auto grid_of = [n](int per) { return (int)((n + kSortThreads * per - 1) / (kSortThreads * per)); };
-  if (n > 0)
-    PMB_CUDA_CHECK(launch_dependent(early, bin_count_kernel, grid_of(kSortPer), kSortThreads, 0, s, pmid, disp, vel,
-                                    drift, n, m, cell, sh, valid, counts, row_of, rank_of, flag));
+  if (n > 0) {
+    auto k = rows <= kFewRows ? bin_count_kernel<true> : bin_count_kernel<false>;
+    PMB_CUDA_CHECK(launch_dependent(early, k, grid_of(kSortPer), kSortThreads, 0, s, pmid, disp, vel, drift, n, m, cell,
+                                    sh, valid, counts, row_of, rank_of, flag));
+  }
   int st = exclusive_scan(counts, offs, len, tile_sums, flag, status, early, s);
   if (st != kOk) return st;
   if (n > 0)

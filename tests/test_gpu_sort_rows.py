@@ -1,6 +1,6 @@
 """Row sort at the edges of its launches: particle counts around the block's
-1024, row counts around the one-block scan (16384 rows), empty rows, long runs
-of one row, a drift; records, permutation and row offsets against the oracle's
+1024, row counts around the grouping of unordered particles (1024 rows) and the
+one-block scan (16384 rows), empty rows, long runs of one row, a drift; records, permutation and row offsets against the oracle's
 binning (whole numbers, so exact)."""
 import numpy as np
 import pytest
@@ -11,7 +11,8 @@ from oracle import pm as opm
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("mesh", [(8, 8, 8), (128, 128, 4), (129, 128, 4), (1, 1, 8), (300, 70, 2)])
+@pytest.mark.parametrize("mesh", [(8, 8, 8), (16, 16, 3), (257, 1, 4), (32, 32, 2), (25, 41, 3), (128, 128, 4), (129, 128, 4), (1, 1, 8),
+                                  (2, 3, 5), (300, 70, 2)])
 @pytest.mark.parametrize("n", [1, 1023, 1025, 5000])
 @pytest.mark.parametrize("drift", [None, 0.5])
 def test_rows_records_and_offsets(mesh, n, drift):

@@ -255,8 +255,9 @@ int pmb_project_density(const float* mesh, int nx, int ny, int nz, int axis, int
 
 /* ---------------- hand-written PM FFT passes -------------------------------
  * For meshes whose sides are powers of two (nx, ny in 64..1024, nz in
- * 128..1024) or three times one (96, 192, 384, 768) the fused force and its adjoint run their spectral stages as a
- * chain of hand-written passes over a y-blocked half-spectrum layout:
+ * 128..1024) or three times one (96, 192, 384, 768) the fused force and its
+ * adjoint run their spectral stages as a chain of hand-written passes over a
+ * y-blocked half-spectrum layout:
  * channel-major, then rows ((y/32)*nx + x)*32 + y%32 of P = nz/2 + 8 complex
  * values (columns above nz/2 zero).  pmb_pmfft_channel_elems gives the complex
  * values per channel (-1 when the mesh is not supported).  Same numpy
@@ -270,7 +271,10 @@ int pmb_project_density(const float* mesh, int nx, int ny, int nz, int axis, int
  *   of channels ch_off, ch_off+1 combined as (-i c_y) Y + (-i c_z) Z, 4 x
  *   forward, 5 x inverse, 6 x forward + Green multiplier + x inverse into
  *   (i c_x phi, phi) (2 output channels), 7 x forward of channels 0, 1 +
- *   adjoint multiplier + x inverse, 8 the same without the x inverse.  Modes 0, 1, 4, 5 transform nbatch
+ *   adjoint multiplier + x inverse, 8 the same without the x inverse, 9 (ny up
+ *   to 512) modes 1 and 2 in one pass: nbatch = 3 n output channels (y inverse
+ *   of W, i c_y Q, i c_z Q) of each of n forces from channels W at ch_off and Q
+ *   at ch_off + n.  Modes 0, 1, 4, 5 transform nbatch
  *   channels starting at ch_off; tables, transfer, radial and post_scale are
  *   those of pmb_green_gradient (tables may be null for modes 0, 1, 4, 5).
  * pmb_set_pmfft(0) routes pmb_force / pmb_force_vjp through cuFFT and the
@@ -281,7 +285,7 @@ int pmb_project_density(const float* mesh, int nx, int ny, int nz, int axis, int
  *   |ky| <= ny_p/2, kz <= nz_p/2 (and the same in kx), so the forward y
  *   passes (modes 0, 3) run only the live kz columns and store only the live
  *   ky rows, the x passes (6, 7) run only live (ky, kz) columns, the inverse
- *   y passes (1, 2) run only live kz columns and read only live ky rows, and
+ *   y passes (1, 2, 9) run only live kz columns and read only live ky rows, and
  *   the z C2R takes the dead kz columns as zeros (the z R2C is unchanged).
  *   Every pass of a chain must then be run pruned with the same tables (the
  *   skipped parts of the intermediate spectra are never written); the results
@@ -289,7 +293,8 @@ int pmb_project_density(const float* mesh, int nx, int ny, int nz, int axis, int
  *   pruned whenever has_masks is set.
  * pmb_pmfft_timeouts: bounded copy waits in these passes that gave up.
  * pmb_pmfft_set_col_ctas(0, 1 or 2): resident CTAs per SM of the column
- *   passes, 0 = the default (one); a tuning knob, results are identical. */
+ *   passes of length 512 and 1024, 0 = the default of each pass and length; a
+ *   tuning knob without effect at other lengths, results are identical. */
 int pmb_set_pmfft(int enabled);
 int pmb_pmfft_supported(int nx, int ny, int nz);
 int64_t pmb_pmfft_channel_elems(int nx, int ny, int nz);

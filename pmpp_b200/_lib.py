@@ -248,6 +248,10 @@ def pmfft_active(nx, ny, nz):
     return _pmfft["enabled"] and bool(lib().pmb_pmfft_supported(int(nx), int(ny), int(nz)))
 
 
+# longest y of the pass that inverts all three force channels (mode 9)
+PMFFT_JOINT_MAX = 512
+
+
 def pmfft_timeouts():
     v = ctypes.c_uint32()
     check(lib().pmb_pmfft_timeouts(ctypes.byref(v)), "pmb_pmfft_timeouts")

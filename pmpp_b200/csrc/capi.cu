@@ -422,7 +422,9 @@ int pmb_pmfft_col(int nx, int ny, int nz, int mode, int nbatch, int ch_off, cons
                   float post_scale, void* stream) {
   Mesh3 m{nx, ny, nz};
   PMB_REQUIRE(pmfft_supported(m), "pmb_pmfft_col: mesh not supported (sides 2^a from 64 to 1024 or 3 2^a from 96 to 768, nz >= 96)");
-  PMB_REQUIRE(mode >= 0 && mode <= 8, "pmb_pmfft_col: mode must be 0..8");
+  PMB_REQUIRE(mode >= 0 && mode <= 9, "pmb_pmfft_col: mode must be 0..9");
+  PMB_REQUIRE(mode != 9 || (nbatch % 3 == 0 && pmfft_joint_inverse(m)),
+              "pmb_pmfft_col: mode 9 takes three outputs a force and ny up to 512");
   PMB_REQUIRE(nbatch >= 1 && ch_off >= 0, "pmb_pmfft_col: bad batch");
   PMB_REQUIRE(tables != nullptr || mode == 0 || mode == 1 || mode == 4 || mode == 5,
               "pmb_pmfft_col: spectral tables required for the multiplier modes");
@@ -449,7 +451,9 @@ int pmb_pmfft_col2(int nx, int ny, int nz, int mode, int nbatch, int ch_off, con
                    float post_scale, int prune, void* stream) {
   Mesh3 m{nx, ny, nz};
   PMB_REQUIRE(pmfft_supported(m), "pmb_pmfft_col2: mesh not supported (sides 2^a from 64 to 1024 or 3 2^a from 96 to 768, nz >= 96)");
-  PMB_REQUIRE(mode >= 0 && mode <= 8, "pmb_pmfft_col2: mode must be 0..8");
+  PMB_REQUIRE(mode >= 0 && mode <= 9, "pmb_pmfft_col2: mode must be 0..9");
+  PMB_REQUIRE(mode != 9 || (nbatch % 3 == 0 && pmfft_joint_inverse(m)),
+              "pmb_pmfft_col2: mode 9 takes three outputs a force and ny up to 512");
   PMB_REQUIRE(nbatch >= 1 && ch_off >= 0, "pmb_pmfft_col2: bad batch");
   PMB_REQUIRE(tables != nullptr || mode == 0 || mode == 1 || mode == 4 || mode == 5,
               "pmb_pmfft_col2: spectral tables required for the multiplier modes");

@@ -99,6 +99,7 @@ int interleave3(const float* planar, float* acc, int64_t n, cudaStream_t s);
 // pmfft.cu: hand-written FFT passes for power-of-two meshes over the
 // y-blocked half-spectrum layout (see pmfft.cu for the layout and modes).
 bool pmfft_supported(Mesh3 m);
+bool pmfft_joint_inverse(Mesh3 m);  // one inverse y pass for all three force channels
 int pmfft_row_len(Mesh3 m);
 int64_t pmfft_channel_elems(Mesh3 m);
 int pmfft_z(Mesh3 m, int inverse, int batch, const float* in_r, const float2* in_c, float* out_r, float2* out_c,

@@ -1458,6 +1458,8 @@ bool pmfft_supported(Mesh3 m) {
          (pow2_in(m.nz, 128, 1024) || third(m.nz));
 }
 
+bool pmfft_joint_inverse(Mesh3 m) { return m.ny <= kInvAllMax; }
+
 int pmfft_row_len(Mesh3 m) { return m.nz / 2 + 8; }
 
 int64_t pmfft_channel_elems(Mesh3 m) { return (int64_t)m.nx * m.ny * pmfft_row_len(m); }
@@ -1657,7 +1659,7 @@ int pmfft_force(Mesh3 m, const float* src, float* force_meshes, float2* work, Sp
   if (st != kOk) return st;
   if ((st = col_pass(m, kYFwd, 1, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
   if ((st = col_pass(m, kXGreen, 1, 0, fp, aq, t, g, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
-  if (m.ny <= kInvAllMax) {
+  if (pmfft_joint_inverse(m)) {
     if ((st = col_pass(m, kYInvAll, 3, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
   } else {
     if ((st = col_pass(m, kYInv, 1, 0, aq, fp, t, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
@@ -1684,7 +1686,7 @@ int pmfft_force_batched(Mesh3 m, int count, const float* src, float* force_meshe
   if ((st = col_pass(m, kYFwd, count, 0, aq, fp, t0, none, nullptr, 0, 0, 0, 1, 1, pr, s)) != kOk) return st;
   if ((st = col_pass(m, kXGreen, count, 0, fp, aq, t0, g, tab_base, tab_stride, has_masks, 0, 1, count, pr, s)) != kOk)
     return st;
-  if (m.ny <= kInvAllMax) {
+  if (pmfft_joint_inverse(m)) {
     st = col_pass(m, kYInvAll, 3 * count, 0, aq, fp, t0, none, tab_base, tab_stride, has_masks, 0, 1, 1, pr, s);
     if (st != kOk) return st;
   } else {

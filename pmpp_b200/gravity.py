@@ -18,7 +18,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from ._lib import call, lib, pmfft_active
+from ._lib import PMFFT_JOINT_MAX, call, lib, pmfft_active
 from .runtime import StageTimer, ptr, require_cuda, stream_handle, workspace
 
 
@@ -369,10 +369,14 @@ def _force_staged(pmid, disp, conf, omega_m, tables, gk, transfer, radial, rl, F
         call("pmb_pmfft_col2", nx, ny, nz, 6, 1, 0, fp, aq, tp, masks, ptr(transfer), ptr(radial), rl,
              float(1.0 / conf.mesh_size), masks, s)
         t = timer.mark("fft_x_green", t)
-        call("pmb_pmfft_col2", nx, ny, nz, 1, 1, 0, aq, fp, tp, masks, None, None, 0, 1.0, masks, s)
-        t = timer.mark("fft_y_inv", t)
-        call("pmb_pmfft_col2", nx, ny, nz, 2, 1, 1, aq, fp + C8, tp, masks, None, None, 0, 1.0, masks, s)
-        t = timer.mark("fft_y_inv_yz", t)
+        if ny <= PMFFT_JOINT_MAX:
+            call("pmb_pmfft_col2", nx, ny, nz, 9, 3, 0, aq, fp, tp, masks, None, None, 0, 1.0, masks, s)
+            t = timer.mark("fft_y_inv_all", t)
+        else:
+            call("pmb_pmfft_col2", nx, ny, nz, 1, 1, 0, aq, fp, tp, masks, None, None, 0, 1.0, masks, s)
+            t = timer.mark("fft_y_inv", t)
+            call("pmb_pmfft_col2", nx, ny, nz, 2, 1, 1, aq, fp + C8, tp, masks, None, None, 0, 1.0, masks, s)
+            t = timer.mark("fft_y_inv_yz", t)
         call("pmb_pmfft_z2", nx, ny, nz, 1, 3, fp, F.data_ptr(), tp, masks, masks, s)
         t = timer.mark("fft_z_c2r3", t)
     else:

@@ -30,7 +30,7 @@ import torch
 
 from . import lpt as _lpt
 from . import modes as _modes
-from ._lib import call, lib
+from ._lib import PMFFT_JOINT_MAX, call, lib
 from .cic import SortedParticles
 from .configuration import Configuration
 from .cosmology import Cosmology
@@ -182,6 +182,10 @@ def pmfft_stages(conf, reps, peak, only=None):
         "fft_z_c2r": lambda: call("pmb_pmfft_z", nx, ny, nz, 1, 1, a, real3b.data_ptr(), s),
         "fft_z_c2r3": lambda: call("pmb_pmfft_z", nx, ny, nz, 1, 3, a, real3b.data_ptr(), s),
     }
+    joint = ny <= PMFFT_JOINT_MAX  # the inverse y passes of a force in one launch
+    if joint:
+        stages["fft_y_inv_all"] = lambda: call("pmb_pmfft_col", nx, ny, nz, 9, 3, 0, a, b, tables, masks, None, None, 0,
+                                               1.0, s)
     # the same passes as stages of a force chain pruned to the particle-Nyquist
     # box (what pmb_force runs when the mesh is finer than the particle grid)
     live = None
@@ -202,6 +206,9 @@ def pmfft_stages(conf, reps, peak, only=None):
             "fft_z_c2r3_pruned": lambda: call("pmb_pmfft_z2", nx, ny, nz, 1, 3, a, real3b.data_ptr(), tables, masks,
                                               1, s),
         })
+        if joint:
+            stages["fft_y_inv_all_pruned"] = lambda: call("pmb_pmfft_col2", nx, ny, nz, 9, 3, 0, a, b, tables, masks,
+                                                          None, None, 0, 1.0, 1, s)
     out = {}
     for name, fn in stages.items():
         if only and name.replace("_pruned", "") not in only:

@@ -33,6 +33,7 @@ def algorithmic_bytes(op, N, M, Mc=None, R=None, T=None, live=None):
             "fft_y_yz": 8 * Mc * fz * (2 + fy),
             "fft_y_inv": 8 * Mc * fz * (fy + 1),
             "fft_y_inv_yz": 8 * Mc * fz * (fy + 2),
+            "fft_y_inv_all": 8 * Mc * fz * (2 * fy + 3),
             "fft_x_green": 24 * Mc * fy * fz,
             "fft_x_green_adj": 24 * Mc * fy * fz,
             "fft_z_c2r": 8 * Mc * fz + 4 * M,
@@ -61,6 +62,7 @@ def algorithmic_bytes(op, N, M, Mc=None, R=None, T=None, live=None):
         "fft_y_yz": 24 * Mc,
         "fft_y_inv": 16 * Mc,
         "fft_y_inv_yz": 24 * Mc,
+        "fft_y_inv_all": 40 * Mc,
         "fft_x_green": 24 * Mc,
         "fft_x_green_adj": 24 * Mc,
         "fft_x_adj": 24 * Mc,

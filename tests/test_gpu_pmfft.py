@@ -173,6 +173,35 @@ def test_staged_route_is_bitwise_the_fused_route():
         assert torch.equal(f, s)
 
 
+@pytest.mark.parametrize("shape,mesh", [((32, 32, 64), 2), ((32, 48, 64), 2), ((32, 64, 64), 2), ((32, 96, 64), 2),
+                                        ((32, 128, 64), 2), ((32, 192, 64), 2), ((32, 256, 64), 2), ((32, 384, 64), 2),
+                                        ((32, 512, 64), 2), ((64, 256, 128), 1)])
+def test_staged_route_runs_the_fused_passes(shape, mesh):
+    """The inverse y passes above all: one launch for all three channels up to 512 rows, two above."""
+    from pmpp_b200.runtime import StageTimer
+    pb, co, conf = _confs(shape, mesh)
+    pmid, disp = random_particles(co, seed=3, spread=2.0)
+    ptcl = pb.Particles(conf, torch.from_numpy(pmid).cuda(), torch.from_numpy(disp).cuda())
+    cos = pb.SimpleLCDM(conf)
+    fused = pb.gravity(1.0, ptcl, cos, conf)
+    with StageTimer() as timer:
+        staged = pb.gravity(1.0, ptcl, cos, conf)
+    assert torch.equal(fused, staged)
+    joint = conf.mesh_shape[1] <= _lib().PMFFT_JOINT_MAX
+    assert ("fft_y_inv_all" in timer.counts) == joint and ("fft_y_inv_yz" in timer.counts) != joint
+
+
+def test_joint_inverse_pass_limits():
+    L = _lib()
+    z = torch.zeros(16, device="cuda")  # refused before anything is read
+    tab = z.data_ptr()
+    for shape, nbatch in (((64, 768, 128), 3), ((64, 1024, 128), 3), ((64, 512, 128), 2), ((64, 64, 128), 1)):
+        for name, more in (("pmb_pmfft_col", ()), ("pmb_pmfft_col2", (0, ))):
+            with pytest.raises(L.PMBError, match="mode 9"):
+                L.call(name, *shape, 9, nbatch, 0, z.data_ptr(), z.data_ptr(), tab, 0, None, None, 0, 1.0, *more,
+                       _stream())
+
+
 def test_split_adjoint_x_pass_matches_fused():
     """Mode 8 (x forward + adjoint multiplier) followed by a plain inverse x pass
     equals the fused mode 7."""

@@ -194,24 +194,62 @@ def check(status, what):
         raise PMBError(f"{what} failed with status {status}: {msg}")
 
 
-# Hand-written kernels launched per entry point (cuFFT's own kernels excluded).
+# Hand-written kernels launched per entry point (cuFFT's own kernels excluded;
+# of an ensemble, which holds them, neither the FFT passes of its mesh classes).
+# Entries not listed here or in kernels_of launch none or are not counted.
 _KERNELS = {
-    "pmb_sort_rows": 3, "pmb_sort_rows_ex": 3, "pmb_cic_general_scatter": 3, "pmb_cic_general_gather": 1,
+    "pmb_cic_general_gather": 1,
     "pmb_cic_general_interp_grad": 1, "pmb_gather_rows": 1, "pmb_gather_rows2": 1, "pmb_interp_grad_rows": 1,
     "pmb_green_gradient": 1, "pmb_interlace_spectra": 1, "pmb_project_density": 1, "pmb_cnn_conv3d": 1,
     "pmb_cnn_conv3d_wgrad": 1, "pmb_cnn_stem_input": 1, "pmb_cnn_residual": 1, "pmb_cnn_residual_adjoint": 1,
     "pmb_cnn_norm_adjoint": 1, "pmb_green_potential": 1, "pmb_gradient_spectra": 1, "pmb_gradient_adjoint_plain": 1,
     "pmb_green_gradient_adjoint": 1, "pmb_axpy": 1,
     "pmb_kick_adj": 1, "pmb_kick_adj2": 1, "pmb_kick_adj3": 1, "pmb_drift_cot_adj": 1, "pmb_drift_adj": 1, "pmb_dot": 1,
-    "pmb_force": 9, "pmb_force2": 9, "pmb_force_streamed": 14, "pmb_force_vjp": 11, "pmb_force_vjp_presorted": 6, "pmb_sum": 1,
-    "pmb_white_noise_nested": 1, "pmb_linear_modes": 1,
-    "pmb_lpt": 4, "pmb_lpt_lattice": 4, "pmb_lpt_vjp": 6, "pmb_pk_shells": 1, "pmb_shell_stats": 1, "pmb_pk_shells_adjoint": 1,
-    "pmb_overdensity": 1, "pmb_ens_force": 7, "pmb_ens_step": 9, "pmb_ens_set_step": 1,
-    "pmb_force64": 5, "pmb_force64_interlaced": 7, "pmb_force_vjp64_interlaced": 6, "pmb_deposit64": 1, "pmb_axpy64": 1, "pmb_sum64": 1, "pmb_force_vjp64": 4, "pmb_dot64": 1, "pmb_lpt64_ex": 4, "pmb_lpt_vjp64": 6,
+    "pmb_sum": 1, "pmb_white_noise_nested": 1, "pmb_linear_modes": 1,
+    "pmb_pk_shells": 1, "pmb_shell_stats": 1, "pmb_pk_shells_adjoint": 1,
+    "pmb_overdensity": 1, "pmb_ens_force": 6, "pmb_ens_step": 8, "pmb_ens_set_step": 1,
+    "pmb_force64": 4, "pmb_force64_interlaced": 6, "pmb_force_vjp64": 4, "pmb_force_vjp64_interlaced": 6,
+    "pmb_deposit64": 1, "pmb_axpy64": 1, "pmb_sum64": 1, "pmb_dot64": 1, "pmb_lpt64_ex": 4, "pmb_lpt_vjp64": 6,
     "pmb_scatter_vjp64": 1, "pmb_white_noise_nested64": 1,
     "pmb_linear_modes64": 1, "pmb_lpt64": 4, "pmb_pk_shells64": 1, "pmb_pk_shells_adjoint64": 1, "pmb_overdensity64": 1,
     "pmb_pmfft_z": 1, "pmb_pmfft_col": 1, "pmb_pmfft_z2": 1, "pmb_pmfft_col2": 1,
 }
+
+
+def _sort_kernels(nx, ny):
+    """Counting, scan (one block up to 2^14 rows, two launches above), placing."""
+    return 3 if nx * ny <= 1 << 14 else 4
+
+
+def kernels_of(name, args):
+    """Hand-written kernels that a call of entry point `name` with `args` launches."""
+    if name in ("pmb_sort_rows", "pmb_sort_rows_ex"):
+        return _sort_kernels(*args[5:7])
+    if name == "pmb_scatter_rows":  # per-particle values: their maximum and the scale
+        return 1 if args[6] is None else 3
+    if name == "pmb_cic_general_scatter":
+        return 3 if args[16] is None else 4
+    if name in ("pmb_force", "pmb_force2"):  # sort, deposit, multiplier or passes, gather
+        nx, ny, nz = args[5:8]
+        chain = (5 if ny <= PMFFT_JOINT_MAX else 6) if pmfft_active(nx, ny, nz) else 1
+        return _sort_kernels(nx, ny) + chain + 2
+    if name == "pmb_force_streamed":  # sort, deposit, multiplier and gather per component, interleaving
+        return _sort_kernels(*args[5:7]) + 8
+    if name == "pmb_force_vjp":
+        return _sort_kernels(*args[3:5]) + (11 if pmfft_active(*args[3:6]) else 6)
+    if name == "pmb_force_vjp_presorted":  # position term, three-channel deposit, multiplier or passes, position term
+        return 11 if pmfft_active(*args[2:5]) else 6
+    if name in ("pmb_lpt", "pmb_lpt_lattice"):
+        return _lpt_kernels(args[6] if name == "pmb_lpt_lattice" else args[7])
+    if name == "pmb_lpt_vjp":
+        return 6
+    return _KERNELS.get(name, 0)
+
+
+def _lpt_kernels(order):
+    return 4 if order == 2 else 3
+
+
 _pmfft = {"enabled": True}
 _launches = [0]
 
@@ -269,14 +307,4 @@ def launch_count():
 def call(name, *args):
     """Call an entry point that returns a status and raise on failure."""
     check(getattr(lib(), name)(*args), name)
-    if name == "pmb_scatter_rows":
-        _launches[0] += 2 if args[6] is None else 3
-    else:
-        _launches[0] += _KERNELS.get(name, 0)
-        # the hand-written FFT chain replaces the multiplier kernel by six passes
-        if name in ("pmb_force", "pmb_force2") and pmfft_active(*args[5:8]):
-            _launches[0] += 5
-        elif name == "pmb_force_vjp" and pmfft_active(*args[3:6]):
-            _launches[0] += 5
-        elif name == "pmb_force_vjp_presorted" and pmfft_active(*args[2:5]):
-            _launches[0] += 5
+    _launches[0] += kernels_of(name, args)

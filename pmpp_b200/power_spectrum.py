@@ -89,11 +89,12 @@ def _shell_sums(spec, conf, mas_power, spec_b=None):
 
 
 def _finalize(p_sum, conf):
-    """:251-256: P = sum[1:] / nmodes * cell^3 / M."""
+    """:251-256: P = sum[1:] / nmodes * cell^3 / M (p_sum: device tensor, or its copy in numpy)."""
+    p_sum = p_sum if isinstance(p_sum, np.ndarray) else p_sum.cpu().numpy()
     k, nmodes = shell_statistics(conf)
     ns = num_shells(conf) - 1
     k, nmodes = k[:ns], nmodes[:ns]
-    pk = p_sum.cpu().numpy()[1:] / nmodes * (conf.cell_size**3 / conf.mesh_size)
+    pk = p_sum[1:] / nmodes * (conf.cell_size**3 / conf.mesh_size)
     return k, pk, nmodes
 
 
@@ -195,7 +196,7 @@ def pk_loss(ptcl, conf, pk_target, mas="CIC", grad=True, kmax=None):
     delta = torch.empty_like(rho)
     call("pmb_overdensity", rho.data_ptr(), delta.data_ptr(), rho.numel(), tot.data_ptr(), s)
     spec = _spectrum(delta, conf)
-    sums, _, _ = _shell_sums(spec, conf, mp)
+    sums = _shell_sums(spec, conf, mp)[0].cpu().numpy()
     k, pk, nmodes = _finalize(sums, conf)
     tgt = np.asarray(pk_target, dtype=np.float64)
     valid = (nmodes > 0) & (pk > 0) & (tgt > 0)
@@ -216,8 +217,10 @@ def pk_loss(ptcl, conf, pk_target, mas="CIC", grad=True, kmax=None):
          wd.data_ptr(), 1.0, gspec.data_ptr(), s)
     # delta = rho / m - 1 with m = sum(rho)/M: rho_cot = (dcot - sum(dcot delta)/M) / m.
     # The sum is 2 sum_s w_s S_s over the shell sums S_s (gspec is 2 w_s times the
-    # spectrum), so the constant enters as the zero mode and 1 / m as the particle value
-    gspec.view(-1)[:1].fill_(-2.0 * float(np.dot(w, sums.cpu().numpy())) / rho.numel())
+    # spectrum), so the constant enters as the zero mode and 1 / m as the particle value.
+    # (It cancels in the position term but for particles on a cell face, whose
+    # two-sided gradient takes the weights of one side.)
+    gspec.view(-1)[:1].fill_(-2.0 * float(np.dot(w, sums)) / rho.numel())
     m = float(tot.item()) / rho.numel()
     fw = workspace(lib().pmb_fft_work_bytes(nx, ny, nz, 1), dev, "fft1")
     dcot = torch.empty((1, nx, ny, nz), dtype=torch.float32, device=dev)

@@ -127,3 +127,53 @@ def test_overdensity_remainders(n, at):
         src[n - 1] = float("nan")
         call("pmb_overdensity", src.data_ptr(), out[at:].data_ptr(), n, tot.data_ptr(), stream_handle(rho.device))
         assert bool(out[at + n - 1].isnan()) and not bool(out[at:at + n - 1].isnan().any())
+
+
+@pytest.mark.parametrize("shape", [(8, 8, 8), (6, 10, 9)])
+def test_loss_gradient_of_particles_on_cell_faces(shape):
+    """The gradient of the P(k) loss against float64 autograd, with the mean density's own gradient, which
+    reaches particles on a cell face only (their two-sided gradient takes one side's weights).  Bar: float32
+    transforms and sums, 1e-5 of the largest component."""
+    import pmpp_b200 as pb
+    from pmpp_b200 import power_spectrum as ps
+    conf = _conf(shape)
+    rng = np.random.default_rng(5)
+    n = conf.ptcl_num
+    pmid = rng.integers(0, shape, size=(n, 3)).astype(np.int16)
+    disp = (rng.integers(0, 2**12, size=(n, 3)) * 2.0**-11).astype(np.float32)  # exact in cells of 2
+    disp[::3] = 0.0
+    ns = ps.num_shells(conf)
+    target = np.full(ns - 1, 50.0)
+    loss, got = ps.pk_loss(pb.Particles(conf, torch.from_numpy(pmid).cuda(), torch.from_numpy(disp).cuda()), conf,
+                           target)
+    shell, (mx, my, mz) = _shells(shape, ns)
+    w = (np.sinc(mx / shape[0]) * np.sinc(my / shape[1]) * np.sinc(mz / shape[2]))**-4.0
+    w = w * np.where((mz == 0) | ((shape[2] % 2 == 0) & (mz == shape[2] // 2)), 1.0, 2.0)
+    k, nmodes = ps.shell_statistics(conf)
+    nmodes = torch.from_numpy(nmodes[:ns - 1].astype(np.float64))
+
+    def reference(with_mean):
+        d = torch.from_numpy(disp).double().requires_grad_(True)
+        q = d / 2.0
+        low = torch.floor(q).detach()
+        f, base = q - low, torch.from_numpy(pmid).long() + low.long()
+        rho = torch.zeros(int(np.prod(shape)), dtype=torch.float64)
+        for b in range(8):
+            bit = torch.tensor([b & 1, (b >> 1) & 1, b >> 2])
+            i = torch.remainder(base + bit, torch.tensor(shape))
+            rho = rho.index_add(0, (i[:, 0] * shape[1] + i[:, 1]) * shape[2] + i[:, 2],
+                                (1 - (f - bit).abs()).prod(-1))
+        mean = rho.mean() if with_mean else rho.mean().detach()
+        spec = torch.fft.rfftn((rho / mean - 1).reshape(shape))
+        p = (spec.real**2 + spec.imag**2) * torch.from_numpy(w)
+        s = torch.zeros(ns, dtype=torch.float64).index_add(0, torch.from_numpy(shell).reshape(-1), p.reshape(-1))[1:]
+        pk = s / nmodes * (8.0 / np.prod(shape))
+        lr = torch.log(pk[nmodes > 0] / 50.0)
+        out = (lr**2).mean()
+        return float(out), torch.autograd.grad(out, d)[0].numpy()
+
+    ref_loss, ref = reference(True)
+    bar = 1e-5 * np.abs(ref).max()
+    np.testing.assert_allclose(loss, ref_loss, rtol=1e-5)
+    assert np.abs(got.cpu().numpy() - ref).max() <= bar
+    assert np.abs(reference(False)[1] - ref).max() > 100 * bar  # the mean's share is seen

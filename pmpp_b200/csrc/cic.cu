@@ -718,8 +718,8 @@ __global__ void __launch_bounds__(kRowThreads)
   const double inv = __hiloint2double(0x7FE00000 - __double2hiint(scale), 0);  // 1 / scale, a power of two
   const float invf = (float)inv, two_s = pow2f(split ? s : 0);
   const bool fconv = split && invf >= 0x1p-126f;
-  constexpr int kOff = SIGNED ? 0x4B400000 : 0x4B000000;
-  const F2 near2 = f2_pack(-__int_as_float(kOff), -__int_as_float(kOff));
+  constexpr unsigned kOff = SIGNED ? 0x4B400000u : 0x4B000000u;  // (sums modulo 2^32, so in unsigned)
+  const F2 near2 = f2_pack(-__uint_as_float(kOff), -__uint_as_float(kOff));
   const F2 two_s2 = f2_pack(two_s, two_s), inv2 = f2_pack(invf, invf);
   // exact integers in double precision through the bits of 2^52 + h (the
   // 64-bit integer conversions are ten times as dear); one fma rounds the sum
@@ -731,9 +731,9 @@ __global__ void __launch_bounds__(kRowThreads)
     if (split) return (float)(fma(as_double(planes[a]), (double)two_s, as_double(planes[PLANE + a])) * inv);
     return (float)((double)(long long)acc64[a] * inv);
   };
-  auto pair = [&](int h0, int h1, int l0, int l1, float& a, float& b) {
-    const F2 h = f2_add(f2_pack(__int_as_float(kOff + h0), __int_as_float(kOff + h1)), near2);
-    const F2 l = f2_add(f2_pack(__int_as_float(kOff + l0), __int_as_float(kOff + l1)), near2);
+  auto pair = [&](unsigned h0, unsigned h1, unsigned l0, unsigned l1, float& a, float& b) {
+    const F2 h = f2_add(f2_pack(__uint_as_float(kOff + h0), __uint_as_float(kOff + h1)), near2);
+    const F2 l = f2_add(f2_pack(__uint_as_float(kOff + l0), __uint_as_float(kOff + l1)), near2);
     int ia, ib;
     f2_bits(f2_mul(f2_fma(h, two_s2, l), inv2), ia, ib);
     a = __int_as_float(ia);
@@ -757,11 +757,11 @@ __global__ void __launch_bounds__(kRowThreads)
       float res[4];
       bool done = false;
       if (fconv) {
-        const int4 hi = reinterpret_cast<const int4*>(acc)[g], lo = reinterpret_cast<const int4*>(acc)[GROUPS + g];
-        const unsigned top = ((kOff + hi.x) ^ 0x4B000000) | ((kOff + hi.y) ^ 0x4B000000) |
-                             ((kOff + hi.z) ^ 0x4B000000) | ((kOff + hi.w) ^ 0x4B000000) |
-                             ((kOff + lo.x) ^ 0x4B000000) | ((kOff + lo.y) ^ 0x4B000000) |
-                             ((kOff + lo.z) ^ 0x4B000000) | ((kOff + lo.w) ^ 0x4B000000);
+        const uint4 hi = reinterpret_cast<const uint4*>(acc)[g], lo = reinterpret_cast<const uint4*>(acc)[GROUPS + g];
+        constexpr unsigned kTwo23 = 0x4B000000u;
+        const unsigned top = ((kOff + hi.x) ^ kTwo23) | ((kOff + hi.y) ^ kTwo23) | ((kOff + hi.z) ^ kTwo23) |
+                             ((kOff + hi.w) ^ kTwo23) | ((kOff + lo.x) ^ kTwo23) | ((kOff + lo.y) ^ kTwo23) |
+                             ((kOff + lo.z) ^ kTwo23) | ((kOff + lo.w) ^ kTwo23);
         if (top < 0x800000u) {
           pair(hi.x, hi.y, lo.x, lo.y, res[0], res[1]);
           pair(hi.z, hi.w, lo.z, lo.w, res[2], res[3]);

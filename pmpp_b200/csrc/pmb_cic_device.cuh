@@ -77,7 +77,10 @@ __device__ __forceinline__ Rec unmasked_or_origin(const Rec& r, bool* masked) {
   return z;
 }
 
-struct FastDiv {  // exact n / d for every 32-bit n
+// Exact n / d for every 32-bit n: a multiplication by a rounded-up reciprocal of 33
+// bits and shifts (Granlund and Montgomery, "Division by Invariant Integers using
+// Multiplication", 1994, figure 4.1).
+struct FastDiv {
   uint32_t mul;
   int sh1, sh2;
 };

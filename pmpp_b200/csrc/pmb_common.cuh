@@ -94,7 +94,6 @@ struct Real<float> {
   __device__ static __forceinline__ float floor_(float a) { return floorf(a); }
   __device__ static __forceinline__ float fabs_(float a) { return fabsf(a); }
   __device__ static __forceinline__ float rint_(float a) { return rintf(a); }
-  __device__ static __forceinline__ float pow_(float a, float b) { return powf(a, b); }
   __device__ static __forceinline__ float2 make2(float a, float b) { return make_float2(a, b); }
 };
 template <>
@@ -111,7 +110,6 @@ struct Real<double> {
   __device__ static __forceinline__ double floor_(double a) { return floor(a); }
   __device__ static __forceinline__ double fabs_(double a) { return fabs(a); }
   __device__ static __forceinline__ double rint_(double a) { return rint(a); }
-  __device__ static __forceinline__ double pow_(double a, double b) { return pow(a, b); }
   __device__ static __forceinline__ double2 make2(double a, double b) { return make_double2(a, b); }
 };
 

@@ -1021,7 +1021,8 @@ __global__ void __launch_bounds__(ColGeom<R1, R2>::T, CTAS)
 // KR rows per tile, T threads and CTAS resident CTAs per SM.  The phases of a
 // tile are separated by barriers, so other CTAs fill the gaps.  M = 512: one
 // CTA of 16 rows filled the shared memory, two of 8 rows take 5.12 -> 4.46 ms
-// (3-channel C2R, 1024^3) and 1.64 -> 1.50 ms (R2C).  M = 128: four CTAs of 8
+// (3-channel C2R, 1024^3) and 1.64 -> 1.50 ms (R2C); M = 384 likewise 2.53 -> 2.27 ms
+// (three R2C, 768^3), C2R 2.57 -> 2.58.  M = 128: four CTAs of 8
 // rows and 128 threads against two of 16 and 256 take 703 -> 644 us (14 R2C of
 // a 128^3-particle run) and 902 -> 865 us (C2R); the same at M = 256 is slower
 // (507 -> 554 us) and at M = 64 no faster.
@@ -1349,33 +1350,44 @@ int launch_col_ctas(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
 
 // Resident CTAs per SM of a pass of length L.  The passes that hold one
 // transform at a time fit 128 registers, so two CTAs share an SM and fill each
-// other's barriers: us with one / two, pruned: forward y 151 / 105 (512^3) and
-// 910 / 799 (1024^3), inverse y 140 / 131 (512^3) but 806 / 819 (1024^3), x +
-// multiplier 212 / 194 (512^3, though it spills).  The others spill too much:
-// x + multiplier 1082 / 1402 (1024^3), inverse y into two outputs 331 / 447
-// (512^3), y combine 310 / 437, adjoint x 222 / 302.  Lengths up to 256 run 128
-// threads a CTA, of which two share an SM at any register count.
+// other's barriers: us with one / two, pruned: forward y 151 / 105 (512^3), 84 / 60
+// (384^3) and 910 / 799 (1024^3), inverse y 140 / 131 (512^3), 78 / 59 (384^3) but
+// 806 / 819 (1024^3), x + multiplier 212 / 194 (512^3, though it spills).  The
+// others spill too much: x + multiplier 1082 / 1402 (1024^3), inverse y into two
+// outputs 331 / 447 (512^3), y combine 310 / 437, adjoint x 222 / 302.  On the
+// largest meshes two CTAs of 768 or 1024 rows lose, the more the fuller the
+// spectrum: whole spectra forward y 1585 / 2325 (1024^3), 411 / 499 (512 x 1024 x
+// 512), 779 / 1290 (768^3), 207 / 213 (384 x 768 x 384) but 100 / 93 (256 x 768 x
+// 256); pruned 436 / 371 (768^3), inverse 417 / 480 (768^3) but 117 / 111 (384 x 768 x
+// 384).  Lengths up to 256 run 128 threads a CTA, of which two share an SM at any
+// register count.
 constexpr int kInvAllMax = 512;  // longest y of the joint inverse pass
 
-constexpr int col_ctas(int mode, int L) {
-  if (L == 1024) return mode == kYFwd ? 2 : 1;
-  if (L == 512) return mode == kYFwd || mode == kYInv || mode == kXGreen || mode == kYInvAll ? 2 : 1;
-  if (L == 384) return mode == kYFwd || mode == kYInv || mode == kYInvAll ? 2 : 1;
-  if (L == 768) return mode == kYFwd || mode == kYInv ? 2 : 1;
-  return 1;
+int col_ctas(int mode, int L, bool pruned, int64_t cells) {
+  const int64_t m26 = (int64_t)1 << 26;
+  const bool y_fwd = mode == kYFwd, y_inv = mode == kYInv;
+  switch (L) {
+    case 384: return y_fwd || y_inv || mode == kYInvAll ? 2 : 1;
+    case 512: return y_fwd || y_inv || mode == kXGreen || mode == kYInvAll ? 2 : 1;
+    case 768: return (y_fwd && pruned) || ((y_fwd || y_inv) && cells <= (pruned ? 2 * m26 : m26)) ? 2 : 1;
+    case 1024: return y_fwd && pruned ? 2 : 1;
+    default: return 1;
+  }
 }
 
 template <int R1, int R2, int MODE, bool PR>
 int launch_col(const CUtensorMap& map, const ColArgs& a, cudaStream_t s) {
   constexpr int L = R1 * R2;
+  constexpr bool kSingle = MODE == kYFwd || MODE == kYInv || MODE == kYInvAll;  // one transform at a time, along y
   if constexpr (MODE == kYInvAll && L > kInvAllMax) {
     return kUnsupported;
-  } else if constexpr (L == 512 || L == 1024) {  // the lengths at which the two differ
-    const int ctas = g_col_ctas != 0 ? g_col_ctas : col_ctas(MODE, L);
+  } else if constexpr (L == 512 || L == 1024 || (L >= 384 && kSingle)) {  // where the two differ
+    int ctas = col_ctas(MODE, L, PR, (int64_t)a.nx * a.ny * a.nz);
+    if (g_col_ctas != 0 && (L == 512 || L == 1024)) ctas = g_col_ctas;
     if (ctas == 2) return launch_col_ctas<R1, R2, MODE, 2, PR>(map, a, s);
     return launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
   } else {
-    return launch_col_ctas<R1, R2, MODE, col_ctas(MODE, L), PR>(map, a, s);
+    return launch_col_ctas<R1, R2, MODE, 1, PR>(map, a, s);
   }
 }
 

@@ -9,6 +9,7 @@
 //    the adjoint of the shell power.
 #include <cmath>
 
+#include "pmb_cic_device.cuh"
 #include "pmb_common.cuh"
 #include "pmb_ic.cuh"
 
@@ -795,6 +796,59 @@ __global__ void __launch_bounds__(kPkThreads)
   }
 }
 
+// Rows too short or too few to occupy a warp each take a lane per mode whatever
+// its row.  us, warp per row / lane per mode: 1024^2 x 2 cells 370 / 31, 256^2 x 16 28.7 /
+// 12.6, 64^3 12.2 / 8.1, 512^2 x 62 92 / 74, 8^2 x 30000 236 / 15, 32^2 x 1024 14.7 / 10.6;
+// but 64^2 x 256 11.5 / 14.6, 128^3 19.0 / 21.0, 256^3 64 / 72.
+static bool mode_per_lane(Mesh3 m) {
+  return (m.nz / 2 + 1 <= 64 || m.rows() < 2048) && m.half_cells() < (int64_t)1 << 32;
+}
+
+// The shell sums with a lane per mode (mode_per_lane): the runs of equal shells end
+// anywhere, so a run's sum is added atomically.
+template <class T, bool CROSS>
+__global__ void __launch_bounds__(kPkThreads)
+    pk_shells_flat_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, FastDiv by_nzh, FastDiv by_ny,
+                          const T* __restrict__ sinc_tab, int mas_power, int num_shells, int copies,
+                          double* __restrict__ sums, const typename Real<T>::T2* __restrict__ spec_b,
+                          double* __restrict__ sums_b, double* __restrict__ sums_x) {
+  using T2 = typename Real<T>::T2;
+  constexpr int NS = CROSS ? 3 : 1;
+  extern __shared__ double sh[];  // copies x NS x num_shells
+  for (int t = threadIdx.x; t < copies * NS * num_shells; t += kPkThreads) sh[t] = 0.0;
+  __syncthreads();
+  const T *sx = sinc_tab, *sy = sx + m.nx, *sz = sy + m.ny;
+  const uint32_t nzh = (uint32_t)(m.nz / 2 + 1), total = (uint32_t)m.half_cells();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* hist = sh + (size_t)(warp % copies) * NS * num_shells;
+  for (int64_t c = ((int64_t)blockIdx.x * kPkWarps + warp) * 32; c < total; c += (int64_t)gridDim.x * kPkThreads) {
+    const bool in = c + lane < total;
+    const uint32_t j = in ? (uint32_t)c + lane : 0u;
+    const uint32_t row = div_by(j, by_nzh), k = j - row * nzh, ix = div_by(row, by_ny), iy = row - ix * m.ny;
+    const T2 va = spec[j];
+    T2 vb = va;
+    if (CROSS) vb = spec_b[j];
+    const long long mx = fft_mode((int)ix, m.nx), my = fft_mode((int)iy, m.ny);
+    const int shell = shell_of(mx * mx + my * my + (long long)k * k, num_shells);
+    const double w = mas_power > 0 ? (double)sx[ix] * (double)sy[iy] * (double)sz[k] : 1.0;
+    const double f = in ? z_factor(w, (int)k, m.nz, mas_power, true) : 0.0;
+    const double ar = va.x, ai = va.y;
+    add_runs((ar * ar + ai * ai) * f, shell, hist, false);
+    if (CROSS) {
+      const double br = vb.x, bi = vb.y;
+      add_runs((br * br + bi * bi) * f, shell, hist + num_shells, false);
+      add_runs((ar * br + ai * bi) * f, shell, hist + 2 * num_shells, false);
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < NS * num_shells; t += kPkThreads) {
+    double v = 0.0;
+    for (int c = 0; c < copies; ++c) v += sh[(size_t)c * NS * num_shells + t];
+    double* out = t < num_shells ? sums : t < 2 * num_shells ? sums_b : sums_x;
+    if (v != 0.0) atomicAdd(&out[t % num_shells], v);
+  }
+}
+
 template <class T, bool CROSS>
 static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
                             int num_shells, double* sums, const typename Real<T>::T2* spec_b, double* sums_b,
@@ -803,10 +857,25 @@ static int launch_pk_shells(const typename Real<T>::T2* spec, Mesh3 m, const T* 
   // no z table where it does not fit beside one copy
   const int64_t one = (int64_t)8 * (CROSS ? 3 : 1) * num_shells;
   if (one > 200 * 1024) return kUnsupported;
+  int copies = kPkWarps;
+  if (mode_per_lane(m)) {
+    while (copies > 1 && copies * one > 100 * 1024) copies /= 2;
+    auto k = pk_shells_flat_kernel<T, CROSS>;
+    const int smem = (int)(copies * one);
+    PMB_CUDA_CHECK(smem_optin((const void*)k, smem));
+    int64_t per_sm = kPkSmem / (smem + 1024);
+    per_sm = per_sm > 8 ? 8 : per_sm < 1 ? 1 : per_sm;
+    int64_t grid = (m.half_cells() + kPkThreads - 1) / kPkThreads;
+    if (grid > 148 * per_sm) grid = 148 * per_sm;
+    k<<<(unsigned)grid, kPkThreads, (size_t)smem, s>>>(spec, m, fast_div((uint32_t)(m.nz / 2 + 1)),
+                                                       fast_div((uint32_t)m.ny), sinc_tab, mas_power, num_shells, copies,
+                                                       sums, spec_b, sums_b, sums_x);
+    PMB_CUDA_CHECK(cudaGetLastError());
+    return kOk;
+  }
   int64_t table = 8 * ((int64_t)m.nz / 2 + 1);
   const bool tabulated = table + one <= kPkSmem;
   if (!tabulated) table = 0;
-  int copies = kPkWarps;
   while (copies > 1 && table + copies * one > 100 * 1024) copies /= 2;
   const int64_t smem = table + copies * one;
   auto k = tabulated ? pk_shells_kernel<T, CROSS, true> : pk_shells_kernel<T, CROSS, false>;
@@ -882,9 +951,39 @@ __global__ void __launch_bounds__(kPkThreads)
 }
 
 template <class T>
+__global__ void __launch_bounds__(kPkThreads)
+    pk_shells_adjoint_flat_kernel(const typename Real<T>::T2* __restrict__ spec, Mesh3 m, FastDiv by_nzh, FastDiv by_ny,
+                                  const T* __restrict__ sinc_tab, int mas_power, int num_shells,
+                                  const double* __restrict__ wshell, double post,
+                                  typename Real<T>::T2* __restrict__ out) {
+  const T *sx = sinc_tab, *sy = sx + m.nx, *sz = sy + m.ny;
+  const uint32_t nzh = (uint32_t)(m.nz / 2 + 1);
+  const int64_t total = m.half_cells();
+  for (int64_t t = (int64_t)blockIdx.x * kPkThreads + threadIdx.x; t < total; t += (int64_t)gridDim.x * kPkThreads) {
+    const uint32_t j = (uint32_t)t;
+    const uint32_t row = div_by(j, by_nzh), k = j - row * nzh, ix = div_by(row, by_ny), iy = row - ix * m.ny;
+    const typename Real<T>::T2 v = spec[j];
+    const long long mx = fft_mode((int)ix, m.nx), my = fft_mode((int)iy, m.ny);
+    const int shell = shell_of(mx * mx + my * my + (long long)k * k, num_shells);
+    const double w = mas_power > 0 ? (double)sx[ix] * (double)sy[iy] * (double)sz[k] : 1.0;
+    const double f = 2.0 * post * window_pow(w, mas_power) * wshell[shell];
+    out[j] = Real<T>::make2((T)(v.x * f), (T)(v.y * f));
+  }
+}
+
+template <class T>
 static int launch_pk_adjoint(const typename Real<T>::T2* spec, Mesh3 m, const T* sinc_tab, int mas_power,
                              int num_shells, const double* wshell, double post, typename Real<T>::T2* out,
                              cudaStream_t s) {
+  if (mode_per_lane(m)) {
+    int64_t grid = (m.half_cells() + kPkThreads - 1) / kPkThreads;
+    if (grid > 148 * 8) grid = 148 * 8;
+    pk_shells_adjoint_flat_kernel<T><<<(unsigned)grid, kPkThreads, 0, s>>>(
+        spec, m, fast_div((uint32_t)(m.nz / 2 + 1)), fast_div((uint32_t)m.ny), sinc_tab, mas_power, num_shells, wshell,
+        post, out);
+    PMB_CUDA_CHECK(cudaGetLastError());
+    return kOk;
+  }
   int64_t grid = (m.rows() + kPkWarps - 1) / kPkWarps;
   if (grid > 148 * 8) grid = 148 * 8;
   const int64_t table = 8 * ((int64_t)m.nz / 2 + 1);

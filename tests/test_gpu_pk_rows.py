@@ -54,10 +54,14 @@ def test_shell_sums_and_cross(shape, mas):
 
 # rows whose window table along z is above 48 KB, and above all of shared memory
 LONG = [(2, 3, 12288), (4, 1, 40001), (2, 1, 57344)]
+# many rows on either side of the length from which a warp takes a row
+EDGE = [(64, 33, 125), (64, 33, 126), (45, 45, 130), (48, 43, 130)]
 
 
 @pytest.mark.parametrize("shape,cross,ns", [(LONG[0], True, 40), (LONG[1], False, 40), (LONG[2], False, 40),
-                                            (LONG[2], True, 40), ((4, 2, 8192), True, 8533), ((2, 2, 40001), False, 25600)])
+                                            (LONG[2], True, 40), ((4, 2, 8192), True, 8533),
+                                            ((2, 2, 40001), False, 25600), ((1030, 2, 12288), True, 40),
+                                            ((2048, 1, 26000), False, 8000)] + [(e, True, 60) for e in EDGE])
 @pytest.mark.parametrize("mas", [0, 2])
 def test_shell_sums_of_long_rows(shape, cross, ns, mas):
     """Rows up to and beyond the length whose table fits beside the sums: FP64 products and sums of at most
@@ -84,7 +88,7 @@ def test_shell_sums_of_long_rows(shape, cross, ns, mas):
         assert np.all(np.abs(out[i].cpu().numpy() - ref) <= 2.0**-34 * mag)
 
 
-@pytest.mark.parametrize("shape", [(4, 4, 4), (5, 3, 7), (9, 8, 65), (3, 2, 1), (2, 70, 130)] + LONG)
+@pytest.mark.parametrize("shape", [(4, 4, 4), (5, 3, 7), (9, 8, 65), (3, 2, 1), (2, 70, 130), (2050, 1, 12288)] + LONG + EDGE)
 def test_adjoint_rows(shape):
     """out = spec * 2 post W^-2p w[shell], in float64 and rounded once (bar 2^-22)."""
     from pmpp_b200 import power_spectrum as ps

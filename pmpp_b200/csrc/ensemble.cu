@@ -36,8 +36,9 @@ namespace pmb {
 
 constexpr int kEnsMaxSims = 1024;
 
-// Tile shapes are limited to 200 KB at this many bytes per cell (the
-// accumulator takes two thirds of it).
+// Tile shapes are limited to 200 KB at this many bytes per cell, the interface's
+// line (the accumulator takes two thirds of it): what set_tiles takes and refuses does
+// not move with the accumulator.
 constexpr int64_t kTileBytesPerCell = 12;
 
 // Device descriptor of one member simulation.
@@ -321,8 +322,8 @@ struct Ensemble {
   uint32_t* tile_sums = nullptr;
   void* fft_work = nullptr;
   int64_t fft_bytes = 0;
-  // the hand-written FFT pass chain (power-of-two member meshes): one work
-  // area of five blocked spectral channels, reused member after member
+  // the hand-written FFT pass chain (member meshes of sides 2^a and 3 2^a): one
+  // work area of five blocked spectral channels, reused member after member
   void* pm_work = nullptr;
   int64_t pm_bytes = 0;
   bool any_cufft = false;

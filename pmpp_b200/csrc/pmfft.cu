@@ -473,7 +473,9 @@ __device__ __forceinline__ bool ky_live(const Live& L, int ky, int ny) { return 
 // column's constants are kyz2 = ky^2 + kz^2 and c0 = -post * my * mz (0 on
 // the zero-padding columns); HAS_T: a transfer or radial table is present.
 // The quotient uses the fast division (2 ulp), well inside the float32 bar
-// of the force parity tests.
+// of the force parity tests; the force and its adjoint lie nearer to float64 than
+// by the library's transforms and the multiplier with a rounded division, on every
+// side 3 2^a tried (192^3: 1.8e-7 against 3.2e-7; 384^3: 1.9e-7 against 4.5e-7).
 template <bool HAS_T>
 __device__ __forceinline__ float green_scalar(const ColArgs& a, const float* kx2, const float* mx, float kyz2,
                                               float c0, int ix, int iy, int iz) {

@@ -137,20 +137,33 @@ class Ensemble:
         return slice(int(self.pstart[j]), int(self.pstart[j + 1]))
 
     def load(self, ptcls):
-        """Copy each member's pmid / disp / vel (Particles, caller order)."""
+        """Copy each member's pmid / disp / vel (Particles, caller order), member after member where the
+        particles are views of the ensemble's own arrays, else an array at a time."""
         dst = {"pmid": [], "disp": [], "vel": []}
         src = {"pmid": [], "disp": [], "vel": []}
+        held = {getattr(self, name).untyped_storage().data_ptr() for name in dst}
         for i, p in enumerate(ptcls):
             sl = self._slot(i)
-            for name in dst:
-                if name == "vel" and p.vel is None:
-                    self.vel[sl].zero_()
-                    continue
-                dst[name].append(getattr(self, name)[sl])
-                src[name].append(getattr(p, name))
+            given = {name: getattr(p, name) for name in dst if getattr(p, name) is not None or name != "vel"}
+            if any(t.untyped_storage().data_ptr() in held for t in given.values()):
+                self._copy_members(dst, src)  # the members before this one, in their order
+                for name, t in given.items():
+                    getattr(self, name)[sl].copy_(t)
+            else:
+                for name, t in given.items():
+                    dst[name].append(getattr(self, name)[sl])
+                    src[name].append(t)
+            if "vel" not in given:
+                self.vel[sl].zero_()
+        self._copy_members(dst, src)
+
+    @staticmethod
+    def _copy_members(dst, src):
         for name in dst:
             if dst[name]:
                 torch._foreach_copy_(dst[name], src[name])
+                dst[name].clear()
+                src[name].clear()
 
     def particles(self, i, clone=True):
         sl = self._slot(i)

@@ -101,3 +101,22 @@ def test_fft_chain_members_are_bitwise_single_runs(graph):
         for name in ("disp", "vel", "acc"):
             assert torch.equal(getattr(out, name), getattr(ref, name)), name
     assert _lib.pmfft_timeouts() == 0
+
+
+def test_load_of_the_ensembles_own_views_in_member_order():
+    """Members moved up by one place from views, a fresh one last, velocities left out once: each copy sees
+    the arrays as the ones before it left them."""
+    import pmpp_b200 as pb
+    from pmpp_b200.ensemble import Ensemble
+    confs, coss, ics = _members([(12, 2, 50.0, 0.3)] * 5)
+    ens = Ensemble(confs, coss)
+    ens.load(ics)
+    ens.load([ens.particles(i + 1, clone=False) for i in range(4)] + [ics[0]])
+    for k, want in enumerate([1, 2, 3, 4, 0]):
+        for name in ("pmid", "disp", "vel"):
+            assert torch.equal(getattr(ens.particles(k), name), getattr(ics[want], name))
+    fresh = [pb.Particles(confs[0], p.pmid, p.disp) for p in ics[:2]]
+    ens.load([ens.particles(1, clone=False), fresh[0], ens.particles(1, clone=False), ics[4], fresh[1]])
+    for k, want in enumerate([ics[2], ics[0], ics[0], ics[4], ics[1]]):
+        assert torch.equal(ens.particles(k).disp, want.disp)
+    assert not bool(ens.particles(1).vel.any()) and not bool(ens.particles(4).vel.any())
